@@ -632,6 +632,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     // gathered position (md_interaction_list_reconstructbpm.cu:141-186). The next record
     // is fetched while the current one is computed.
     f3 fsb = mk3(0.f, 0.f, 0.f), msb = fsb;
+    SumTerms bsum{fsb, msb};
     uint32_t nbroken = 0;
     {
         const uint32_t wb = __reduce_or_sync(FULL, bmask);
@@ -666,7 +667,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
             const f3 r = mk3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
             f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
             f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
-            const bool broke = bond_slot(c.bp, r, vi, f4to3(vj), wi, f4to3(wj), il, rij, oijt, mijn, mijt, fsb, msb);
+            const bool broke = bond_slot(c.bp, r, vi, f4to3(vj), wi, f4to3(wj), il, rij, oijt, mijn, mijt, bsum);
             d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
             d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
             d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
@@ -685,6 +686,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     const uint32_t cm_in = cm;
     const float twoR = 2.0f * c.cp.rP;
     f3 fsc = mk3(0.f, 0.f, 0.f), msc = fsc;
+    SumTerms csum{fsc, msc};
     uint32_t cm_out = 0;
     {
         uint32_t m = live & ~bond;
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
             if (!(rijm < twoR)) continue;
             const uint32_t bit = 1u << k;
             f3 o = (cm_in & bit) ? mk3(oin[3 * k], oin[3 * k + 1], oin[3 * k + 2]) : mk3(0.f, 0.f, 0.f);
-            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, fsc, msc);
+            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, csum);
             oout[3 * k] = o.x; oout[3 * k + 1] = o.y; oout[3 * k + 2] = o.z;
             cm_out |= bit;
         }
@@ -763,7 +765,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
             if (!(rijm < twoR)) continue;
             const uint32_t bit = 1u << k;
             f3 o = (cm & bit) ? mk3(oin[3 * k], oin[3 * k + 1], oin[3 * k + 2]) : mk3(0.f, 0.f, 0.f);
-            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, fsc, msc);
+            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, csum);
             oout[3 * k] = o.x; oout[3 * k + 1] = o.y; oout[3 * k + 2] = o.z;
             cm_out |= bit;
         }

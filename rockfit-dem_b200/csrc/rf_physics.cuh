@@ -24,13 +24,32 @@ __device__ __forceinline__ float norm3(float x, float y, float z) {
     return __fsqrt_rn(x * x + y * y + z * z);
 }
 
+// A slot's force and moment terms, in the order the reference adds them to the particle's
+// sums. SumTerms adds them at once; KeepTerms keeps them apart, for a particle's lane to add
+// in slot order when other lanes evaluated its slots (the rounding of the sums is the same).
+struct SumTerms {
+    f3 &fs, &ms;
+    __device__ __forceinline__ void f(float x, float y, float z) { fs.x += x; fs.y += y; fs.z += z; }
+    __device__ __forceinline__ void m(float x, float y, float z) { ms.x += x; ms.y += y; ms.z += z; }
+    __device__ __forceinline__ void clear_m() { ms = mk3(0.f, 0.f, 0.f); }
+};
+struct KeepTerms {
+    f3 ft[2], mt[3];
+    int nf = 0, nm = 0;
+    bool clear = false;          // the contact's zero-spin rule clears the moment sum after its terms
+    __device__ __forceinline__ void f(float x, float y, float z) { ft[nf++] = mk3(x, y, z); }
+    __device__ __forceinline__ void m(float x, float y, float z) { mt[nm++] = mk3(x, y, z); }
+    __device__ __forceinline__ void clear_m() { clear = true; }
+};
+
 // One bond slot i->j (d_CalculateForcesDEM_22 loop body, :441-473). r = Rj - Ri.
-// Accumulates into fs, ms in the reference's order and updates the slot state.
-// Returns true when the break check fired (the slot is then type 0 and its
-// Oijt, Mijn, Mijt are zero).
+// Hands its terms (two of force, three of moment) to `acc` in the reference's order and
+// updates the slot state. Returns true when the break check fired (the slot is then type 0
+// and its Oijt, Mijn, Mijt are zero).
+template <class Acc>
 __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const f3 vi, const f3 vj,
                                           const f3 wi, const f3 wj, const float il, f3& Rij, f3& Oijt,
-                                          f3& Mijn, f3& Mijt, f3& fs, f3& ms) {
+                                          f3& Mijn, f3& Mijt, Acc& acc) {
     // dd_Calculate_rijm_nij_2 (:38-52)
     const float rijm = norm3(r.x, r.y, r.z);
     const float inv_rm = __frcp_rn(rijm);
@@ -39,7 +58,7 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
     float cef = p.m_E * (rijm - __frcp_rn(il)) * il;
     float Sc = cef;
     cef *= p.b_r * p.b_r * RF_PI_F;
-    fs.x += nx * cef; fs.y += ny * cef; fs.z += nz * cef;
+    acc.f(nx * cef, ny * cef, nz * cef);
     // dd_Calculate_M123_bpm_2 (:54-89)
     const float tx = Rij.y * nz - Rij.z * ny;
     const float ty = Rij.z * nx - Rij.x * nz;
@@ -68,7 +87,7 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
         const float mz = M3x * o.x + M3y * o.y + M3z * o.z + nz * c1;
         Mijn = mk3(mx, my, mz);
         c1 = RF_PI_F * p.b_r * p.b_r * p.b_r * p.b_r;
-        ms.x += mx * c1; ms.y += my * c1; ms.z += mz * c1;
+        acc.m(mx * c1, my * c1, mz * c1);
     }
     // dd_Calculate_mijt_bpm_2 (:131-152): the summed moment carries dt*E/(4 L0) twice
     {
@@ -80,7 +99,7 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
         const float mz = M3x * o.x + M3y * o.y + M3z * o.z + (dwz - nz * c1) * c2;
         Mijt = mk3(mx, my, mz);
         c2 *= RF_PI_F * p.b_r * p.b_r * p.b_r * p.b_r;
-        ms.x += mx * c2; ms.y += my * c2; ms.z += mz * c2;
+        acc.m(mx * c2, my * c2, mz * c2);
     }
     // dd_Calculate_fijt_mijunsym_bpm_2 (:154-197)
     float Mc;
@@ -97,11 +116,9 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
         c = p.m_G * il;
         Mc = c;
         c *= p.b_r * p.b_r * RF_PI_F;
-        fs.x += ox * c; fs.y += oy * c; fs.z += oz * c;
+        acc.f(ox * c, oy * c, oz * c);
         Oijt = mk3(ox, oy, oz);
-        ms.x += 0.5f * (r.y * oz - r.z * oy) * c;
-        ms.y += 0.5f * (r.z * ox - r.x * oz) * c;
-        ms.z += 0.5f * (r.x * oy - r.y * ox) * c;
+        acc.m(0.5f * (r.y * oz - r.z * oy) * c, 0.5f * (r.z * ox - r.x * oz) * c, 0.5f * (r.x * oy - r.y * ox) * c);
     }
     // dd_CheckBreakConditionDEM_2 (:20-36)
     Mc *= norm3(Oijt.x, Oijt.y, Oijt.z);
@@ -116,23 +133,13 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
     return false;
 }
 
-// One contact slot of type 0 (d_CalculateForcesDEM_21 loop body, :356-402).
-// r = Rj - Ri. Returns true when the pair overlaps (rijm < 2 rP); otherwise the
-// caller sets Oijt to zero, as the reference does.
-// The overlapping pair (rijm < 2 rP) part of the contact slot; rijm = norm3(r).
+// One overlapping contact slot of type 0 (d_CalculateForcesDEM_21 loop body, :356-402);
+// r = Rj - Ri, rijm = norm3(r) < 2 rP (a pair that does not overlap has its Oijt set to zero
+// by the caller, as the reference does). Hands two force and two moment terms to `acc`, or
+// one moment term and the clear of the moment sum.
+template <class Acc>
 __device__ __forceinline__ void contact_pair(const ContactParams& p, const f3 r, const float rijm, const f3 vi,
-                                             const f3 vj, const f3 wi, const f3 wj, f3& Oijt, f3& fs, f3& ms);
-
-__device__ __forceinline__ bool contact_slot(const ContactParams& p, const f3 r, const f3 vi, const f3 vj,
-                                             const f3 wi, const f3 wj, f3& Oijt, f3& fs, f3& ms) {
-    const float rijm = norm3(r.x, r.y, r.z);
-    if (!(rijm < 2.0f * p.rP)) return false;
-    contact_pair(p, r, rijm, vi, vj, wi, wj, Oijt, fs, ms);
-    return true;
-}
-
-__device__ __forceinline__ void contact_pair(const ContactParams& p, const f3 r, const float rijm, const f3 vi,
-                                             const f3 vj, const f3 wi, const f3 wj, f3& Oijt, f3& fs, f3& ms) {
+                                             const f3 vj, const f3 wi, const f3 wj, f3& Oijt, Acc& acc) {
     const float inv_rm = __frcp_rn(rijm);
     const float nx = r.x * inv_rm, ny = r.y * inv_rm, nz = r.z * inv_rm;
     // dd_Calculate_fijn_ppHM_2 (:199-253)
@@ -146,7 +153,7 @@ __device__ __forceinline__ void contact_pair(const ContactParams& p, const f3 r,
     const float vn = nx * vx + ny * vy + nz * vz;
     const float fn = (rijm - 2.0f * p.rP) * Kn * RF_2D3_F;
     c1 = -1.8257f * p.p_A * vn * __fsqrt_rn(Kn * 0.5f * p.mP);
-    fs.x += nx * (fn + c1); fs.y += ny * (fn + c1); fs.z += nz * (fn + c1);
+    acc.f(nx * (fn + c1), ny * (fn + c1), nz * (fn + c1));
     const float vtx = vx - nx * vn, vty = vy - ny * vn, vtz = vz - nz * vn;
     // dd_Calculate_fijtmijt_ppHM_2 (:255-314)
     const f3 o = Oijt;
@@ -172,17 +179,15 @@ __device__ __forceinline__ void contact_pair(const ContactParams& p, const f3 r,
         ftx += vtx * c; fty += vty * c; ftz += vtz * c;
     }
     Oijt = mk3(ox, oy, oz);
-    fs.x += ftx; fs.y += fty; fs.z += ftz;
-    ms.x += (ny * ftz - nz * fty) * p.rP;
-    ms.y += (nz * ftx - nx * ftz) * p.rP;
-    ms.z += (nx * fty - ny * ftx) * p.rP;
+    acc.f(ftx, fty, ftz);
+    acc.m((ny * ftz - nz * fty) * p.rP, (nz * ftx - nx * ftz) * p.rP, (nx * fty - ny * ftx) * p.rP);
     // dd_Calculate_mijroll_ppHM_2 (:316-336): a (near-)zero spin clears the whole sum
     const float wim = wi.x * wi.x + wi.y * wi.y + wi.z * wi.z;
     if ((double)wim > 1e-18) {
         const float cr = -p.m_muroll * fabsf(fn) * __frsqrt_rn(wim);
-        ms.x += wi.x * cr; ms.y += wi.y * cr; ms.z += wi.z * cr;
+        acc.m(wi.x * cr, wi.y * cr, wi.z * cr);
     } else {
-        ms = mk3(0.f, 0.f, 0.f);
+        acc.clear_m();
     }
 }
 
@@ -191,6 +196,12 @@ __device__ __forceinline__ float dist2_rn(const f3 a, const f3 b) {
     const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
+
+// The list kernels' (double)rr > 1e-10 and (double)rr < 1e-10 without the conversion to
+// double: the float 1e-10f is the smallest one above 1e-10 (and no float equals it), so the
+// comparisons with it decide every float, NaN included, as those in double do.
+__device__ __forceinline__ bool above_1em10(float rr) { return rr >= 1e-10f; }
+__device__ __forceinline__ bool below_1em10(float rr) { return rr < 1e-10f; }
 
 // Cell grid of the reference (cell_data): cell edge a, 1/a, Nr.
 struct RefGrid {
