@@ -51,7 +51,7 @@
 #define RF_CB1 0.05f
 #define RF_CB2 0.15f
 #define RF_CB3 0.3f
-#define RF_REC_DELETE 1u          // beyond the bond's keep distance: the slot is deleted (partner id in the force word)
+#define RF_REC_DELETE 1u          // beyond the bond's keep distance: the slot is deleted
 #define RF_REC_BROKE 2u           // the bond broke this step
 #define RF_REC_PARALLEL 4u        // the pair overlaps: the slot's contact was taken with the bond
 #define RF_REC_CLEAR 8u           // that contact's zero-spin rule cleared the particle's moment sum
@@ -72,7 +72,7 @@ struct DevScalars {
     float RR, _1d_Area, Hd2;
     int32_t Loading, Fracture;
     unsigned long long steps, target, rebuilds, curve_n, broken;
-    uint32_t done, err, rebuild, moved, block_counter, pad;
+    uint32_t done, err, rebuild, moved, block_counter, spec_counter;
     // largest displacement since the last candidate build of the positions a step reads
     // (FP32 bits of its square, accumulated by the step writing them), for skipping scans
     uint32_t d2max_next;
@@ -121,20 +121,20 @@ struct Consts {
 };
 
 // Per-specimen geometry of a batch (constant during a run): the platen's cut height, the
-// cut box and its hidden point, the specimen's particle range and the CTAs touching it.
+// cut box and its hidden point, the specimen's particle range.
 struct SpecGeom {
     float zcut;
     rf_float3 box_c, box_h, hp;
     uint32_t p0, p1;
-    uint32_t b0, b1;
 };
 
 struct Dev {
     // batch of specimens (one specimen: spec == sc, geom[0], blk_spec == nullptr)
     DevScalars* spec;           // [nspec] per-specimen platen / result scalars
     const SpecGeom* geom;       // [nspec]
-    const uint16_t* blk_spec;   // [blocks] first specimen of each 128-particle CTA
-    double2* partial2;          // [blocks] load partials of a CTA's second specimen
+    const uint16_t* blk_spec;   // [N / 128] specimen of the first of every 128 particles
+    double2* partial2;          // [CTAs] load partials of a CTA's second specimen
+    uint32_t *nz, *nz2;         // [CTAs / 32] CTAs whose partial / partial2 was written this step
     uint32_t nspec;
     double4* posd[2];   // extended model: x, y, z (FP64) and radius
     double* bL0;        // extended model: [QB][N] rest length of each bond record
@@ -169,13 +169,17 @@ struct Dev {
     uint32_t* cg_start; // [cells+1]
     uint32_t* cg_fill;  // [cells+1]
     uint32_t* cg_bsum;
-    uint32_t* cg_sorted;   // [N]
-    double2* partial;   // [blocks]
+    uint32_t* cg_sorted;   // [N] particle ids in cell order
+    uint32_t* cg_slot;     // [N] place of each particle in that order
+    float4* cg_pos;        // [N] positions (x, y, z, radius) in that order
+    double2* partial;   // [CTAs] load partials (extended model: where the CTA has any, see nz)
     // FIRE relaxation (allocated on first use)
     float4* frc;        // [N] net force after the platen clamp
     float4* mom;        // [N] net moment
-    double* fpart;      // [blocks][FIRE_SUMS] FP64 block partial sums (of a CTA's first specimen)
-    double* fpart2;     // [blocks][FIRE_SUMS] the same for a CTA's second specimen (batches)
+    double* fpart;      // [CTAs][FIRE_SUMS] FP64 partial sums (of a CTA's first specimen)
+    double* fpart2;     // [CTAs][FIRE_SUMS] the same for a CTA's second specimen (batches)
+    double* fgrp;       // [groups][FIRE_SUMS] sums over FIRE_GROUP CTAs of a specimen
+    uint32_t* fgrp_n;   // [groups] CTAs of the group that have arrived
     double4* rot;       // [N] accumulated rotation of the increment (sum of w dt)
     double4* x0;        // [N] positions at the start of the increment
     unsigned long long n_particles;
@@ -255,9 +259,14 @@ __global__ void k_rb_scan_sums(Dev d, Consts c) {
 __global__ void k_rb_scan_totals(Dev d, Consts c) {
     if (gate_closed(d, c)) return;
     const uint32_t nb = (c.cg_cells + 1 + 4095) / 4096;
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (uint32_t b = 0; b < nb; ++b) { uint32_t v = d.cg_bsum[b]; d.cg_bsum[b] = acc; acc += v; }
+    const uint32_t lane = threadIdx.x;             // one warp
+    uint32_t acc = 0;
+    for (uint32_t b0 = 0; b0 < nb; b0 += 32) {
+        const uint32_t v = b0 + lane < nb ? d.cg_bsum[b0 + lane] : 0;
+        uint32_t incl = v;
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= (uint32_t)o) incl += y; }
+        if (b0 + lane < nb) d.cg_bsum[b0 + lane] = acc + incl - v;
+        acc += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
@@ -287,100 +296,96 @@ __global__ void k_rb_scan_apply(Dev d, Consts c) {
 
 __global__ void k_rb_scatter(Dev d, Consts c) {
     if (gate_closed(d, c)) return;
+    const uint32_t cur = (uint32_t)(d.sc->steps & 1);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
         const uint32_t key = d.cg_key[i];
-        d.cg_sorted[d.cg_start[key] + atomicAdd(&d.cg_fill[key], 1u)] = i;
+        const uint32_t s = d.cg_start[key] + atomicAdd(&d.cg_fill[key], 1u);
+        d.cg_sorted[s] = i;
+        d.cg_slot[i] = s;
+        d.cg_pos[s] = posf(d, c, cur, i);
     }
 }
 
-// Candidates: every j != i within rc of i (27 cells), and which of them sit in i's row.
-__global__ void k_rb_cand(Dev d, Consts c) {
+// Candidates: every j != i within rc of i (27 cells), in the order of their margin bucket (a
+// scan needs no candidate of a bucket whose lower bound the displacements since this build
+// cannot have closed, see scan_limit), which of them sit in i's row, and the margin of the
+// nearest that does not. Positions are read in cell order (three x-neighbouring cells are one
+// run of float4 records, nine runs a particle) and the candidates wait in shared memory, as
+// places in that order, until their buckets and the row's members are known; a row member
+// is found by its place. 4M particles: 3.0 ms with an id and a position gathered for
+// every occupant and the list ordered and matched in memory, RB_AFTER ms so.
+#define RF_RB_CTA 128
+__global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
     if (gate_closed(d, c)) return;
-    const uint32_t cur = (uint32_t)(d.sc->steps & 1);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
-        const float4 xi = posf(d, c, cur, i);
+    __shared__ uint32_t s_c[64][RF_RB_CTA];
+    const uint32_t tid = threadIdx.x, mine = blockIdx.x * RF_RB_CTA + tid;
+    if (mine < c.N) {
+        const uint32_t i = d.cg_sorted[mine], key = d.cg_key[i];
+        const float4 xi = d.cg_pos[mine];
         d.pos_ref[i] = xi;
-        const uint32_t key = d.cg_key[i];
+        auto cut_of = [&](const float4 xj) { return c.lgap_f > 0.f ? fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) : c.acut_f; };
         uint32_t n = 0;
+        unsigned long long k0 = 0ull, k1 = 0ull;           // bits 0 and 1 of the candidates' buckets
         if (key < c.cg_cells) {
             const int ix = key % c.cg_nx, iy = (key / c.cg_nx) % c.cg_ny, iz = key / (c.cg_nx * c.cg_ny);
-            for (int dz = -1; dz <= 1; ++dz) {
-                const int z = iz + dz;
-                if (z < 0 || z >= (int)c.cg_nz) continue;
-                for (int dy = -1; dy <= 1; ++dy) {
-                    const int y = iy + dy;
-                    if (y < 0 || y >= (int)c.cg_ny) continue;
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        const int x = ix + dx;
-                        if (x < 0 || x >= (int)c.cg_nx) continue;
-                        const uint32_t cell = x + c.cg_nx * (y + c.cg_ny * z);
-                        const uint32_t s = d.cg_start[cell], e = s + d.cg_count[cell];
-                        for (uint32_t q = s; q < e; ++q) {
-                            const uint32_t j = d.cg_sorted[q];
-                            if (j == i) continue;
-                            const float4 xj = posf(d, c, cur, j);
-                            const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
-                            const float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                            bool near = d2 < c.rc2;
-                            if (c.lgap_f > 0.f && near) {
-                                const float q = fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) + c.skin_f;
-                                near = d2 < q * q;
-                            }
-                            if (near) {
-                                if (n < c.KC) d.cand[(size_t)n * c.N + i] = j;
-                                else raise_status(&d.sc->err, RF_ERR_CAPACITY);
-                                ++n;
-                            }
+            const uint32_t xa = ix > 0 ? ix - 1 : 0, xb = ix + 1 < (int)c.cg_nx ? ix + 1 : ix;
+            for (int z = max(iz - 1, 0); z <= min(iz + 1, (int)c.cg_nz - 1); ++z) {
+                for (int y = max(iy - 1, 0); y <= min(iy + 1, (int)c.cg_ny - 1); ++y) {
+                    const uint32_t line = c.cg_nx * (y + c.cg_ny * z);
+                    const uint32_t e = d.cg_start[line + xb + 1];
+#pragma unroll 4
+                    for (uint32_t q = d.cg_start[line + xa]; q < e; ++q) {
+                        const float4 xj = __ldg(&d.cg_pos[q]);
+                        const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
+                        const float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
+                        if (!(d2 < c.rc2) || q == mine) continue;
+                        const float cut = cut_of(xj);
+                        const float reach = cut + c.skin_f;
+                        if (c.lgap_f > 0.f && !(d2 < reach * reach)) continue;
+                        if (n < c.KC) {
+                            const float mg = sqrtf(d2) - cut;
+                            const uint32_t b = mg < RF_CB1 * c.skin_f ? 0u : mg < RF_CB2 * c.skin_f ? 1u : mg < RF_CB3 * c.skin_f ? 2u : 3u;
+                            s_c[n][tid] = q;
+                            k0 |= (unsigned long long)(b & 1u) << n;
+                            k1 |= (unsigned long long)(b >> 1) << n;
+                        } else {
+                            raise_status(&d.sc->err, RF_ERR_CAPACITY);
                         }
+                        ++n;
                     }
                 }
             }
         }
         if (n > c.KC) n = c.KC;
         d.cand_n[i] = n;
-        // candidates in the order of their margin bucket (stable within a bucket): a scan
-        // needs no candidate of a bucket whose lower bound the displacements since this
-        // build cannot have closed (scan_limit)
-        {
-            uint32_t jl[64];
-            uint8_t bq[64];
-            uint32_t cnt[4] = {0u, 0u, 0u, 0u};
-            for (uint32_t q = 0; q < n; ++q) {
-                const uint32_t j = d.cand[(size_t)q * c.N + i];
-                const float4 xj = posf(d, c, cur, j);
-                const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
-                const float cut = c.lgap_f > 0.f ? fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) : c.acut_f;
-                const float mg = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz) - cut;
-                const uint32_t b = mg < RF_CB1 * c.skin_f ? 0u : mg < RF_CB2 * c.skin_f ? 1u : mg < RF_CB3 * c.skin_f ? 2u : 3u;
-                jl[q] = j;
-                bq[q] = (uint8_t)b;
-                ++cnt[b];
-            }
-            uint32_t pos[4] = {0u, cnt[0], cnt[0] + cnt[1], cnt[0] + cnt[1] + cnt[2]};
-            d.cbound[i] = pos[1] | (pos[2] << 8) | (pos[3] << 16);
-            for (uint32_t q = 0; q < n; ++q) d.cand[(size_t)(pos[bq[q]]++) * c.N + i] = jl[q];
-        }
-        // membership: candidates already in the row
-        unsigned long long mem = 0ull;
+        unsigned long long in_row = 0ull;                  // candidates already in the row
         uint32_t live = d.live[i];
         while (live) {
             const uint32_t k = __ffs(live) - 1;
             live &= live - 1;
-            const uint32_t j = d.ids[(size_t)i * c.K + k];
+            const uint32_t sj = d.cg_slot[d.ids[(size_t)i * c.K + k]];
             for (uint32_t q = 0; q < n; ++q)
-                if (d.cand[(size_t)q * c.N + i] == j) { mem |= 1ull << q; break; }
+                if (s_c[q][tid] == sj) { in_row |= 1ull << q; break; }
         }
-        d.member[i] = mem;
+        const unsigned long long all = n < 64 ? (1ull << n) - 1ull : ~0ull;
+        const uint32_t n0 = __popcll(~k1 & ~k0 & all), n1 = n0 + __popcll(~k1 & k0 & all), n2 = n1 + __popcll(k1 & ~k0);
+        d.cbound[i] = n0 | (n1 << 8) | (n2 << 16);
+        uint32_t next = (n0 << 8) | (n1 << 16) | (n2 << 24);   // next place of each bucket (bytes; at most 64)
+        unsigned long long mem = 0ull;
         // margin of the nearest non-member candidate: until the displacements since this
         // build add up to it, no candidate can come within its list cutoff
         float mg = 3.0e38f;
         for (uint32_t q = 0; q < n; ++q) {
-            if ((mem >> q) & 1ull) continue;
-            const float4 xj = posf(d, c, cur, d.cand[(size_t)q * c.N + i]);
+            const uint32_t sh = 8u * ((uint32_t)((k0 >> q) & 1ull) + 2u * (uint32_t)((k1 >> q) & 1ull));
+            const uint32_t at = (next >> sh) & 0xFFu, s = s_c[q][tid];
+            next += 1u << sh;
+            d.cand[(size_t)at * c.N + i] = d.cg_sorted[s];
+            if ((in_row >> q) & 1ull) { mem |= 1ull << at; continue; }
+            const float4 xj = __ldg(&d.cg_pos[s]);
             const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
-            const float cut = c.lgap_f > 0.f ? fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) : c.acut_f;
-            mg = fminf(mg, sqrtf(ddx * ddx + ddy * ddy + ddz * ddz) - cut);
+            mg = fminf(mg, sqrtf(ddx * ddx + ddy * ddy + ddz * ddz) - cut_of(xj));
         }
+        d.member[i] = mem;
         d.cmargin[i] = mg;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -496,344 +501,16 @@ __global__ void k_delete_pending(Dev d, Consts c) {
     }
 }
 
-// End of a step: block partial sums of the platen loads (fixed tree, deterministic);
-// the last block to finish does SumForcesULoading (md_results.cu:34-74) and
-// CompressB/U (md_data_types.h:223-293) and sets the graph conditions.
-template <int KIND>
-__device__ __forceinline__ void step_finish(const Dev& d, const Consts& c, double sfb, double sft,
-                                            uint32_t nbroken, uint32_t moved) {
-    DevScalars* sc = d.sc;
-    const uint32_t FULL = 0xffffffffu;
-    // ---- block reductions (fixed tree: deterministic)
-    __shared__ double s_b[4], s_t[4];
-    __shared__ uint32_t s_n[4], s_m[4];
-    __shared__ bool s_last;
-    for (int o = 16; o; o >>= 1) {
-        sfb += __shfl_xor_sync(FULL, sfb, o);
-        sft += __shfl_xor_sync(FULL, sft, o);
-    }
-    const uint32_t wn = __reduce_add_sync(FULL, nbroken), wm = __reduce_or_sync(FULL, moved);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { s_b[w] = sfb; s_t[w] = sft; s_n[w] = wn; s_m[w] = wm; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double b = (s_b[0] + s_b[1]) + (s_b[2] + s_b[3]);
-        const double t = (s_t[0] + s_t[1]) + (s_t[2] + s_t[3]);
-        d.partial[blockIdx.x] = make_double2(b, t);
-        const uint32_t nb = s_n[0] + s_n[1] + s_n[2] + s_n[3];
-        if (nb) atomicAdd(&sc->broken, (unsigned long long)nb);
-        if (s_m[0] | s_m[1] | s_m[2] | s_m[3]) atomicOr(&sc->moved, 1u);
-        __threadfence();
-        const uint32_t ticket = atomicAdd(&sc->block_counter, 1u);
-        s_last = (ticket == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
-
-    // ---- last block: SumForcesULoading (md_results.cu:34-74) and CompressB/U
-    __threadfence();
-    double pb = 0.0, pt = 0.0;
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        const double2 v = __ldcg(&d.partial[b]);
-        pb += v.x; pt += v.y;
-    }
-    for (int o = 16; o; o >>= 1) {
-        pb += __shfl_xor_sync(FULL, pb, o);
-        pt += __shfl_xor_sync(FULL, pt, o);
-    }
-    __syncthreads();
-    if (l == 0) { s_b[w] = pb; s_t[w] = pt; }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    const double sfb_all = (s_b[0] + s_b[1]) + (s_b[2] + s_b[3]);
-    const double sft_all = (s_t[0] + s_t[1]) + (s_t[2] + s_t[3]);
-    sc->block_counter = 0;
-    // curve record and stress
-    const double a1 = (double)sc->_1d_Area;
-    if (sc->curve_n < c.curve_cap) {
-        double* rec = d.curve + 3 * sc->curve_n;
-        rec[0] = (sc->size_d[2] - sc->sz0) / sc->sz0;
-        rec[1] = sfb_all * a1;
-        rec[2] = sft_all * a1;
-    }
-    sc->curve_n += 1;
-    sc->Stress = 0.5 * (fabs(sfb_all) + fabs(sft_all)) * a1;
-    if (!sc->Loading && sc->Stress > sc->MinStress) sc->Loading = 1;
-    if (sc->FractureStress < sc->Stress) {
-        sc->FractureStress = sc->Stress;
-        sc->FractureStrain = (sc->sz0 - sc->size_d[2]) / sc->sz0;
-    }
-    if (sc->Loading && sc->Stress < sc->ZeroStress) sc->Fracture = 1;
-    // CompressU / CompressB (md_data_types.h:223-293)
-    const int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
-    sc->V = (sc->Stress < 1e-9) ? 10.0 * sc->VLoad : sc->VLoad;
-    sc->size_d[ax] += sc->V * c.dt_d;
-    sc->Top += sc->V * c.dt_d;
-    sc->TopR = sc->Top - 2.0 * c.p_r_d;
-    sc->size[ax] = (float)sc->size_d[ax];
-    sc->sized2[ax] = (float)(0.5 * sc->size_d[ax]);
-    sc->center_d[ax] += sc->V * c.dt_d;
-    sc->center[ax] = (float)sc->center_d[ax];
-    sc->Hd2 = sc->sized2[ax];
-    sc->Strain = (sc->size_d[ax] - sc->Size0) / sc->Size0;
-    sc->steps += 1;
-    sc->dmax = sqrtf(__uint_as_float(sc->d2max_next));
-    sc->d2max_next = 0;
-    const bool running = (sc->Strain < sc->MaxStrain) && !sc->Fracture;
-    sc->done = running ? 0u : 1u;
-    const uint32_t mv = sc->moved;
-    sc->moved = 0;
-    sc->rebuild = mv;
-    if (c.use_graph) {
-        cudaGraphSetConditional(c.h_rebuild, mv ? 1u : 0u);
-        cudaGraphSetConditional(c.h_loop, (running && sc->steps < sc->target) ? 1u : 0u);
-    }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts c) {
-    DevScalars* sc = d.sc;
-    // Loop safety: clear the WHILE condition first. Only the last block's finalize,
-    // which runs after every block has passed this point and advances the step
-    // counter towards the target, sets it again, so the device loop always ends.
-    if (c.use_graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c.h_loop, 0u);
-    if (sc->done || sc->steps >= sc->target) return;
-    const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
-    const float4* __restrict__ P = d.pos[cur];
-    const float4* __restrict__ Vv = d.vel[cur];
-    const float4* __restrict__ Wv = d.ang[cur];
-    const uint32_t N = c.N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < N;
-    const uint32_t FULL = 0xffffffffu;
-
-    // platen arguments of this step, as the driver passes them (double -> float)
-    const float Top = (float)sc->Top, Bottom = (float)sc->Bottom, TopR = (float)sc->TopR,
-                BottomR = (float)sc->BottomR, vt = (float)sc->V, RR = sc->RR;
-    rf_float3 cc;
-    cc.x = sc->center[0]; cc.y = sc->center[1]; cc.z = sc->center[2];
-
-    f3 xi = mk3(0.f, 0.f, 0.f), vi = xi, wi = xi;
-    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, bmask = 0;
-    unsigned long long mem = 0ull;
-    uint32_t ncand = 0;
-    if (valid) {
-        xi = f4to3(P[i]); vi = f4to3(Vv[i]); wi = f4to3(Wv[i]);
-        live = d.live[i]; bond = d.bond[i]; cm = d.cmask[i];
-        mem = d.member[i]; ncand = d.cand_n[i];
-        nbq = d.nbq[i]; bmask = d.bmask[i];
-    }
-    const uint32_t live0 = live, bond0 = bond, cm0 = cm, bmask0 = bmask;
-    const unsigned long long mem0 = mem;
-    const size_t QN = (size_t)d.QB * N;
-
-    // ---- bonds: d_CalculateForcesDEM_22 (md_calculateforcesdem3.cu:424-483) over the bond
-    // records in slot order, with the DeleteFarLinks test of each bond slot on the same
-    // gathered position (md_interaction_list_reconstructbpm.cu:141-186). The next record
-    // is fetched while the current one is computed.
-    f3 fsb = mk3(0.f, 0.f, 0.f), msb = fsb;
-    SumTerms bsum{fsb, msb};
-    uint32_t nbroken = 0;
-    {
-        const uint32_t wb = __reduce_or_sync(FULL, bmask);
-        const uint32_t qend = 32u - __clz(wb);
-        uint32_t nj = i;
-        float nil = 0.f;
-        float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0, n2 = n0;
-        if (qend > 0 && (bmask & 1u)) {
-            const size_t s = (size_t)i;
-            nj = __ldg(&d.bj[s]); nil = __ldg(&d.bil[s]);
-            n0 = d.bst[s]; n1 = d.bst[s + QN]; n2 = d.bst[s + 2 * QN];
-        }
-        for (uint32_t q = 0; q < qend; ++q) {
-            const uint32_t j = nj;
-            const float il = nil;
-            const float4 s0 = n0, s1 = n1, s2 = n2;
-            const bool act = (bmask >> q) & 1u;
-            if (q + 1 < qend && ((bmask >> (q + 1)) & 1u)) {
-                const size_t s = (size_t)(q + 1) * N + i;
-                nj = __ldg(&d.bj[s]); nil = __ldg(&d.bil[s]);
-                n0 = d.bst[s]; n1 = d.bst[s + QN]; n2 = d.bst[s + 2 * QN];
-            }
-            if (!act) continue;
-            const size_t s = (size_t)q * N + i;
-            const float4 pj = __ldg(&P[j]), vj = __ldg(&Vv[j]), wj = __ldg(&Wv[j]);
-            const f3 xj = f4to3(pj);
-            const float rr = dist2_rn(xi, xj);
-            if (rr > c.aa_farcut || (double)rr < 1e-10) {
-                delete_slot(d, c, i, d.bk[s], j, ncand, nbq, live, bond, cm, bmask, mem);
-                continue;
-            }
-            const f3 r = mk3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
-            f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
-            f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
-            const bool broke = bond_slot(c.bp, r, vi, f4to3(vj), wi, f4to3(wj), il, rij, oijt, mijn, mijt, bsum);
-            d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
-            d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
-            d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
-            if (broke) { bmask &= ~(1u << q); bond &= ~(1u << d.bk[s]); ++nbroken; }
-        }
-    }
-
-    // ---- type-0 slots, one gather each: the rest of the previous step's DeleteFarLinks,
-    // then d_CalculateForcesDEM_21 (md_calculateforcesdem3.cu:338-422) in slot order
-    // (bonds broken above included). Overlaps are read from this step's buffer and
-    // written to the next one, so the pass can be replayed below if a link added by
-    // this step's list update turns out to be in contact.
-    const uint32_t* row = d.ids + (size_t)i * c.K;
-    const float* oin = d.cO[cur] + (size_t)i * c.K * 3;
-    float* oout = d.cO[nxt] + (size_t)i * c.K * 3;
-    const uint32_t cm_in = cm;
-    const float twoR = 2.0f * c.cp.rP;
-    f3 fsc = mk3(0.f, 0.f, 0.f), msc = fsc;
-    SumTerms csum{fsc, msc};
-    uint32_t cm_out = 0;
-    {
-        uint32_t m = live & ~bond;
-        while (m) {
-            const uint32_t k = __ffs(m) - 1;
-            m &= m - 1;
-            const uint32_t j = row[k];
-            const f3 xj = f4to3(__ldg(&P[j]));
-            const float rr = dist2_rn(xi, xj);
-            if (rr > c.aa_farcut || (double)rr < 1e-10) {
-                delete_slot(d, c, i, k, j, ncand, nbq, live, bond, cm, bmask, mem);
-                continue;
-            }
-            const f3 r = mk3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
-            const float rijm = norm3(r.x, r.y, r.z);
-            if (!(rijm < twoR)) continue;
-            const uint32_t bit = 1u << k;
-            f3 o = (cm_in & bit) ? mk3(oin[3 * k], oin[3 * k + 1], oin[3 * k + 2]) : mk3(0.f, 0.f, 0.f);
-            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, csum);
-            oout[3 * k] = o.x; oout[3 * k + 1] = o.y; oout[3 * k + 2] = o.z;
-            cm_out |= bit;
-        }
-    }
-
-    // ---- add: InteractionListReConstructBPM (md_interaction_list_reconstructbpm.cu:13-46,80-139)
-    // (skipped when no candidate can have come within a_farcut since the build: the scan
-    // would add nothing)
-    bool replay = false;
-    if (valid && !scan_not_needed(d, c, i, xi.x, xi.y, xi.z)) {
-        unsigned long long tried = mem;
-        bool have_cells = false;
-        Octant oc;
-        for (;;) {
-            unsigned long long best = ~0ull;
-            uint32_t best_q = 0;
-            for (uint32_t q = 0; q < ncand; ++q) {
-                if ((tried >> q) & 1ull) continue;
-                const uint32_t j = __ldg(&d.cand[(size_t)q * N + i]);
-                const f3 xj = f4to3(__ldg(&P[j]));
-                const float rr = dist2_rn(xi, xj);
-                if (!(rr < c.aacut && (double)rr > 1e-10)) continue;
-                if (!have_cells) { oc = octant_of(xi, c.g); have_cells = true; }
-                const int rank = octant_rank(oc, ref_cell(xj, c.g));
-                if (rank < 0) continue;
-                const unsigned long long key = ((unsigned long long)rank << 32) | j;
-                if (key < best) { best = key; best_q = q; }
-            }
-            if (best == ~0ull) break;
-            tried |= 1ull << best_q;
-            const uint32_t free = ~live & (c.K >= 32 ? 0xffffffffu : ((1u << c.K) - 1u));
-            if (!free) { raise_status(&sc->err, RF_ERR_ROW_OVERFLOW); continue; }
-            uint32_t k;
-            if (i == 0 && (free & 1u) && (free & ~1u)) k = __ffs(free & ~1u) - 1;   // kdxfree==0 quirk
-            else k = __ffs(free) - 1;
-            const uint32_t j = (uint32_t)(best & 0xffffffffull);
-            d.ids[(size_t)i * c.K + k] = j;
-            live |= 1u << k;
-            mem |= 1ull << best_q;
-            const f3 xj = f4to3(__ldg(&P[j]));
-            if (norm3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z) < twoR) replay = true;
-        }
-    }
-    // A new link already in contact: _21 would have visited it in slot order among the
-    // others, so the contact pass is replayed over the final row from the unchanged
-    // overlaps of this step.
-    if (replay) {
-        fsc = mk3(0.f, 0.f, 0.f); msc = fsc; cm_out = 0;
-        uint32_t m = live & ~bond;
-        while (m) {
-            const uint32_t k = __ffs(m) - 1;
-            m &= m - 1;
-            const uint32_t j = row[k];
-            const f3 xj = f4to3(__ldg(&P[j]));
-            const f3 r = mk3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
-            const float rijm = norm3(r.x, r.y, r.z);
-            if (!(rijm < twoR)) continue;
-            const uint32_t bit = 1u << k;
-            f3 o = (cm & bit) ? mk3(oin[3 * k], oin[3 * k + 1], oin[3 * k + 2]) : mk3(0.f, 0.f, 0.f);
-            contact_pair(c.cp, r, rijm, vi, f4to3(__ldg(&Vv[j])), wi, f4to3(__ldg(&Wv[j])), o, csum);
-            oout[3 * k] = o.x; oout[3 * k + 1] = o.y; oout[3 * k + 2] = o.z;
-            cm_out |= bit;
-        }
-    }
-    cm = cm_out;
-
-    float e2max = 0.f;
-    double sfb = 0.0, sft = 0.0;
-    uint32_t moved = 0;
-    if (valid) {
-        if (live != live0) d.live[i] = live;
-        if (bond != bond0) d.bond[i] = bond;
-        if (cm != cm0) d.cmask[i] = cm;
-        if (mem != mem0) d.member[i] = mem;
-        if (bmask != bmask0) d.bmask[i] = bmask;
-        // F = 0 after the memset, then += _22 sums, then += _21 sums
-        float Fx = 0.0f + fsb.x, Fy = 0.0f + fsb.y, Fz = 0.0f + fsb.z;
-        Fx += fsc.x; Fy += fsc.y; Fz += fsc.z;
-        float Mx = 0.0f + msb.x, My = 0.0f + msb.y, Mz = 0.0f + msb.z;
-        Mx += msc.x; My += msc.y; Mz += msc.z;
-        float Rx = xi.x, Ry = xi.y, Rz = xi.z, Vx = vi.x, Vy = vi.y, Vz = vi.z;
-        if (KIND == RF_TEST_BRAZIL)
-            brazil_particle(Rx, Ry, Rz, Vx, Vy, Vz, Fx, Fy, Fz, cc, RR, Top, Bottom, TopR, BottomR, vt, c.zcut, sfb, sft);
-        else
-            uniaxial_particle(Rx, Ry, Rz, Vz, Fz, cc, RR, Top, Bottom, TopR, BottomR, vt, c.zcut, sfb, sft);
-        // d_CalculateIncrementsDEM (md_calculateincrementsdem.cu:19-49)
-        Vx += __fmul_rn(Fx, c.dtm); Vy += __fmul_rn(Fy, c.dtm); Vz += __fmul_rn(Fz, c.dtm);
-        Rx += __fmul_rn(Vx, c.dt); Ry += __fmul_rn(Vy, c.dt); Rz += __fmul_rn(Vz, c.dt);
-        float Wx = wi.x + __fmul_rn(Mx, c.dtI), Wy = wi.y + __fmul_rn(My, c.dtI), Wz = wi.z + __fmul_rn(Mz, c.dtI);
-        // d_ParallelepipedCutRestriction (md_parallelepipedrestriction.cu:73-159)
-        if (outside_box(Rx, Ry, Rz, c.box_c, c.box_h)) {
-            Rx = c.hp.x; Ry = c.hp.y; Rz = c.hp.z;
-            Vx = 0.f; Vy = 0.f; Vz = 0.f;
-        }
-        d.pos[nxt][i] = make_float4(Rx, Ry, Rz, 0.f);
-        d.vel[nxt][i] = make_float4(Vx, Vy, Vz, 0.f);
-        d.ang[nxt][i] = make_float4(Wx, Wy, Wz, 0.f);
-        const float4 pr = d.pos_ref[i];
-        const float ex = Rx - pr.x, ey = Ry - pr.y, ez = Rz - pr.z;
-        const float e2 = ex * ex + ey * ey + ez * ez;
-        moved = (e2 > c.disp2) ? 1u : 0u;
-        // lists may have missed a neighbour (a particle moved to the hidden point has none)
-        const bool hidden = Rx == c.hp.x && Ry == c.hp.y && Rz == c.hp.z;
-        if (e2 > c.hard2 && !hidden) raise_status(&d.sc->err, RF_ERR_CAPACITY);
-        if (!hidden) e2max = e2;
-    }
-    note_displacement(d, e2max);
-    step_finish<KIND>(d, c, sfb, sft, nbroken, moved);
-}
-
 // ===========================================================================
 // Extended model step: FP64 positions (x, y, z, radius), per-particle mass and
 // inertia from the radius, bond records with an FP64 rest length and their own
-// strengths, contacts with equivalent radius and mass. Same structure and order as
-// k_step; list maintenance compares FP64 squared distances.
+// strengths, contacts with equivalent radius and mass; list maintenance compares FP64
+// squared distances. (The reference model's k_step follows below with the same structure.)
 // ===========================================================================
 // Read-only load of a 32-byte particle record (two 16-byte loads of one sector pair).
 __device__ __forceinline__ double4 ldg_d4(const double4* p) {
     const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
     return make_double4(a.x, a.y, b.x, b.y);
-}
-// A read of three floats that the compiler may not merge with an earlier read of the same
-// address: the value is fetched again (an L1 hit) instead of being held in registers.
-__device__ __forceinline__ f3 reload3(const float4* p) {
-    float x, y, z, w;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(w) : "l"(p));
-    (void)w;
-    return mk3(x, y, z);
 }
 __device__ __forceinline__ double3 dsub(const double4 a, const double4 b) {
     return make_double3(a.x - b.x, a.y - b.y, a.z - b.z);
@@ -986,121 +663,225 @@ __device__ __forceinline__ void brazil_particle_ext(double& Rx, double& Ry, doub
     }
 }
 
-// End of an extended-model step for a batch of specimens. The platen reaction sums of a
-// CTA are kept per specimen (its first and, if it touches one, its second); the last CTA
-// adds each specimen's CTA partials in CTA order and runs SumForcesULoading
-// (md_results.cu:34-74), the fracture test and CompressB/U (md_data_types.h:223-293)
-// for every specimen still running; the loop ends when all are done. With one specimen
-// this is step_finish's arithmetic, sum for sum.
-template <int KIND>
-__device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, double sfb, double sft,
-                                                uint32_t nbroken, uint32_t moved, uint32_t second) {
-    DevScalars* sc = d.sc;
-    const uint32_t FULL = 0xffffffffu;
-    __shared__ double s_b[4], s_t[4], s_b2[4], s_t2[4];
-    __shared__ uint32_t s_n[4], s_m[4];
-    __shared__ bool s_last;
-    double b1 = second ? sfb : 0.0, t1 = second ? sft : 0.0;
-    if (second) { sfb = 0.0; sft = 0.0; }
-    for (int o = 16; o; o >>= 1) {
-        sfb += __shfl_xor_sync(FULL, sfb, o);
-        sft += __shfl_xor_sync(FULL, sft, o);
-        b1 += __shfl_xor_sync(FULL, b1, o);
-        t1 += __shfl_xor_sync(FULL, t1, o);
-    }
-    const uint32_t wn = __reduce_add_sync(FULL, nbroken), wm = __reduce_or_sync(FULL, moved);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { s_b[w] = sfb; s_t[w] = sft; s_b2[w] = b1; s_t2[w] = t1; s_n[w] = wn; s_m[w] = wm; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        d.partial[blockIdx.x] = make_double2((s_b[0] + s_b[1]) + (s_b[2] + s_b[3]), (s_t[0] + s_t[1]) + (s_t[2] + s_t[3]));
-        d.partial2[blockIdx.x] =
-            make_double2((s_b2[0] + s_b2[1]) + (s_b2[2] + s_b2[3]), (s_t2[0] + s_t2[1]) + (s_t2[2] + s_t2[3]));
-        const uint32_t nb = s_n[0] + s_n[1] + s_n[2] + s_n[3];
-        if (nb) atomicAdd(&sc->broken, (unsigned long long)nb);
-        if (s_m[0] | s_m[1] | s_m[2] | s_m[3]) atomicOr(&sc->moved, 1u);
-        __threadfence();
-        const uint32_t ticket = atomicAdd(&sc->block_counter, 1u);
-        s_last = (ticket == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
+// ---------------------------------------------------------------------------
+// End of a step or force pass. A CTA of the extended kernels holds 4 * PW particles (PW per
+// warp). Its warps leave their sums in shared memory and return; the one that arrives last
+// combines them, and the last CTA of a specimen finishes that specimen, so a batch's
+// specimens are finished side by side and nobody waits at a barrier.
+// ---------------------------------------------------------------------------
+// CTAs of a specimen's particles [p0, p1) in CTAs of `n` particles. A CTA touches at most
+// two specimens (each has at least 128 particles): it counts as the second one's too.
+__device__ __forceinline__ uint32_t spec_first_cta(const SpecGeom& G, uint32_t n) { return G.p0 / n; }
+__device__ __forceinline__ uint32_t spec_last_cta(const SpecGeom& G, uint32_t n) { return (G.p1 - 1u) / n; }
+
+// Arrival of one CTA's last warp at specimen s; true (on every lane) for the last CTA.
+__device__ __forceinline__ bool arrive_last(uint32_t* counter, uint32_t expected) {
+    uint32_t t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(counter, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t != expected - 1u) return false;
     __threadfence();
-    bool all_done = true;
-    for (uint32_t s = 0; s < d.nspec; ++s) {
-        DevScalars* S = d.spec + s;
-        const SpecGeom& G = d.geom[s];
-        if (S->done) continue;                               // uniform across the CTA
-        double pb = 0.0, pt = 0.0;
-        for (uint32_t b = G.b0 + threadIdx.x; b <= G.b1; b += blockDim.x) {
-            const double2 v = (d.blk_spec == nullptr || d.blk_spec[b] == s) ? __ldcg(&d.partial[b])
-                                                                             : __ldcg(&d.partial2[b]);
+    return true;
+}
+
+// Platen sums of a specimen: only the CTAs at the platens have any, so a CTA whose sums are
+// zero writes nothing, one that has some sets its bit (nz: the CTA's first specimen, nz2: its
+// second), and the specimen's last CTA reads the bits and the partials behind them, a lane a
+// bit (the platens' CTAs are neighbours in the numbering: whole words of bits), adds them in
+// a fixed order and clears the bits again.
+__device__ __forceinline__ void spec_platen_sums(const Dev& d, const SpecGeom& G, uint32_t n, double& pb, double& pt) {
+    const uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t b0 = spec_first_cta(G, n), b1 = spec_last_cta(G, n), w0 = b0 >> 5, w1 = b1 >> 5;
+    const bool shared0 = b0 * n < G.p0;              // the first CTA's first specimen is the one before
+    pb = 0.0; pt = 0.0;
+    for (uint32_t wb = w0; wb <= w1; wb += 256u) {
+        uint32_t m[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            const uint32_t w = wb + u * 32u + lane;
+            m[u] = w <= w1 ? __ldcg(&d.nz[w]) : 0u;
+            if (w == w0) m[u] &= (0xffffffffu << (b0 & 31u)) & (shared0 ? ~(1u << (b0 & 31u)) : 0xffffffffu);
+            if (w == w1) m[u] &= 0xffffffffu >> (31u - (b1 & 31u));
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            if (m[u]) atomicAnd(&d.nz[wb + u * 32u + lane], ~m[u]);
+            uint32_t has = __ballot_sync(FULL, m[u] != 0u);
+            while (has) {                            // four words' partials in flight
+                double2 v[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    v[t] = make_double2(0.0, 0.0);
+                    if (has) {
+                        const uint32_t l = (uint32_t)__ffs(has) - 1u, bits = __shfl_sync(FULL, m[u], l);
+                        has &= has - 1u;
+                        if ((bits >> lane) & 1u) v[t] = __ldcg(&d.partial[(wb + u * 32u + l) * 32u + lane]);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) { pb += v[t].x; pt += v[t].y; }
+            }
+        }
+    }
+    if (shared0 && lane == 0) {
+        const uint32_t bit = 1u << (b0 & 31u);
+        if (__ldcg(&d.nz2[w0]) & bit) {
+            atomicAnd(&d.nz2[w0], ~bit);
+            const double2 v = __ldcg(&d.partial2[b0]);
             pb += v.x; pt += v.y;
         }
-        for (int o = 16; o; o >>= 1) {
-            pb += __shfl_xor_sync(FULL, pb, o);
-            pt += __shfl_xor_sync(FULL, pt, o);
-        }
-        __syncthreads();
-        if (l == 0) { s_b[w] = pb; s_t[w] = pt; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const double sfb_all = (s_b[0] + s_b[1]) + (s_b[2] + s_b[3]);
-            const double sft_all = (s_t[0] + s_t[1]) + (s_t[2] + s_t[3]);
-            const double a1 = (double)S->_1d_Area;
-            if (S->curve_n < c.curve_cap) {
-                double* rec = d.curve + 3 * ((size_t)s * c.curve_cap + S->curve_n);
-                rec[0] = (S->size_d[2] - S->sz0) / S->sz0;
-                rec[1] = sfb_all * a1;
-                rec[2] = sft_all * a1;
-            }
-            S->curve_n += 1;
-            S->Stress = 0.5 * (fabs(sfb_all) + fabs(sft_all)) * a1;
-            if (!S->Loading && S->Stress > S->MinStress) S->Loading = 1;
-            if (S->FractureStress < S->Stress) {
-                S->FractureStress = S->Stress;
-                S->FractureStrain = (S->sz0 - S->size_d[2]) / S->sz0;
-            }
-            if (S->Loading && S->Stress < S->ZeroStress) S->Fracture = 1;
-            if (S->Loading && S->Stress < S->keep_frac * S->FractureStress) S->Fracture = 1;
-            const int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
-            S->V = (S->Stress < 1e-9) ? 10.0 * S->VLoad : S->VLoad;
-            S->size_d[ax] += S->V * c.dt_d;
-            S->Top += S->V * c.dt_d;
-            S->TopR = S->Top - 2.0 * c.p_r_d;
-            S->size[ax] = (float)S->size_d[ax];
-            S->sized2[ax] = (float)(0.5 * S->size_d[ax]);
-            S->center_d[ax] += S->V * c.dt_d;
-            S->center[ax] = (float)S->center_d[ax];
-            S->Hd2 = S->sized2[ax];
-            S->Strain = (S->size_d[ax] - S->Size0) / S->Size0;
-            S->steps += 1;                                    // the specimen's own step count
-            const bool running = (S->Strain < S->MaxStrain) && !S->Fracture;
-            S->done = running ? 0u : 1u;
-        }
-        __syncthreads();
-        if (!S->done) all_done = false;
     }
-    if (threadIdx.x != 0) return;
-    sc->block_counter = 0;
-    if (d.nspec > 1) sc->steps += 1;                          // (with one specimen sc == spec)
-    sc->dmax = sqrtf(__uint_as_float(sc->d2max_next));
-    sc->d2max_next = 0;
-    sc->done = all_done ? 1u : 0u;
-    const uint32_t mv = sc->moved;
-    sc->moved = 0;
-    sc->rebuild = mv;
-    if (c.use_graph) {
-        cudaGraphSetConditional(c.h_rebuild, mv ? 1u : 0u);
-        cudaGraphSetConditional(c.h_loop, (!all_done && sc->steps < sc->target) ? 1u : 0u);
+    for (int o = 16; o; o >>= 1) {
+        pb += __shfl_xor_sync(FULL, pb, o);
+        pt += __shfl_xor_sync(FULL, pt, o);
+    }
+}
+
+// A specimen's scalar step (one thread): SumForcesULoading (md_results.cu:34-74), the
+// fracture test and CompressB/U (md_data_types.h:223-293) from its platen sums; true while
+// the specimen runs on.
+template <int KIND>
+__device__ __forceinline__ bool spec_scalars(const Dev& d, const Consts& c, DevScalars* S, uint32_t s, double sfb_all,
+                                             double sft_all) {
+    const double a1 = (double)S->_1d_Area;
+    if (S->curve_n < c.curve_cap) {
+        double* rec = d.curve + 3 * ((size_t)s * c.curve_cap + S->curve_n);
+        rec[0] = (S->size_d[2] - S->sz0) / S->sz0;
+        rec[1] = sfb_all * a1;
+        rec[2] = sft_all * a1;
+    }
+    S->curve_n += 1;
+    S->Stress = 0.5 * (fabs(sfb_all) + fabs(sft_all)) * a1;
+    if (!S->Loading && S->Stress > S->MinStress) S->Loading = 1;
+    if (S->FractureStress < S->Stress) {
+        S->FractureStress = S->Stress;
+        S->FractureStrain = (S->sz0 - S->size_d[2]) / S->sz0;
+    }
+    if (S->Loading && S->Stress < S->ZeroStress) S->Fracture = 1;
+    if (S->Loading && S->Stress < S->keep_frac * S->FractureStress) S->Fracture = 1;
+    const int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
+    S->V = (S->Stress < 1e-9) ? 10.0 * S->VLoad : S->VLoad;
+    S->size_d[ax] += S->V * c.dt_d;
+    S->Top += S->V * c.dt_d;
+    S->TopR = S->Top - 2.0 * c.p_r_d;
+    S->size[ax] = (float)S->size_d[ax];
+    S->sized2[ax] = (float)(0.5 * S->size_d[ax]);
+    S->center_d[ax] += S->V * c.dt_d;
+    S->center[ax] = (float)S->center_d[ax];
+    S->Hd2 = S->sized2[ax];
+    S->Strain = (S->size_d[ax] - S->Size0) / S->Size0;
+    S->steps += 1;                                    // the specimen's own step count
+    const bool running = (S->Strain < S->MaxStrain) && !S->Fracture;
+    S->done = running ? 0u : 1u;
+    return running;
+}
+
+// Shared memory of the end of a step: the warps' sums and their arrivals.
+struct FinishSmem {
+    double b[2][4], t[2][4];
+    uint32_t nb[4], mv[4];
+    uint32_t arrived;
+};
+
+template <int KIND, int PW>
+__device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, double sfb, double sft,
+                                                uint32_t nbroken, uint32_t moved, uint32_t sA, bool second,
+                                                FinishSmem& sh) {
+    DevScalars* sc = d.sc;
+    constexpr uint32_t CTA = 4u * PW;
+    const uint32_t FULL = 0xffffffffu;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const bool has = sfb != 0.0 || sft != 0.0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        double b = (second == (q == 1)) ? sfb : 0.0, t = (second == (q == 1)) ? sft : 0.0;
+        if (__any_sync(FULL, has && second == (q == 1)))
+            for (int o = 16; o; o >>= 1) {
+                b += __shfl_xor_sync(FULL, b, o);
+                t += __shfl_xor_sync(FULL, t, o);
+            }
+        if (l == 0) { sh.b[q][w] = b; sh.t[q][w] = t; }
+    }
+    const uint32_t wn = __reduce_add_sync(FULL, nbroken), wm = __reduce_or_sync(FULL, moved);
+    const bool two = __any_sync(FULL, second);
+    uint32_t t = 0;
+    if (l == 0) {
+        sh.nb[w] = wn; sh.mv[w] = wm | (two ? 0x100u : 0u);
+        __threadfence_block();
+        t = atomicAdd(&sh.arrived, 1u);
+    }
+    if (__shfl_sync(FULL, t, 0) != 3u) return;
+    // the CTA's last warp
+    __threadfence_block();
+    const uint32_t mv = sh.mv[0] | sh.mv[1] | sh.mv[2] | sh.mv[3];
+    if (l == 0) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double b = (sh.b[q][0] + sh.b[q][1]) + (sh.b[q][2] + sh.b[q][3]);
+            const double tt = (sh.t[q][0] + sh.t[q][1]) + (sh.t[q][2] + sh.t[q][3]);
+            if (b != 0.0 || tt != 0.0) {
+                (q ? d.partial2 : d.partial)[blockIdx.x] = make_double2(b, tt);
+                atomicOr(&(q ? d.nz2 : d.nz)[blockIdx.x >> 5], 1u << (blockIdx.x & 31u));
+            }
+        }
+        const uint32_t nb = sh.nb[0] + sh.nb[1] + sh.nb[2] + sh.nb[3];
+        if (nb) atomicAdd(&sc->broken, (unsigned long long)nb);
+        if (mv & 0xFFu) atomicOr(&sc->moved, 1u);
+        __threadfence();
+    }
+    __syncwarp();
+    const uint32_t sN = sA + (((mv & 0x100u) && sA + 1u < d.nspec) ? 1u : 0u);
+    for (uint32_t s = sA; s <= sN; ++s) {
+        DevScalars* S = d.spec + s;
+        const SpecGeom& G = d.geom[s];
+        if (!arrive_last(&S->block_counter, spec_last_cta(G, CTA) - spec_first_cta(G, CTA) + 1u)) continue;
+        // (final once the last CTA has arrived; read here, beside the platen sums)
+        uint32_t d2max = 0, moved_any = 0;
+        if (l == 0) { d2max = __ldcg(&sc->d2max_next); moved_any = __ldcg(&sc->moved); }
+        bool running = false;
+        if (!S->done) {
+            double pb, pt;
+            spec_platen_sums(d, G, CTA, pb, pt);
+            if (l == 0) running = spec_scalars<KIND>(d, c, S, s, pb, pt);
+        }
+        if (l == 0) S->block_counter = 0;
+        if (d.nspec > 1) {
+            __threadfence();
+            if (!arrive_last(&sc->spec_counter, d.nspec)) continue;
+            running = false;
+            for (uint32_t q = l; q < d.nspec; q += 32) running = running || !__ldcg(&d.spec[q].done);
+            running = __any_sync(FULL, running);
+            if (l == 0) { d2max = __ldcg(&sc->d2max_next); moved_any = __ldcg(&sc->moved); }
+        }
+        if (l == 0) {
+            const unsigned long long steps = sc->steps + (d.nspec > 1 ? 1u : 0u);    // (with one specimen sc == spec)
+            if (d.nspec > 1) { sc->steps = steps; sc->spec_counter = 0; }
+            sc->dmax = sqrtf(__uint_as_float(d2max));
+            sc->d2max_next = 0;
+            sc->done = running ? 0u : 1u;
+            sc->moved = 0;
+            sc->rebuild = moved_any;
+            if (c.use_graph) {
+                cudaGraphSetConditional(c.h_rebuild, moved_any ? 1u : 0u);
+                cudaGraphSetConditional(c.h_loop, (running && steps < sc->target) ? 1u : 0u);
+            }
+        }
     }
 }
 
 #define FIRE_SUMS 9     // F.v + M.w, |F|^2, |v|^2, |M|^2, |w|^2, sum |f_n|, pair count, platen sums (2)
+#define FIRE_GROUP 64   // CTAs whose partials the last of them adds up before the specimen's last CTA does
 
-template <int KIND>
-__device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c, double (&acc)[FIRE_SUMS],
-                                                  uint32_t second);
+struct FireSmem {
+    double a[2][4][FIRE_SUMS];
+    uint32_t mv[4];
+    uint32_t arrived;
+};
+
+template <int PW>
+__device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c, double (&acc)[FIRE_SUMS], uint32_t sA,
+                                                  bool second, FireSmem& sh);
 
 // MODE 0: explicit step (Verlet increments, platen moving at V). MODE 1: force evaluation
 // of one FIRE iteration: the same forces with the FIRE time step, platens at rest; net
@@ -1108,30 +889,44 @@ __device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c,
 // squared norms and the mean normal pair force are reduced for the FIRE decision.
 // MINB: resident 128-thread CTAs per SM the kernel is compiled for (the register cap);
 // rf_engine_autotune picks among the compiled variants by timing them.
-template <int KIND, int MODE, int MINB = RF_STEP_MIN_BLOCKS>
+// PW: particles of a warp (particles_per_warp). 32 where they fill the GPU, fewer where not:
+// the lanes beyond the particles take part in the record and contact rounds and share the
+// particles' slot and candidate scans, so the chain of a warp (its rounds and scans, one
+// memory latency after another) is shorter, over more warps.
+template <int KIND, int MODE, int MINB = RF_STEP_MIN_BLOCKS, int PW = 32>
 __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
+    constexpr int SUB = 32 / PW;                   // lanes a particle has in the scans
     DevScalars* sc = d.sc;
     if (c.use_graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c.h_loop, 0u);
     if (MODE == 0 && (sc->done || sc->steps >= sc->target)) return;
     if (MODE == 1 && sc->fstop) return;
+    union Finish { FinishSmem step; FireSmem fire; };
+    __shared__ Finish s_fin;
+    if (threadIdx.x == 0) { if (MODE == 0) s_fin.step.arrived = 0u; else s_fin.fire.arrived = 0u; }
+    __syncthreads();
     const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
     const double4* __restrict__ P = d.posd[cur];
     const float4* __restrict__ Vv = d.vel[cur];
     const float4* __restrict__ Wv = d.ang[cur];
     const uint32_t N = c.N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    // specimen of this particle: the CTA's first one, or the next (each specimen has at
-    // least 128 particles, so a CTA touches at most two)
-    const uint32_t sA = d.blk_spec ? (uint32_t)d.blk_spec[blockIdx.x] : 0u;
+    const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
+    const uint32_t pl = lane % PW, sub = lane / PW;            // particle of the warp, share of its scans
+    const uint32_t wbase = (blockIdx.x * 4u + wp) * PW;
+    const uint32_t i = wbase + pl;
+    const bool mine = i < N && (SUB == 1 || sub == 0);         // the lane keeps the particle's state
+    // specimen of this particle: the CTA's first one, or the next
+    uint32_t sA = d.blk_spec ? (uint32_t)d.blk_spec[(blockIdx.x * 4u * PW) >> 7] : 0u;
+    if (d.blk_spec && blockIdx.x * 4u * PW >= d.geom[sA].p1) ++sA;
     const uint32_t sI = (i < N && i >= d.geom[sA].p1) ? sA + 1u : sA;
     const SpecGeom& G = d.geom[sI];
     const DevScalars* S = d.spec + sI;
     // a finished specimen of a batch is frozen: its state is carried to the next buffer
     // (explicit steps: it reached its stop rule; FIRE: its relaxation of this increment stopped)
     const bool frozen = i < N && (MODE == 0 ? S->done != 0 : S->fstop != 0);
-    const bool valid = i < N && !frozen;
+    const bool active = i < N && !frozen;                      // (on every lane of the particle)
+    const bool valid = mine && !frozen;
     const uint32_t FULL = 0xffffffffu;
-    if (frozen) {
+    if (frozen && mine) {
         d.posd[nxt][i] = P[i];
         d.vel[nxt][i] = Vv[i];
         d.ang[nxt][i] = Wv[i];
@@ -1155,44 +950,37 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     }
     float fnabs = 0.f, kt = 0.f, kr = 0.f;
     uint32_t npair = 0;
-
-    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, bmask = 0, ncand = 0;
-    unsigned long long mem = 0ull;
-    if (valid) {
-        live = d.live[i]; bond = d.bond[i]; cm = d.cmask[i];
-        mem = d.member[i]; ncand = d.cand_n[i];
-        nbq = d.nbq[i]; bmask = d.bmask[i];
-    }
+    uint32_t bmask = valid ? d.bmask[i] : 0u;
     const size_t QN = (size_t)d.QB * N;
-
     bool dirty = false;          // live, bond, bmask or member changed
     // bond slots whose pair overlaps: their contact (in parallel with the bond) was taken
     // in the bond pass, with its tangential overlap kept in the slot's contact state
     uint32_t pc = 0;
-    const uint32_t cm0 = cm;
-    constexpr int NA = MODE == 1 ? 9 : 6;         // the particle's bond sums (float)
-    __shared__ float s_acc[4][NA][32];
-    __shared__ uint32_t s_msk[4][10][32];
-    enum { W_LIVE, W_BOND, W_CM, W_BMASK, W_PC, W_NB, W_MEMLO, W_MEMHI, W_NPAIR, W_DIRTY };
+    uint32_t nbroken = 0;
+    f3 fsb = mk3(0.f, 0.f, 0.f), msb = fsb;        // the particle's bond sums
+    uint32_t cm_end = 0, bond_end = 0, del = 0;    // slots whose contact state ends, whose bond broke; deleted records
+    // One record's result is 7 words (FIRE: 10), one contact's 12 (15); CH records are evaluated
+    // before the particles add them.
+    constexpr int CH = PW == 32 ? 128 : 64;
+    constexpr int NR = MODE == 1 ? 10 : 7, NC = MODE == 1 ? 15 : 12;
+    constexpr int BUF = NR * CH > NC * 32 ? NR * CH : NC * 32;
+    __shared__ float s_buf[4][BUF];
     {
         // Bond records, spread over the warp. The warp's active records are listed
         // ordinal-major (every particle's first record, then every second one, ...; lane
         // order within an ordinal), so consecutive lanes read consecutive entries of the
         // [QB][N] record arrays, and in each round every lane takes one record whatever the
-        // 32 particles' bond counts. The lane that takes a record forms its force, moment
-        // and outcome from zero and hands them to the particle's lane through shared
-        // memory; the particle adds them in record order. While the pass runs, each
-        // particle's sums and masks wait in shared memory, leaving the registers to the
-        // record arithmetic. FIRE mode reads the records' increment-start state and the
-        // motion since then.
-        constexpr int NO = MODE == 1 ? 10 : 7;        // words of one record's result
-        __shared__ float s_res[4][NO][32];
+        // particles' bond counts. The lane that takes a record forms its force, moment
+        // and outcome from zero and leaves them in shared memory; after every CH records each
+        // particle adds its own in record order, in registers (added round by round into sums
+        // kept in shared memory, that took a third of a round's time). A pair that overlaps is
+        // only marked in its round; the marked ones of a chunk are then taken side by side
+        // (contacts within the rounds were run for a few lanes at a time). FIRE mode reads the
+        // records' increment-start state and the motion since then.
         __shared__ uint32_t s_q0[4][32], s_qb[4][32];  // per ordinal: first list entry, lanes holding one
         extern __shared__ __align__(16) unsigned char rf_step_smem[];
-        const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
         const uint32_t lt = (1u << lane) - 1u;
-        const uint32_t wbase = i - lane;
-        uint16_t* lst = reinterpret_cast<uint16_t*>(rf_step_smem) + (size_t)wp * 32u * d.QB;
+        uint16_t* lst = reinterpret_cast<uint16_t*>(rf_step_smem) + (size_t)wp * (uint32_t)PW * d.QB;
         const uint32_t qend = 32u - __clz(__reduce_or_sync(FULL, bmask));
         uint32_t T = 0;
         for (uint32_t q = 0; q < qend; ++q) {
@@ -1203,216 +991,219 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
             T += __popc(bal);
         }
         uint32_t rem = bmask;                          // this particle's records not yet added
-#pragma unroll
-        for (int a = 0; a < NA; ++a) s_acc[wp][a][lane] = 0.f;   // (read back after the contact pass)
-        s_msk[wp][W_NB][lane] = 0u;
-        s_msk[wp][W_NPAIR][lane] = 0u;
-        if (T) {
-            s_msk[wp][W_LIVE][lane] = live; s_msk[wp][W_BOND][lane] = bond; s_msk[wp][W_CM][lane] = cm;
-            s_msk[wp][W_BMASK][lane] = bmask; s_msk[wp][W_PC][lane] = 0u;
-            s_msk[wp][W_MEMLO][lane] = (uint32_t)mem; s_msk[wp][W_MEMHI][lane] = (uint32_t)(mem >> 32);
-            s_msk[wp][W_DIRTY][lane] = 0u;
-        }
         __syncwarp();
         const float4* src = MODE == 1 ? d.bst0 : d.bst;
-        for (uint32_t base = 0; base < T; base += 32u) {
-            const uint32_t p = base + lane;
-            if (p < T) {
-                const uint32_t e = lst[p];
-                const uint32_t ol = e & 31u, q = e >> 5, io = wbase + ol;
-                const size_t s = (size_t)q * N + io;
-                // every load of the record is issued before the partner's gathers
-                const uint32_t j = __ldg(&d.bj[s]);
-                const float4 s0 = src[s], s1 = src[s + QN], s2 = src[s + 2 * QN];
-                const float2 str = __ldg(&d.bstr[s]);
-                const double L0 = __ldg(&d.bL0[s]);
-                const uint32_t k = d.bk[s];
-                const double4 xo = ldg_d4(&P[io]);
-                const double4 xj = ldg_d4(&P[j]);
-                const float4 vj = __ldg(&Vv[j]), wj = __ldg(&Wv[j]);
-                const double3 rd = dsub(xj, xo);
-                const double rr = dlen2(rd);
-                uint32_t fl = k << 8;
-                f3 fr = mk3(0.f, 0.f, 0.f), mr = fr;
-                float fnr = 0.f, ktr = 0.f, krr = 0.f;
-                if (rr > bond_cut2_del(c, xo.w, xj.w, L0) || rr < 1e-10) {
-                    fl |= RF_REC_DELETE;
-                    fr.x = __uint_as_float(j);
-                } else {
-                    const float ro = (float)xo.w, rj = (float)xj.w;
-                    // parallel contact (extended model, explicit steps): an overlapping bonded pair
-                    // also carries the Hertz-Mindlin contact, and a broken bond's slot keeps that
-                    // contact's state. Its overlap counts from min(r_i + r_j, L0), so a bond formed
-                    // between overlapping particles is force-free at its rest length. FIRE
-                    // relaxation leaves it out: its state would depend on the path.
-                    const double sr = fmin(xo.w + xj.w, L0);
-                    const bool pcon = MODE == 0 && !c.ref_mode && rr < sr * sr;
-                    BondExt b;
-                    b.kn = c.kn; b.ks = c.ks; b.br = c.br_lambda * fminf(ro, rj);
-                    b.sc = str.x; b.tc = str.y; b.L0 = L0;
-                    if (MODE == 0 && c.ref_mode) {
-                        const float il = __ldg(&d.bil[s]);
-                        b.kn = c.refE * il; b.ks = c.refG * il; b.br = c.ref_br;
-                    }
-                    const f3 r = mk3((float)rd.x, (float)rd.y, (float)rd.z);
-                    f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
-                    f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
-                    bool broke;
-                    if (MODE == 1) {
-                        const double4 xi0 = ldg_d4(&d.x0[io]), ri0 = ldg_d4(&d.rot[io]);
-                        const double4 xj0 = ldg_d4(&d.x0[j]), rj0 = ldg_d4(&d.rot[j]);
-                        const double hx = 0.5 * (ri0.x + rj0.x), hy = 0.5 * (ri0.y + rj0.y), hz = 0.5 * (ri0.z + rj0.z);
-                        const f3 du = mk3((float)(rd.x - (xj0.x - xi0.x) - (hy * rd.z - hz * rd.y)),
-                                          (float)(rd.y - (xj0.y - xi0.y) - (hz * rd.x - hx * rd.z)),
-                                          (float)(rd.z - (xj0.z - xi0.z) - (hx * rd.y - hy * rd.x)));
-                        broke = bond_slot_ext_total(b, r, rr, du, mk3((float)ri0.x, (float)ri0.y, (float)ri0.z),
-                                                    mk3((float)rj0.x, (float)rj0.y, (float)rj0.z), rij, oijt, mijn,
-                                                    mijt, rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr);
+        float* res = s_buf[wp];
+        __shared__ uint8_t s_par[4][CH];               // records of the chunk whose pair overlaps
+        for (uint32_t base = 0; base < T; base += CH) {
+            uint32_t npar = 0;
+            for (uint32_t x0 = 0; x0 < CH && base + x0 < T; x0 += 32u) {
+                const uint32_t x = x0 + lane, p = base + x;
+                bool par = false;
+                if (p < T) {
+                    const uint32_t e = lst[p];
+                    const uint32_t ol = e & 31u, q = e >> 5, io = wbase + ol;
+                    const size_t s = (size_t)q * N + io;
+                    // every load of the record is issued before the partner's gathers
+                    const uint32_t j = __ldg(&d.bj[s]);
+                    const float4 s0 = src[s], s1 = src[s + QN], s2 = src[s + 2 * QN];
+                    const float2 str = __ldg(&d.bstr[s]);
+                    const double L0 = __ldg(&d.bL0[s]);
+                    const uint32_t k = d.bk[s];
+                    const double4 xo = ldg_d4(&P[io]);
+                    const double4 xj = ldg_d4(&P[j]);
+                    const float4 vj = __ldg(&Vv[j]), wj = __ldg(&Wv[j]);
+                    const double3 rd = dsub(xj, xo);
+                    const double rr = dlen2(rd);
+                    uint32_t fl = k << 8;
+                    f3 fr = mk3(0.f, 0.f, 0.f), mr = fr;
+                    float fnr = 0.f, ktr = 0.f, krr = 0.f;
+                    if (rr > bond_cut2_del(c, xo.w, xj.w, L0) || rr < 1e-10) {
+                        fl |= RF_REC_DELETE;
                     } else {
-                        broke = bond_slot_ext(ep, b, r, rr, f4to3(__ldg(&Vv[io])), f4to3(vj), f4to3(__ldg(&Wv[io])),
-                                              f4to3(wj), rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr, c.ref_mode != 0);
+                        const float ro = (float)xo.w, rj = (float)xj.w;
+                        // parallel contact (extended model, explicit steps): an overlapping bonded pair
+                        // also carries the Hertz-Mindlin contact, and a broken bond's slot keeps that
+                        // contact's state. Its overlap counts from min(r_i + r_j, L0), so a bond formed
+                        // between overlapping particles is force-free at its rest length. FIRE
+                        // relaxation leaves it out: its state would depend on the path.
+                        const double sr = fmin(xo.w + xj.w, L0);
+                        par = MODE == 0 && !c.ref_mode && rr < sr * sr;
+                        BondExt b;
+                        b.kn = c.kn; b.ks = c.ks; b.br = c.br_lambda * fminf(ro, rj);
+                        b.sc = str.x; b.tc = str.y; b.L0 = L0;
+                        if (MODE == 0 && c.ref_mode) {
+                            const float il = __ldg(&d.bil[s]);
+                            b.kn = c.refE * il; b.ks = c.refG * il; b.br = c.ref_br;
+                        }
+                        const f3 r = mk3((float)rd.x, (float)rd.y, (float)rd.z);
+                        f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
+                        f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
+                        bool broke;
+                        if (MODE == 1) {
+                            const double4 xi0 = ldg_d4(&d.x0[io]), ri0 = ldg_d4(&d.rot[io]);
+                            const double4 xj0 = ldg_d4(&d.x0[j]), rj0 = ldg_d4(&d.rot[j]);
+                            const double hx = 0.5 * (ri0.x + rj0.x), hy = 0.5 * (ri0.y + rj0.y), hz = 0.5 * (ri0.z + rj0.z);
+                            const f3 du = mk3((float)(rd.x - (xj0.x - xi0.x) - (hy * rd.z - hz * rd.y)),
+                                              (float)(rd.y - (xj0.y - xi0.y) - (hz * rd.x - hx * rd.z)),
+                                              (float)(rd.z - (xj0.z - xi0.z) - (hx * rd.y - hy * rd.x)));
+                            broke = bond_slot_ext_total(b, r, rr, du, mk3((float)ri0.x, (float)ri0.y, (float)ri0.z),
+                                                        mk3((float)rj0.x, (float)rj0.y, (float)rj0.z), rij, oijt, mijn,
+                                                        mijt, rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr);
+                        } else {
+                            broke = bond_slot_ext(ep, b, r, rr, f4to3(__ldg(&Vv[io])), f4to3(vj), f4to3(__ldg(&Wv[io])),
+                                                  f4to3(wj), rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr, c.ref_mode != 0);
+                        }
+                        d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
+                        d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
+                        d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
+                        if (broke) fl |= RF_REC_BROKE;
                     }
-                    d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
-                    d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
-                    d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
-                    if (broke) fl |= RF_REC_BROKE;
-                    if (pcon) {
-                        // the pair's velocities and spins are read again (cache hits) rather
-                        // than held through the bond arithmetic
-                        const size_t so = ((size_t)io * c.K + k) * 3;
-                        const float* oi = d.cO[cur] + so;
-                        // the particle's contacts at the step's start (its own record's
-                        // bit is only cleared after this record is added)
-                        const uint32_t cmo = s_msk[wp][W_CM][ol];
-                        f3 o = ((cmo >> k) & 1u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
-                        if (contact_pair_ext(ep, r, rr, sr, ro, rj, c.cmass * ro * ro * ro, c.cmass * rj * rj * rj,
-                                             reload3(&Vv[io]), reload3(&Vv[j]), reload3(&Wv[io]), reload3(&Wv[j]), o,
-                                             fr, mr, fnr, ktr, krr))
-                            fl |= RF_REC_CLEAR;
-                        float* oo = d.cO[nxt] + so;
-                        oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
-                        fl |= RF_REC_PARALLEL;
-                    }
+                    res[x] = fr.x; res[CH + x] = fr.y; res[2 * CH + x] = fr.z;
+                    res[3 * CH + x] = mr.x; res[4 * CH + x] = mr.y; res[5 * CH + x] = mr.z;
+                    res[6 * CH + x] = __uint_as_float(fl);
+                    if (MODE == 1) { res[7 * CH + x] = fnr; res[8 * CH + x] = ktr; res[9 * CH + x] = krr; }
                 }
-                s_res[wp][0][lane] = fr.x; s_res[wp][1][lane] = fr.y; s_res[wp][2][lane] = fr.z;
-                s_res[wp][3][lane] = mr.x; s_res[wp][4][lane] = mr.y; s_res[wp][5][lane] = mr.z;
-                s_res[wp][6][lane] = __uint_as_float(fl);
-                if (MODE == 1) { s_res[wp][7][lane] = fnr; s_res[wp][8][lane] = ktr; s_res[wp][9][lane] = krr; }
+                if (MODE == 0) {
+                    const uint32_t bal = __ballot_sync(FULL, par);
+                    if (par) s_par[wp][npar + __popc(bal & lt)] = (uint8_t)x;
+                    npar += __popc(bal);
+                }
             }
             __syncwarp();
-            // this particle's records that fell in this round, in record order
+            if (MODE == 0) {
+                for (uint32_t t0 = 0; t0 < npar; t0 += 32u) {
+                    if (t0 + lane < npar) {
+                        const uint32_t x = s_par[wp][t0 + lane], e = lst[base + x], io = wbase + (e & 31u);
+                        const size_t s = (size_t)(e >> 5) * N + io;
+                        const uint32_t j = __ldg(&d.bj[s]), k = d.bk[s];
+                        const double L0 = __ldg(&d.bL0[s]);
+                        const double4 xo = ldg_d4(&P[io]), xj = ldg_d4(&P[j]);
+                        const size_t so = ((size_t)io * c.K + k) * 3;
+                        const float* oi = d.cO[cur] + so;
+                        // (a record's slot is in contact at the step's start until this record is added)
+                        f3 o = ((d.cmask[io] >> k) & 1u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
+                        const f3 wo = f4to3(__ldg(&Wv[io]));
+                        const double3 rd = dsub(xj, xo);
+                        const float ro = (float)xo.w, rj = (float)xj.w;
+                        const ContactTerms ct = contact_terms_ext(
+                            ep, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), fmin(xo.w + xj.w, L0), ro, rj,
+                            c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(__ldg(&Vv[io])), f4to3(__ldg(&Vv[j])), wo,
+                            f4to3(__ldg(&Wv[j])), o);
+                        float* oo = d.cO[nxt] + so;
+                        oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
+                        f3 fr = mk3(res[x], res[CH + x], res[2 * CH + x]);
+                        f3 mr = mk3(res[3 * CH + x], res[4 * CH + x], res[5 * CH + x]);
+                        float u0 = 0.f, u1 = 0.f, u2 = 0.f;    // (FIRE's sums: no contact in parallel there)
+                        add_contact(ct, ro, wo, fr, mr, u0, u1, u2);
+                        res[x] = fr.x; res[CH + x] = fr.y; res[2 * CH + x] = fr.z;
+                        res[3 * CH + x] = mr.x; res[4 * CH + x] = mr.y; res[5 * CH + x] = mr.z;
+                        res[6 * CH + x] = __uint_as_float(__float_as_uint(res[6 * CH + x]) | RF_REC_PARALLEL |
+                                                          (ct.clear ? RF_REC_CLEAR : 0u));
+                    }
+                }
+                __syncwarp();
+            }
+            // this particle's records of the chunk, in record order
             while (rem) {
                 const uint32_t q = __ffs(rem) - 1u;
                 const uint32_t x = s_q0[wp][q] + __popc(s_qb[wp][q] & lt) - base;
-                if (x >= 32u) break;
+                if (x >= (uint32_t)CH) break;
                 rem &= rem - 1u;
-                const uint32_t fl = __float_as_uint(s_res[wp][6][x]);
-                const uint32_t k = (fl >> 8) & 31u;
-                if (fl & RF_REC_DELETE) {
-                    uint32_t lv = s_msk[wp][W_LIVE][lane], bd = s_msk[wp][W_BOND][lane];
-                    uint32_t cmm = s_msk[wp][W_CM][lane], bm = s_msk[wp][W_BMASK][lane];
-                    unsigned long long mm = (unsigned long long)s_msk[wp][W_MEMLO][lane] |
-                                            ((unsigned long long)s_msk[wp][W_MEMHI][lane] << 32);
-                    delete_slot(d, c, i, k, __float_as_uint(s_res[wp][0][x]), d.cand_n[i], d.nbq[i], lv, bd, cmm, bm,
-                                mm);
-                    s_msk[wp][W_LIVE][lane] = lv; s_msk[wp][W_BOND][lane] = bd;
-                    s_msk[wp][W_CM][lane] = cmm; s_msk[wp][W_BMASK][lane] = bm;
-                    s_msk[wp][W_MEMLO][lane] = (uint32_t)mm; s_msk[wp][W_MEMHI][lane] = (uint32_t)(mm >> 32);
-                    s_msk[wp][W_DIRTY][lane] = 1u;
-                    continue;
-                }
-                s_acc[wp][0][lane] += s_res[wp][0][x];
-                s_acc[wp][1][lane] += s_res[wp][1][x];
-                s_acc[wp][2][lane] += s_res[wp][2][x];
-                if (fl & RF_REC_CLEAR) {       // the contact's zero-spin rule clears the moment sum
-                    s_acc[wp][3][lane] = 0.f; s_acc[wp][4][lane] = 0.f; s_acc[wp][5][lane] = 0.f;
-                } else {
-                    s_acc[wp][3][lane] += s_res[wp][3][x];
-                    s_acc[wp][4][lane] += s_res[wp][4][x];
-                    s_acc[wp][5][lane] += s_res[wp][5][x];
-                }
+                const uint32_t fl = __float_as_uint(res[6 * CH + x]);
+                const uint32_t bit = 1u << ((fl >> 8) & 31u);
+                if (fl & RF_REC_DELETE) { del |= 1u << q; continue; }
+                fsb.x += res[x]; fsb.y += res[CH + x]; fsb.z += res[2 * CH + x];
+                msb.x += res[3 * CH + x]; msb.y += res[4 * CH + x]; msb.z += res[5 * CH + x];
+                if (fl & RF_REC_CLEAR) msb = mk3(0.f, 0.f, 0.f);   // the contact's zero-spin rule clears the moment sum
                 if (MODE == 1) {
-                    s_acc[wp][6][lane] += s_res[wp][7][x];
-                    s_acc[wp][7][lane] += s_res[wp][8][x];
-                    s_acc[wp][8][lane] += s_res[wp][9][x];
+                    fnabs += res[7 * CH + x]; kt += res[8 * CH + x]; kr += res[9 * CH + x];
+                    ++npair;
                 }
-                uint32_t np = 1;
-                if (fl & RF_REC_BROKE) {
-                    s_msk[wp][W_BMASK][lane] &= ~(1u << q);
-                    s_msk[wp][W_BOND][lane] &= ~(1u << k);
-                    s_msk[wp][W_NB][lane] += 1u;
-                    s_msk[wp][W_DIRTY][lane] = 1u;
-                }
-                if (fl & RF_REC_PARALLEL) { s_msk[wp][W_PC][lane] |= 1u << k; ++np; }
-                else s_msk[wp][W_CM][lane] &= ~(1u << k);    // not in contact: the parallel contact's state ends
-                if (MODE == 1) s_msk[wp][W_NPAIR][lane] += np;
+                if (fl & RF_REC_BROKE) { bmask &= ~(1u << q); bond_end |= bit; ++nbroken; }
+                if (fl & RF_REC_PARALLEL) pc |= bit;
+                else cm_end |= bit;                    // not in contact: the parallel contact's state ends
             }
             __syncwarp();
         }
-        if (T) {
-            live = s_msk[wp][W_LIVE][lane]; bond = s_msk[wp][W_BOND][lane]; cm = s_msk[wp][W_CM][lane];
-            bmask = s_msk[wp][W_BMASK][lane]; pc = s_msk[wp][W_PC][lane];
-            mem = (unsigned long long)s_msk[wp][W_MEMLO][lane] | ((unsigned long long)s_msk[wp][W_MEMHI][lane] << 32);
-            dirty = s_msk[wp][W_DIRTY][lane] != 0u;
-        }
+    }
+    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, ncand = 0;
+    unsigned long long mem = 0ull;
+    if (valid) {
+        live = d.live[i]; bond = d.bond[i]; cm = d.cmask[i];
+        mem = d.member[i]; ncand = d.cand_n[i];
+        nbq = d.nbq[i];
+    }
+    const uint32_t cm0 = cm;
+    bond &= ~bond_end;
+    cm &= ~cm_end;
+    dirty = (bond_end | del) != 0u;
+    while (del) {
+        const uint32_t q = __ffs(del) - 1u;
+        del &= del - 1u;
+        const size_t s = (size_t)q * N + i;
+        delete_slot(d, c, i, d.bk[s], d.bj[s], ncand, nbq, live, bond, cm, bmask, mem);
     }
 
     // the particle's own position (the bond pass read it through the cache; its velocity
     // and spin are read where they are used)
     double4 xi = make_double4(0, 0, 0, 1);
-    if (valid) xi = P[i];
+    if (active) xi = P[i];
     const float ri = (float)xi.w;
-    const float mi = c.cmass * ri * ri * ri;
     const uint32_t* row = d.ids + (size_t)i * c.K;
-    const float* oin = d.cO[cur] + (size_t)i * c.K * 3;
-    float* oout = d.cO[nxt] + (size_t)i * c.K * 3;
 
-    f3 fsc = mk3(0.f, 0.f, 0.f), msc = fsc;
-    uint32_t cm_out = 0;
-    float fnc = 0.f, ktc = 0.f, krc = 0.f;   // contact force magnitudes and stiffness (recounted on a replay)
-    uint32_t npc = 0;
-    auto contact_pass = [&](bool with_delete) {
-        uint32_t m = live & ~bond & ~pc;
+    // ---- open slots: the previous step's DeleteFarLinks on them, and which of them overlap
+    uint32_t ct = 0;                             // slots in contact
+    {
+        uint32_t m = live & ~bond & ~pc, far = 0;
+        if (SUB > 1) {                           // every SUB-th open slot of the particle
+            uint32_t all = __shfl_sync(FULL, m, pl), q = 0;
+            m = 0;
+            while (all) {
+                if ((q++ % SUB) == sub) m |= all & (0u - all);
+                all &= all - 1u;
+            }
+        }
         while (m) {
             const uint32_t k = __ffs(m) - 1;
             m &= m - 1;
-            const uint32_t j = row[k];
-            const double4 xj = ldg_d4(&P[j]);
-            const double3 rd = dsub(xj, xi);
-            const double rr = dlen2(rd);
-            if (with_delete && (rr > cut2_del(c, xi.w, xj.w) || rr < 1e-10)) {
-                delete_slot(d, c, i, k, j, ncand, nbq, live, bond, cm, bmask, mem);
-                dirty = true;
-                continue;
-            }
-            const float rj = (float)xj.w;
+            const double4 xj = ldg_d4(&P[row[k]]);
+            const double rr = dlen2(dsub(xj, xi));
+            if (rr > cut2_del(c, xi.w, xj.w) || rr < 1e-10) { far |= 1u << k; continue; }
             const double sr = xi.w + xj.w;
-            if (!(rr < sr * sr)) continue;
-            const uint32_t bit = 1u << k;
-            // cm: step-start contacts minus slots deleted this step (a refilled slot starts at zero)
-            f3 o = (cm & bit) ? mk3(oin[3 * k], oin[3 * k + 1], oin[3 * k + 2]) : mk3(0.f, 0.f, 0.f);
-            const f3 r = mk3((float)rd.x, (float)rd.y, (float)rd.z);
-            contact_pair_ext(ep, r, rr, sr, ri, rj, mi, c.cmass * rj * rj * rj, f4to3(__ldg(&Vv[i])),
-                             f4to3(__ldg(&Vv[j])), f4to3(__ldg(&Wv[i])), f4to3(__ldg(&Wv[j])), o, fsc, msc, fnc, ktc,
-                             krc);
-            ++npc;
-            oout[3 * k] = o.x; oout[3 * k + 1] = o.y; oout[3 * k + 2] = o.z;
-            cm_out |= bit;
+            if (rr < sr * sr) ct |= 1u << k;
         }
-    };
-    contact_pass(true);
+#pragma unroll
+        for (int o = PW; o < 32; o <<= 1) {
+            far |= __shfl_xor_sync(FULL, far, o);
+            ct |= __shfl_xor_sync(FULL, ct, o);
+        }
+        if (SUB > 1 && sub) { far = 0; ct = 0; }
+        while (far) {
+            const uint32_t k = __ffs(far) - 1;
+            far &= far - 1;
+            delete_slot(d, c, i, k, row[k], ncand, nbq, live, bond, cm, bmask, mem);
+            dirty = true;
+        }
+    }
 
-    bool replay = false;
-    if (valid && !scan_not_needed(d, c, i, (float)xi.x, (float)xi.y, (float)xi.z)) {
+    // ---- new neighbours, in the reference's insertion order
+    {
+        bool scan = valid && !scan_not_needed(d, c, i, (float)xi.x, (float)xi.y, (float)xi.z);
+        const f3 xif = mk3((float)xi.x, (float)xi.y, (float)xi.z);
+        uint32_t qlim = scan ? scan_limit(d, c, i, xif.x, xif.y, xif.z, ncand) : 0u;
         unsigned long long tried = mem;
+        if (SUB > 1) {                           // the particle's lanes share the candidates
+            scan = __shfl_sync(FULL, (int)scan, pl) != 0;
+            qlim = __shfl_sync(FULL, qlim, pl);
+            tried = __shfl_sync(FULL, tried, pl);
+        }
         bool have_cells = false;
         Octant oc;
-        const f3 xif = mk3((float)xi.x, (float)xi.y, (float)xi.z);
-        const uint32_t qlim = scan_limit(d, c, i, xif.x, xif.y, xif.z, ncand);
-        for (;;) {
+        while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q = 0; q < qlim; ++q) {
+            for (uint32_t q = sub; scan && q < qlim; q += SUB) {
                 if ((tried >> q) & 1ull) continue;
                 const uint32_t j = __ldg(&d.cand[(size_t)q * N + i]);
                 const double4 xj = ldg_d4(&P[j]);
@@ -1424,8 +1215,15 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 const unsigned long long key = ((unsigned long long)rank << 32) | j;
                 if (key < best) { best = key; best_q = q; }
             }
-            if (best == ~0ull) break;
+#pragma unroll
+            for (int o = PW; o < 32; o <<= 1) {
+                const unsigned long long b = __shfl_xor_sync(FULL, best, o);
+                const uint32_t bq = __shfl_xor_sync(FULL, best_q, o);
+                if (b < best) { best = b; best_q = bq; }
+            }
+            if (best == ~0ull) { scan = false; continue; }
             tried |= 1ull << best_q;
+            if (SUB > 1 && sub) continue;
             const uint32_t free = ~live & (c.K >= 32 ? 0xffffffffu : ((1u << c.K) - 1u));
             if (!free) { raise_status(&sc->err, RF_ERR_ROW_OVERFLOW); continue; }
             uint32_t k;
@@ -1438,18 +1236,92 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
             dirty = true;
             const double4 xj = ldg_d4(&P[j]);
             const double sr = xi.w + xj.w;
-            if (dlen2(dsub(xj, xi)) < sr * sr) replay = true;
+            if (dlen2(dsub(xj, xi)) < sr * sr) ct |= 1u << k;      // a new link already in contact
         }
     }
-    if (replay) {
-        fsc = mk3(0.f, 0.f, 0.f); msc = fsc; cm_out = 0; fnc = 0.f; ktc = 0.f; krc = 0.f; npc = 0;
-        contact_pass(false);
+
+    // ---- contacts (_21's pairs), gathered over the warp like the bond records: few particles
+    // have one, so a lane takes one contact of the warp's list and the particle adds its
+    // contacts' terms in slot order
+    f3 fsc = mk3(0.f, 0.f, 0.f), msc = fsc;
+    float fnc = 0.f, ktc = 0.f, krc = 0.f;       // contact force magnitudes and stiffness
+    {
+        __shared__ uint16_t s_ent[4][32];
+        float* res = s_buf[wp];
+        const uint32_t n = __popc(ct);
+        uint32_t rk = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, rk, o);
+            if (lane >= (uint32_t)o) rk += y;
+        }
+        const uint32_t total = __shfl_sync(FULL, rk, 31);
+        rk -= n;
+        uint32_t rem = ct;
+        for (uint32_t base = 0; base < total; base += 32u) {
+            {
+                uint32_t r2 = rem, x = rk;
+                while (r2 && x < base + 32u) {
+                    const uint32_t k = __ffs(r2) - 1u;
+                    r2 &= r2 - 1u;
+                    // cm: step-start contacts minus slots deleted this step (a refilled slot starts at zero)
+                    s_ent[wp][x - base] = (uint16_t)(pl | (k << 5) | (((cm >> k) & 1u) << 10));
+                    ++x;
+                }
+            }
+            __syncwarp();
+            if (base + lane < total) {
+                const uint32_t e = s_ent[wp][lane], io = wbase + (e & 31u), k = (e >> 5) & 31u;
+                const size_t so = (size_t)io * c.K + k;
+                const uint32_t j = d.ids[so];
+                const double4 xo = ldg_d4(&P[io]), xj = ldg_d4(&P[j]);
+                const float* oi = d.cO[cur] + 3 * so;
+                f3 o = (e & 1024u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
+                const double3 rd = dsub(xj, xo);
+                const float ro = (float)xo.w, rj = (float)xj.w;
+                const ContactTerms t =
+                    contact_terms_ext(ep, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), xo.w + xj.w, ro, rj,
+                                      c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(__ldg(&Vv[io])),
+                                      f4to3(__ldg(&Vv[j])), f4to3(__ldg(&Wv[io])), f4to3(__ldg(&Wv[j])), o);
+                float* oo = d.cO[nxt] + 3 * so;
+                oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
+                res[lane] = t.n.x; res[1 * 32 + lane] = t.n.y; res[2 * 32 + lane] = t.n.z;
+                res[3 * 32 + lane] = t.fnd;
+                res[4 * 32 + lane] = t.ft.x; res[5 * 32 + lane] = t.ft.y; res[6 * 32 + lane] = t.ft.z;
+                res[7 * 32 + lane] = t.cr.x; res[8 * 32 + lane] = t.cr.y; res[9 * 32 + lane] = t.cr.z;
+                res[10 * 32 + lane] = t.roll;
+                res[11 * 32 + lane] = t.clear ? 1.f : 0.f;
+                if (MODE == 1) { res[12 * 32 + lane] = t.fn; res[13 * 32 + lane] = t.k1; res[14 * 32 + lane] = t.kt; }
+            }
+            __syncwarp();
+            if (rem && rk < base + 32u) {
+                const f3 wi = f4to3(__ldg(&Wv[i]));
+                while (rem && rk < base + 32u) {
+                    const uint32_t x = rk - base;
+                    rem &= rem - 1u;
+                    ++rk;
+                    ContactTerms t;
+                    t.n = mk3(res[x], res[1 * 32 + x], res[2 * 32 + x]);
+                    t.fnd = res[3 * 32 + x];
+                    t.ft = mk3(res[4 * 32 + x], res[5 * 32 + x], res[6 * 32 + x]);
+                    t.cr = mk3(res[7 * 32 + x], res[8 * 32 + x], res[9 * 32 + x]);
+                    t.roll = res[10 * 32 + x];
+                    t.clear = res[11 * 32 + x] != 0.f;
+                    t.rolling = ep.mur != 0.f;
+                    t.fn = MODE == 1 ? res[12 * 32 + x] : 0.f;
+                    t.k1 = MODE == 1 ? res[13 * 32 + x] : 0.f;
+                    t.kt = MODE == 1 ? res[14 * 32 + x] : 0.f;
+                    add_contact(t, ri, wi, fsc, msc, fnc, ktc, krc);
+                }
+            }
+            __syncwarp();
+        }
+        npair += n;
     }
-    cm = cm_out | pc;
-    fnabs += fnc;
-    npair += npc;
-    kt += ktc;
-    kr += krc;
+    cm = ct | pc;
+    fnabs = fnc + fnabs;
+    kt = ktc + kt;
+    kr = krc + kr;
 
     float e2max = 0.f;
     double sfb = 0.0, sft = 0.0;
@@ -1458,15 +1330,8 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
 #pragma unroll
     for (int q = 0; q < FIRE_SUMS; ++q) acc[q] = 0.0;
     if (valid) {
-        // the bond pass's sums, waiting in shared memory through the contact pass
-        const uint32_t wq = threadIdx.x >> 5, lq = threadIdx.x & 31u;
         const f3 vi = f4to3(Vv[i]), wi = f4to3(Wv[i]);
-        const f3 fsb = mk3(s_acc[wq][0][lq], s_acc[wq][1][lq], s_acc[wq][2][lq]);
-        const f3 msb = mk3(s_acc[wq][3][lq], s_acc[wq][4][lq], s_acc[wq][5][lq]);
-        if (MODE == 1) {
-            fnabs += s_acc[wq][6][lq]; kt += s_acc[wq][7][lq]; kr += s_acc[wq][8][lq];
-            npair += s_msk[wq][W_NPAIR][lq];
-        }
+        const float mi = c.cmass * ri * ri * ri;
         if (dirty) { d.live[i] = live; d.bond[i] = bond; d.member[i] = mem; d.bmask[i] = bmask; }
         if (cm != cm0) d.cmask[i] = cm;
         // platens of this particle's specimen (with the reference constants their
@@ -1532,15 +1397,349 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         if (!hidden) e2max = e2;
         }
     }
-    const uint32_t nbroken = s_msk[threadIdx.x >> 5][W_NB][threadIdx.x & 31u];
     if (MODE == 0) {
         note_displacement(d, e2max);
-        step_finish_ext<KIND>(d, c, sfb, sft, nbroken, moved, sI - sA);
+        step_finish_ext<KIND, PW>(d, c, sfb, sft, nbroken, moved, sA, sI != sA, s_fin.step);
     } else {
         const uint32_t nb = __reduce_add_sync(FULL, nbroken);
-        if ((threadIdx.x & 31) == 0 && nb) atomicAdd(&sc->broken, (unsigned long long)nb);
-        fire_force_finish<KIND>(d, c, acc, sI - sA);
+        if (lane == 0 && nb) atomicAdd(&sc->broken, (unsigned long long)nb);
+        fire_force_finish<PW>(d, c, acc, sA, sI != sA, s_fin.fire);
     }
+}
+
+// The reference model's step. Same structure as the extended model's k_step_ext above (bond
+// records and contacts spread over the warp, PW particles a warp); a record's and a contact's
+// terms are kept apart and added by the particle's lane one by one, as the reference's slot
+// loops add them.
+template <int KIND, int PW>
+__global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts c) {
+    constexpr int SUB = 32 / PW;                   // lanes a particle has in the scans
+    DevScalars* sc = d.sc;
+    // Loop safety: clear the WHILE condition first. Only the last block's finalize,
+    // which runs after every block has passed this point and advances the step
+    // counter towards the target, sets it again, so the device loop always ends.
+    if (c.use_graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c.h_loop, 0u);
+    if (sc->done || sc->steps >= sc->target) return;
+    __shared__ FinishSmem s_fin;
+    if (threadIdx.x == 0) s_fin.arrived = 0u;
+    __syncthreads();
+    const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
+    const float4* __restrict__ P = d.pos[cur];
+    const float4* __restrict__ Vv = d.vel[cur];
+    const float4* __restrict__ Wv = d.ang[cur];
+    const uint32_t N = c.N;
+    const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
+    const uint32_t pl = lane % PW, sub = lane / PW;            // particle of the warp, share of its scans
+    const uint32_t wbase = (blockIdx.x * 4u + wp) * PW;
+    const uint32_t i = wbase + pl;
+    const bool active = i < N;                                 // (on every lane of the particle)
+    const bool valid = active && (SUB == 1 || sub == 0);       // the lane keeps the particle's state
+    const uint32_t FULL = 0xffffffffu;
+    const uint32_t lt = (1u << lane) - 1u;
+
+    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, bmask = 0, ncand = 0;
+    unsigned long long mem = 0ull;
+    if (valid) {
+        live = d.live[i]; bond = d.bond[i]; cm = d.cmask[i];
+        mem = d.member[i]; ncand = d.cand_n[i];
+        nbq = d.nbq[i]; bmask = d.bmask[i];
+    }
+    const uint32_t cm0 = cm;
+    const size_t QN = (size_t)d.QB * N;
+    bool dirty = false;
+    uint32_t nbroken = 0;
+
+    // ---- bonds: d_CalculateForcesDEM_22 (md_calculateforcesdem3.cu:424-483) over the bond
+    // records, with the DeleteFarLinks test of each bond slot on the same gathered position
+    // (md_interaction_list_reconstructbpm.cu:141-186)
+    constexpr int NB = 16, NC = 13;               // words of a record's and of a contact's result
+    __shared__ float s_res[4][NB][32];
+    f3 fsb = mk3(0.f, 0.f, 0.f), msb = fsb;
+    {
+        __shared__ uint32_t s_q0[4][32], s_qb[4][32];
+        extern __shared__ __align__(16) unsigned char rf_step_smem[];
+        uint16_t* lst = reinterpret_cast<uint16_t*>(rf_step_smem) + (size_t)wp * (uint32_t)PW * d.QB;
+        const uint32_t qend = 32u - __clz(__reduce_or_sync(FULL, bmask));
+        uint32_t T = 0;
+        for (uint32_t q = 0; q < qend; ++q) {
+            const bool has = (bmask >> q) & 1u;
+            const uint32_t bal = __ballot_sync(FULL, has);
+            if (has) lst[T + __popc(bal & lt)] = (uint16_t)(lane | (q << 5));
+            if (lane == q) { s_q0[wp][q] = T; s_qb[wp][q] = bal; }
+            T += __popc(bal);
+        }
+        uint32_t rem = bmask;                          // this particle's records not yet added
+        __syncwarp();
+        for (uint32_t base = 0; base < T; base += 32u) {
+            if (base + lane < T) {
+                const uint32_t e = lst[base + lane];
+                const uint32_t q = e >> 5, io = wbase + (e & 31u);
+                const size_t s = (size_t)q * N + io;
+                const uint32_t j = __ldg(&d.bj[s]);
+                const float il = __ldg(&d.bil[s]);
+                const float4 s0 = d.bst[s], s1 = d.bst[s + QN], s2 = d.bst[s + 2 * QN];
+                uint32_t fl = (uint32_t)d.bk[s] << 8;
+                const f3 xo = f4to3(__ldg(&P[io])), vo = f4to3(__ldg(&Vv[io])), wo = f4to3(__ldg(&Wv[io]));
+                const f3 xj = f4to3(__ldg(&P[j])), vj = f4to3(__ldg(&Vv[j])), wj = f4to3(__ldg(&Wv[j]));
+                const float rr = dist2_rn(xo, xj);
+                if (rr > c.aa_farcut || below_1em10(rr)) {
+                    fl |= RF_REC_DELETE;
+                    s_res[wp][0][lane] = __uint_as_float(j);
+                } else {
+                    const f3 r = mk3(xj.x - xo.x, xj.y - xo.y, xj.z - xo.z);
+                    f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
+                    f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
+                    KeepTerms t;
+                    if (bond_slot(c.bp, r, vo, vj, wo, wj, il, rij, oijt, mijn, mijt, t)) fl |= RF_REC_BROKE;
+                    d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
+                    d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
+                    d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        s_res[wp][3 * a][lane] = t.ft[a].x; s_res[wp][3 * a + 1][lane] = t.ft[a].y;
+                        s_res[wp][3 * a + 2][lane] = t.ft[a].z;
+                    }
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        s_res[wp][6 + 3 * a][lane] = t.mt[a].x; s_res[wp][7 + 3 * a][lane] = t.mt[a].y;
+                        s_res[wp][8 + 3 * a][lane] = t.mt[a].z;
+                    }
+                }
+                s_res[wp][15][lane] = __uint_as_float(fl);
+            }
+            __syncwarp();
+            while (rem) {                              // this particle's records of the round, in record order
+                const uint32_t q = __ffs(rem) - 1u;
+                const uint32_t x = s_q0[wp][q] + __popc(s_qb[wp][q] & lt) - base;
+                if (x >= 32u) break;
+                rem &= rem - 1u;
+                const uint32_t fl = __float_as_uint(s_res[wp][15][x]), k = fl >> 8;
+                if (fl & RF_REC_DELETE) {
+                    delete_slot(d, c, i, k, __float_as_uint(s_res[wp][0][x]), ncand, nbq, live, bond, cm, bmask, mem);
+                    dirty = true;
+                    continue;
+                }
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    fsb.x += s_res[wp][3 * a][x]; fsb.y += s_res[wp][3 * a + 1][x]; fsb.z += s_res[wp][3 * a + 2][x];
+                }
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    msb.x += s_res[wp][6 + 3 * a][x]; msb.y += s_res[wp][7 + 3 * a][x]; msb.z += s_res[wp][8 + 3 * a][x];
+                }
+                if (fl & RF_REC_BROKE) { bmask &= ~(1u << q); bond &= ~(1u << k); ++nbroken; dirty = true; }
+            }
+            __syncwarp();
+        }
+    }
+
+    // ---- open slots (bonds broken above included): the rest of the previous step's
+    // DeleteFarLinks, and which of them overlap
+    f3 xi = mk3(0.f, 0.f, 0.f);
+    if (active) xi = f4to3(__ldg(&P[i]));
+    const uint32_t* row = d.ids + (size_t)i * c.K;
+    const float twoR = 2.0f * c.cp.rP;
+    uint32_t ct = 0;                             // slots in contact
+    {
+        uint32_t m = live & ~bond, far = 0;
+        if (SUB > 1) {                           // every SUB-th open slot of the particle
+            uint32_t all = __shfl_sync(FULL, m, pl), q = 0;
+            m = 0;
+            while (all) {
+                if ((q++ % SUB) == sub) m |= all & (0u - all);
+                all &= all - 1u;
+            }
+        }
+        while (m) {
+            const uint32_t k = __ffs(m) - 1;
+            m &= m - 1;
+            const f3 xj = f4to3(__ldg(&P[row[k]]));
+            const float rr = dist2_rn(xi, xj);
+            if (rr > c.aa_farcut || below_1em10(rr)) { far |= 1u << k; continue; }
+            if (norm3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z) < twoR) ct |= 1u << k;
+        }
+#pragma unroll
+        for (int o = PW; o < 32; o <<= 1) {
+            far |= __shfl_xor_sync(FULL, far, o);
+            ct |= __shfl_xor_sync(FULL, ct, o);
+        }
+        if (SUB > 1 && sub) { far = 0; ct = 0; }
+        while (far) {
+            const uint32_t k = __ffs(far) - 1;
+            far &= far - 1;
+            delete_slot(d, c, i, k, row[k], ncand, nbq, live, bond, cm, bmask, mem);
+            dirty = true;
+        }
+    }
+
+    // ---- add: InteractionListReConstructBPM (md_interaction_list_reconstructbpm.cu:13-46,80-139)
+    // (skipped when no candidate can have come within a_farcut since the build: the scan
+    // would add nothing)
+    {
+        bool scan = valid && !scan_not_needed(d, c, i, xi.x, xi.y, xi.z);
+        uint32_t qlim = scan ? scan_limit(d, c, i, xi.x, xi.y, xi.z, ncand) : 0u;
+        unsigned long long tried = mem;
+        if (SUB > 1) {                           // the particle's lanes share the candidates
+            scan = __shfl_sync(FULL, (int)scan, pl) != 0;
+            qlim = __shfl_sync(FULL, qlim, pl);
+            tried = __shfl_sync(FULL, tried, pl);
+        }
+        bool have_cells = false;
+        Octant oc;
+        while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
+            unsigned long long best = ~0ull;
+            uint32_t best_q = 0;
+            for (uint32_t q = sub; scan && q < qlim; q += SUB) {
+                if ((tried >> q) & 1ull) continue;
+                const uint32_t j = __ldg(&d.cand[(size_t)q * N + i]);
+                const f3 xj = f4to3(__ldg(&P[j]));
+                const float rr = dist2_rn(xi, xj);
+                if (!(rr < c.aacut && above_1em10(rr))) continue;
+                if (!have_cells) { oc = octant_of(xi, c.g); have_cells = true; }
+                const int rank = octant_rank(oc, ref_cell(xj, c.g));
+                if (rank < 0) continue;
+                const unsigned long long key = ((unsigned long long)rank << 32) | j;
+                if (key < best) { best = key; best_q = q; }
+            }
+#pragma unroll
+            for (int o = PW; o < 32; o <<= 1) {
+                const unsigned long long b = __shfl_xor_sync(FULL, best, o);
+                const uint32_t bq = __shfl_xor_sync(FULL, best_q, o);
+                if (b < best) { best = b; best_q = bq; }
+            }
+            if (best == ~0ull) { scan = false; continue; }
+            tried |= 1ull << best_q;
+            if (SUB > 1 && sub) continue;
+            const uint32_t free = ~live & (c.K >= 32 ? 0xffffffffu : ((1u << c.K) - 1u));
+            if (!free) { raise_status(&sc->err, RF_ERR_ROW_OVERFLOW); continue; }
+            uint32_t k;
+            if (i == 0 && (free & 1u) && (free & ~1u)) k = __ffs(free & ~1u) - 1;   // kdxfree==0 quirk
+            else k = __ffs(free) - 1;
+            const uint32_t j = (uint32_t)(best & 0xffffffffull);
+            d.ids[(size_t)i * c.K + k] = j;
+            live |= 1u << k;
+            mem |= 1ull << best_q;
+            dirty = true;
+            const f3 xj = f4to3(__ldg(&P[j]));
+            if (norm3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z) < twoR) ct |= 1u << k;    // already in contact
+        }
+    }
+
+    // ---- contacts: d_CalculateForcesDEM_21 (md_calculateforcesdem3.cu:338-422) over the
+    // warp's overlapping type-0 slots, each particle's in slot order. Overlaps are read from
+    // this step's buffer and written to the next one.
+    f3 fsc = mk3(0.f, 0.f, 0.f), msc = fsc;
+    {
+        __shared__ uint16_t s_ent[4][32];
+        uint32_t rk = __popc(ct);
+        const uint32_t n = rk;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, rk, o);
+            if (lane >= (uint32_t)o) rk += y;
+        }
+        const uint32_t total = __shfl_sync(FULL, rk, 31);
+        rk -= n;
+        uint32_t rem = ct;
+        for (uint32_t base = 0; base < total; base += 32u) {
+            {
+                uint32_t r2 = rem, x = rk;
+                while (r2 && x < base + 32u) {
+                    const uint32_t k = __ffs(r2) - 1u;
+                    r2 &= r2 - 1u;
+                    s_ent[wp][x - base] = (uint16_t)(pl | (k << 5) | (((cm >> k) & 1u) << 10));
+                    ++x;
+                }
+            }
+            __syncwarp();
+            if (base + lane < total) {
+                const uint32_t e = s_ent[wp][lane], io = wbase + (e & 31u), k = (e >> 5) & 31u;
+                const size_t so = (size_t)io * c.K + k;
+                const uint32_t j = d.ids[so];
+                const f3 xo = f4to3(__ldg(&P[io])), xj = f4to3(__ldg(&P[j]));
+                const float* oi = d.cO[cur] + 3 * so;
+                f3 o = (e & 1024u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
+                const f3 r = mk3(xj.x - xo.x, xj.y - xo.y, xj.z - xo.z);
+                KeepTerms t;
+                contact_pair(c.cp, r, norm3(r.x, r.y, r.z), f4to3(__ldg(&Vv[io])), f4to3(__ldg(&Vv[j])),
+                             f4to3(__ldg(&Wv[io])), f4to3(__ldg(&Wv[j])), o, t);
+                float* oo = d.cO[nxt] + 3 * so;
+                oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
+                if (t.clear) t.mt[1] = mk3(0.f, 0.f, 0.f);
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    s_res[wp][3 * a][lane] = t.ft[a].x; s_res[wp][3 * a + 1][lane] = t.ft[a].y;
+                    s_res[wp][3 * a + 2][lane] = t.ft[a].z;
+                    s_res[wp][6 + 3 * a][lane] = t.mt[a].x; s_res[wp][7 + 3 * a][lane] = t.mt[a].y;
+                    s_res[wp][8 + 3 * a][lane] = t.mt[a].z;
+                }
+                s_res[wp][NC - 1][lane] = t.clear ? 1.f : 0.f;
+            }
+            __syncwarp();
+            while (rem && rk < base + 32u) {
+                const uint32_t x = rk - base;
+                rem &= rem - 1u;
+                ++rk;
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    fsc.x += s_res[wp][3 * a][x]; fsc.y += s_res[wp][3 * a + 1][x]; fsc.z += s_res[wp][3 * a + 2][x];
+                }
+                if (s_res[wp][NC - 1][x] != 0.f) { msc = mk3(0.f, 0.f, 0.f); continue; }   // zero spin: sum cleared
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    msc.x += s_res[wp][6 + 3 * a][x]; msc.y += s_res[wp][7 + 3 * a][x]; msc.z += s_res[wp][8 + 3 * a][x];
+                }
+            }
+            __syncwarp();
+        }
+    }
+    cm = ct;
+
+    float e2max = 0.f;
+    double sfb = 0.0, sft = 0.0;
+    uint32_t moved = 0;
+    if (valid) {
+        if (dirty) { d.live[i] = live; d.bond[i] = bond; d.member[i] = mem; d.bmask[i] = bmask; }
+        if (cm != cm0) d.cmask[i] = cm;
+        // platen arguments of this step, as the driver passes them (double -> float)
+        const float Top = (float)sc->Top, Bottom = (float)sc->Bottom, TopR = (float)sc->TopR,
+                    BottomR = (float)sc->BottomR, vt = (float)sc->V, RR = sc->RR;
+        rf_float3 cc;
+        cc.x = sc->center[0]; cc.y = sc->center[1]; cc.z = sc->center[2];
+        const f3 vi = f4to3(__ldg(&Vv[i])), wi = f4to3(__ldg(&Wv[i]));
+        // F = 0 after the memset, then += _22 sums, then += _21 sums
+        float Fx = 0.0f + fsb.x, Fy = 0.0f + fsb.y, Fz = 0.0f + fsb.z;
+        Fx += fsc.x; Fy += fsc.y; Fz += fsc.z;
+        float Mx = 0.0f + msb.x, My = 0.0f + msb.y, Mz = 0.0f + msb.z;
+        Mx += msc.x; My += msc.y; Mz += msc.z;
+        float Rx = xi.x, Ry = xi.y, Rz = xi.z, Vx = vi.x, Vy = vi.y, Vz = vi.z;
+        if (KIND == RF_TEST_BRAZIL)
+            brazil_particle(Rx, Ry, Rz, Vx, Vy, Vz, Fx, Fy, Fz, cc, RR, Top, Bottom, TopR, BottomR, vt, c.zcut, sfb, sft);
+        else
+            uniaxial_particle(Rx, Ry, Rz, Vz, Fz, cc, RR, Top, Bottom, TopR, BottomR, vt, c.zcut, sfb, sft);
+        // d_CalculateIncrementsDEM (md_calculateincrementsdem.cu:19-49)
+        Vx += __fmul_rn(Fx, c.dtm); Vy += __fmul_rn(Fy, c.dtm); Vz += __fmul_rn(Fz, c.dtm);
+        Rx += __fmul_rn(Vx, c.dt); Ry += __fmul_rn(Vy, c.dt); Rz += __fmul_rn(Vz, c.dt);
+        float Wx = wi.x + __fmul_rn(Mx, c.dtI), Wy = wi.y + __fmul_rn(My, c.dtI), Wz = wi.z + __fmul_rn(Mz, c.dtI);
+        // d_ParallelepipedCutRestriction (md_parallelepipedrestriction.cu:73-159)
+        if (outside_box(Rx, Ry, Rz, c.box_c, c.box_h)) {
+            Rx = c.hp.x; Ry = c.hp.y; Rz = c.hp.z;
+            Vx = 0.f; Vy = 0.f; Vz = 0.f;
+        }
+        d.pos[nxt][i] = make_float4(Rx, Ry, Rz, 0.f);
+        d.vel[nxt][i] = make_float4(Vx, Vy, Vz, 0.f);
+        d.ang[nxt][i] = make_float4(Wx, Wy, Wz, 0.f);
+        const float4 pr = d.pos_ref[i];
+        const float ex = Rx - pr.x, ey = Ry - pr.y, ez = Rz - pr.z;
+        const float e2 = ex * ex + ey * ey + ez * ez;
+        moved = (e2 > c.disp2) ? 1u : 0u;
+        // lists may have missed a neighbour (a particle moved to the hidden point has none)
+        const bool hidden = Rx == c.hp.x && Ry == c.hp.y && Rz == c.hp.z;
+        if (e2 > c.hard2 && !hidden) raise_status(&d.sc->err, RF_ERR_CAPACITY);
+        if (!hidden) e2max = e2;
+    }
+    note_displacement(d, e2max);
+    step_finish_ext<KIND, PW>(d, c, sfb, sft, nbroken, moved, 0u, false, s_fin);
 }
 
 // The FIRE decision of one specimen from its sums tot (FP64; n its particle count), by
@@ -1590,80 +1789,105 @@ __device__ __forceinline__ void fire_decide(DevScalars* S, const Consts& c, cons
     }
 }
 
-// Block sums of the FIRE accumulators (fixed tree, per specimen); the last block adds
-// each specimen's block partials in block order and makes its FIRE decision.
-template <int KIND>
-__device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c, double (&acc)[FIRE_SUMS],
-                                                  uint32_t second) {
+// The FIRE sums of a force pass: warps to CTA as in step_finish_ext, then in a fixed order the
+// last CTA of every FIRE_GROUP of a specimen's CTAs adds that group's partials and the
+// specimen's last CTA the groups' (a lane's share, then the warp tree), and makes the
+// specimen's FIRE decision. (One CTA adding all partials of a 1M-particle specimen was a
+// tail of 61 dependent rounds of loads.)
+template <int PW>
+__device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c, double (&acc)[FIRE_SUMS], uint32_t sA,
+                                                  bool second, FireSmem& sh) {
     DevScalars* sc = d.sc;
+    constexpr uint32_t CTA = 4u * PW;
     const uint32_t FULL = 0xffffffffu;
-    __shared__ double s_acc[4][FIRE_SUMS], s_acc2[4][FIRE_SUMS];
-    __shared__ bool s_last;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    // a CTA touches at most two specimens: its sums are kept apart per specimen
+    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u;
+    const bool two = __any_sync(FULL, second);
 #pragma unroll
-    for (int q = 0; q < FIRE_SUMS; ++q) {
-        double v = second ? 0.0 : acc[q], v2 = second ? acc[q] : 0.0;
-        for (int o = 16; o; o >>= 1) {
-            v += __shfl_xor_sync(FULL, v, o);
-            v2 += __shfl_xor_sync(FULL, v2, o);
+    for (int q = 0; q < 2; ++q) {
+        if (q == 1 && !two) break;                            // (uniform; read only if a warp has two)
+#pragma unroll
+        for (int k = 0; k < FIRE_SUMS; ++k) {
+            double v = (second == (q == 1)) ? acc[k] : 0.0;
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+            if (l == 0) sh.a[q][w][k] = v;
         }
-        if (l == 0) { s_acc[w][q] = v; s_acc2[w][q] = v2; }
     }
-    __syncthreads();
-    if (threadIdx.x < FIRE_SUMS) {
-        const int q = threadIdx.x;
-        d.fpart[(size_t)blockIdx.x * FIRE_SUMS + q] = (s_acc[0][q] + s_acc[1][q]) + (s_acc[2][q] + s_acc[3][q]);
-        if (d.fpart2)
-            d.fpart2[(size_t)blockIdx.x * FIRE_SUMS + q] =
-                (s_acc2[0][q] + s_acc2[1][q]) + (s_acc2[2][q] + s_acc2[3][q]);
+    uint32_t t = 0;
+    if (l == 0) {
+        if (!two)
+            for (int k = 0; k < FIRE_SUMS; ++k) sh.a[1][w][k] = 0.0;
+        sh.mv[w] = two ? 1u : 0u;
+        __threadfence_block();
+        t = atomicAdd(&sh.arrived, 1u);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    if (__shfl_sync(FULL, t, 0) != 3u) return;
+    __threadfence_block();
+    const bool any2 = (sh.mv[0] | sh.mv[1] | sh.mv[2] | sh.mv[3]) != 0u;
+    if (l < FIRE_SUMS) {
+        d.fpart[(size_t)blockIdx.x * FIRE_SUMS + l] = (sh.a[0][0][l] + sh.a[0][1][l]) + (sh.a[0][2][l] + sh.a[0][3][l]);
+        if (any2)
+            d.fpart2[(size_t)blockIdx.x * FIRE_SUMS + l] =
+                (sh.a[1][0][l] + sh.a[1][1][l]) + (sh.a[1][2][l] + sh.a[1][3][l]);
         __threadfence();
-        s_last = (atomicAdd(&sc->fcounter, 1u) == gridDim.x - 1);
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // the last CTA: per specimen still relaxing, its sums over its CTAs in CTA order, then
-    // its FIRE decision
-    __shared__ double tot[FIRE_SUMS];
-    bool all_stopped = true;
-    for (uint32_t sp = 0; sp < d.nspec; ++sp) {
-        DevScalars* S = d.spec + sp;
-        if (S->fstop) continue;                               // uniform across the CTA
-        const SpecGeom& G = d.geom[sp];
-        // fixed order: each thread a CTA-strided share of the blocks, then the warp trees,
-        // then the four warps
+    __syncwarp();
+    const uint32_t sN = sA + ((any2 && sA + 1u < d.nspec) ? 1u : 0u);
+    for (uint32_t s = sA; s <= sN; ++s) {
+        DevScalars* S = d.spec + s;
+        const SpecGeom& G = d.geom[s];
+        const uint32_t b0 = spec_first_cta(G, CTA), b1 = spec_last_cta(G, CTA);
+        // the specimen's groups follow one another in the group arrays; consecutive specimens'
+        // never meet (the +1 a specimen makes up for the rounding of b0 / FIRE_GROUP)
+        const uint32_t g = (blockIdx.x - b0) / FIRE_GROUP, glast = (b1 - b0) / FIRE_GROUP;
+        const size_t gbase = (size_t)s + b0 / FIRE_GROUP;
+        const uint32_t first = b0 + g * FIRE_GROUP, count = min((uint32_t)FIRE_GROUP, b1 + 1u - first);
+        if (!arrive_last(&d.fgrp_n[gbase + g], count)) continue;
         double v[FIRE_SUMS];
 #pragma unroll
-        for (int q = 0; q < FIRE_SUMS; ++q) v[q] = 0.0;
-        for (uint32_t b = G.b0 + threadIdx.x; b <= G.b1; b += blockDim.x) {
-            const double* src = (d.blk_spec == nullptr || d.blk_spec[b] == sp) ? d.fpart : d.fpart2;
+        for (int k = 0; k < FIRE_SUMS; ++k) v[k] = 0.0;
 #pragma unroll
-            for (int q = 0; q < FIRE_SUMS; ++q) v[q] += __ldcg(&src[(size_t)b * FIRE_SUMS + q]);
+        for (uint32_t u = 0; u < FIRE_GROUP; u += 32u) {
+            const uint32_t b = first + u + l;
+            if (u + l >= count) continue;
+            const double* src = (b * CTA >= G.p0 ? d.fpart : d.fpart2) + (size_t)b * FIRE_SUMS;
+#pragma unroll
+            for (int k = 0; k < FIRE_SUMS; ++k) v[k] += __ldcg(&src[k]);
         }
 #pragma unroll
-        for (int q = 0; q < FIRE_SUMS; ++q) {
-            double x = v[q];
-            for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
-            if (l == 0) s_acc[w][q] = x;
+        for (int k = 0; k < FIRE_SUMS; ++k)
+            for (int o = 16; o; o >>= 1) v[k] += __shfl_xor_sync(FULL, v[k], o);
+        if (l == 0) {
+            d.fgrp_n[gbase + g] = 0u;
+#pragma unroll
+            for (int k = 0; k < FIRE_SUMS; ++k) d.fgrp[(gbase + g) * FIRE_SUMS + k] = v[k];
+            __threadfence();
         }
-        __syncthreads();
-        if (threadIdx.x < FIRE_SUMS) {
-            const int q = threadIdx.x;
-            tot[q] = (s_acc[0][q] + s_acc[1][q]) + (s_acc[2][q] + s_acc[3][q]);
+        __syncwarp();
+        if (!arrive_last(&S->fcounter, glast + 1u)) continue;
+        if (!S->fstop) {
+#pragma unroll
+            for (int k = 0; k < FIRE_SUMS; ++k) v[k] = 0.0;
+            for (uint32_t q = l; q <= glast; q += 32u)
+#pragma unroll
+                for (int k = 0; k < FIRE_SUMS; ++k) v[k] += __ldcg(&d.fgrp[(gbase + q) * FIRE_SUMS + k]);
+#pragma unroll
+            for (int k = 0; k < FIRE_SUMS; ++k)
+                for (int o = 16; o; o >>= 1) v[k] += __shfl_xor_sync(FULL, v[k], o);
+            if (l == 0) fire_decide(S, c, v, G.p1 - G.p0);
         }
-        __syncthreads();
-        if (threadIdx.x == 0) fire_decide(S, c, tot, G.p1 - G.p0);
-        __syncthreads();
-        if (!S->fstop) all_stopped = false;
+        bool running = false;
+        if (l == 0) { S->fcounter = 0u; __threadfence(); }
+        if (d.nspec > 1) {
+            if (!arrive_last(&sc->spec_counter, d.nspec)) continue;
+            for (uint32_t q = l; q < d.nspec; q += 32u) running = running || !__ldcg(&d.spec[q].fstop);
+            running = __any_sync(FULL, running);
+        }
+        if (l == 0) {
+            sc->spec_counter = 0u;
+            sc->steps += 1;                     // buffer parity: the update works on what this pass wrote
+            if (d.nspec > 1) sc->fstop = running ? 0u : 1u;      // (with one specimen sc == spec)
+        }
     }
-    if (threadIdx.x != 0) return;
-    sc->fcounter = 0;
-    sc->steps += 1;                     // buffer parity: the update works on what this pass wrote
-    if (d.nspec > 1) sc->fstop = all_stopped ? 1u : 0u;      // (with one specimen sc == spec)
 }
 
 // FIRE update of one iteration, in place on the buffers the force pass wrote:
@@ -2297,7 +2521,9 @@ struct rf_engine {
     cudaStream_t stream;
     cudaGraph_t graph;
     cudaGraphExec_t exec;
-    uint32_t nblocks;
+    uint32_t nblocks;                      // 128-particle blocks of the per-particle kernels
+    int pw = 32;                           // particles a warp of the step kernel takes
+    uint32_t ncta;                         // CTAs of the step kernel (4 warps each)
     uint32_t cg_nb;
     bool graph_ok;
     std::vector<void*> allocs;
@@ -2331,23 +2557,57 @@ template <class T> rf_status dalloc(rf_engine* e, T** p, size_t n) {
 
 #define TRY(x) do { rf_status s__ = (x); if (s__ != RF_OK) return s__; } while (0)
 
-// Explicit extended-model step kernels compiled for 5, 6 or 8 CTAs per SM.
-void* ext_step_variant(bool brazil, int minb) {
-    switch (minb) {
-        case 8: return brazil ? (void*)k_step_ext<RF_TEST_BRAZIL, 0, 8> : (void*)k_step_ext<RF_TEST_UNIAXIAL, 0, 8>;
-        case 5: return brazil ? (void*)k_step_ext<RF_TEST_BRAZIL, 0, 5> : (void*)k_step_ext<RF_TEST_UNIAXIAL, 0, 5>;
-        default: return brazil ? (void*)k_step_ext<RF_TEST_BRAZIL, 0, 6> : (void*)k_step_ext<RF_TEST_UNIAXIAL, 0, 6>;
+// Explicit extended-model step kernels: compiled for 5, 6 or 8 CTAs per SM at 32 particles a
+// warp; with fewer (specimens that do not fill the GPU) the register cap has nothing to give.
+template <int KIND>
+void* ext_step_kind(int pw, int minb) {
+    switch (pw) {
+        case 4: return (void*)k_step_ext<KIND, 0, RF_STEP_MIN_BLOCKS, 4>;
+        case 8: return (void*)k_step_ext<KIND, 0, RF_STEP_MIN_BLOCKS, 8>;
+        case 16: return (void*)k_step_ext<KIND, 0, RF_STEP_MIN_BLOCKS, 16>;
     }
+    return minb == 8 ? (void*)k_step_ext<KIND, 0, 8> : minb == 5 ? (void*)k_step_ext<KIND, 0, 5> : (void*)k_step_ext<KIND, 0, 6>;
+}
+void* ext_step_variant(const rf_engine* e, int minb) {
+    return e->task.kind == RF_TEST_BRAZIL ? ext_step_kind<RF_TEST_BRAZIL>(e->pw, minb) : ext_step_kind<RF_TEST_UNIAXIAL>(e->pw, minb);
+}
+template <int KIND>
+void* fire_force_kind(int pw) {
+    switch (pw) {
+        case 4: return (void*)k_step_ext<KIND, 1, RF_STEP_MIN_BLOCKS, 4>;
+        case 8: return (void*)k_step_ext<KIND, 1, RF_STEP_MIN_BLOCKS, 8>;
+        case 16: return (void*)k_step_ext<KIND, 1, RF_STEP_MIN_BLOCKS, 16>;
+    }
+    return (void*)k_step_ext<KIND, 1>;
+}
+void* fire_force_kernel(const rf_engine* e) {
+    return e->task.kind == RF_TEST_BRAZIL ? fire_force_kind<RF_TEST_BRAZIL>(e->pw) : fire_force_kind<RF_TEST_UNIAXIAL>(e->pw);
 }
 
-// dynamic shared memory of a step launch: the extended kernel's per-warp record list
-// (32 particles x QB records, 2 bytes each, 4 warps)
-unsigned step_smem(const rf_engine* e) { return e->c.ext ? 4u * 32u * e->d.QB * 2u : 0u; }
+// Particles a warp of the step kernels takes. While all CTAs of a step are resident at once
+// the chain of a warp (its rounds and scans, one memory latency after another) is what a
+// step waits for, and a warp of fewer particles has a shorter one; beyond that the step is a
+// matter of throughput. 8 or 16 as long as their CTAs are resident together, 4 while they are
+// at most three an SM. Measured, us per step at 4 / 8 / 16 / 32 particles a warp, extended
+// model: 900 particles 19 / 21 / 24 / 31, 8k 22 / 23 / 27 / 35, 14k 26 / 25 / 29 / 36, 26k 40 / 30 / 32 /
+// 40, 40k 55 / 44 / 35 / 42, 55k 70 / 48 / 38 / 44, 70k 87 / 63 / 57 / 48; reference model: 570
+// particles 16 / 18 / 21 / 23, 4.6k 17 / 18 / 22 / 27, 17k 28 / 22 / 24 / 28, 36k 41 / 35 / 28 / 32.
+int particles_per_warp(uint32_t N, int sms) {
+    const uint64_t resident = (uint64_t)sms * RF_STEP_MIN_BLOCKS * 4u;      // warps
+    return N <= 4u * (uint64_t)sms * 3u * 4u ? 4 : N <= 8u * resident ? 8 : N <= 16u * resident ? 16 : 32;
+}
 
+// dynamic shared memory of a step launch: the per-warp record list (pw particles x QB
+// records, 2 bytes each, 4 warps)
+unsigned step_smem(const rf_engine* e) { return 4u * (unsigned)e->pw * e->d.QB * 2u; }
+
+template <int KIND>
+void* ref_step_kind(int pw) {
+    return pw == 4 ? (void*)k_step<KIND, 4> : pw == 8 ? (void*)k_step<KIND, 8> : pw == 16 ? (void*)k_step<KIND, 16> : (void*)k_step<KIND, 32>;
+}
 void* step_kernel(const rf_engine* e) {
-    const bool br = e->task.kind == RF_TEST_BRAZIL;
-    if (e->c.ext) return ext_step_variant(br, e->step_minb);
-    return br ? (void*)k_step<RF_TEST_BRAZIL> : (void*)k_step<RF_TEST_UNIAXIAL>;
+    if (e->c.ext) return ext_step_variant(e, e->step_minb);
+    return e->task.kind == RF_TEST_BRAZIL ? ref_step_kind<RF_TEST_BRAZIL>(e->pw) : ref_step_kind<RF_TEST_UNIAXIAL>(e->pw);
 }
 
 rf_status build_graph(rf_engine* e) {
@@ -2401,7 +2661,7 @@ rf_status build_graph(rf_engine* e) {
         {(void*)k_rb_zero, gC, 256},      {(void*)k_rb_bin, gN, 256},
         {(void*)k_rb_scan_sums, e->cg_nb, 1024}, {(void*)k_rb_scan_totals, 1, 32},
         {(void*)k_rb_scan_apply, e->cg_nb, 1024}, {(void*)k_rb_scatter, gN, 256},
-        {(void*)k_rb_cand, (e->c.N + 127) / 128, 128},
+        {(void*)k_rb_cand, (e->c.N + RF_RB_CTA - 1) / RF_RB_CTA, RF_RB_CTA},
     };
     void* fn = step_kernel(e);
     // per step node: Consts with the handle of the IF node that follows it (node parameters
@@ -2433,7 +2693,7 @@ rf_status build_graph(rf_engine* e) {
         sargs[u][0] = &d;
         sargs[u][1] = &cs[u];
         cudaGraphNode_t step;
-        kp = kparams(fn, e->nblocks, 128, sargs[u]);
+        kp = kparams(fn, e->ncta, 128, sargs[u]);
         kp.sharedMemBytes = step_smem(e);
         RF_CUDA(cudaGraphAddKernelNode(&step, body, &last, 1, &kp));
         last = step;
@@ -2485,7 +2745,7 @@ rf_status build_fire_graph(rf_engine* e) {
         {(void*)k_rb_zero, gC, 256},      {(void*)k_rb_bin, gN, 256},
         {(void*)k_rb_scan_sums, e->cg_nb, 1024}, {(void*)k_rb_scan_totals, 1, 32},
         {(void*)k_rb_scan_apply, e->cg_nb, 1024}, {(void*)k_rb_scatter, gN, 256},
-        {(void*)k_rb_cand, (c.N + 127) / 128, 128},
+        {(void*)k_rb_cand, (c.N + RF_RB_CTA - 1) / RF_RB_CTA, RF_RB_CTA},
     };
     cudaGraphNode_t prev = nullptr;
     for (auto& q : seq) {
@@ -2495,8 +2755,7 @@ rf_status build_fire_graph(rf_engine* e) {
         prev = n;
     }
     cudaGraphNode_t fnode, unode;
-    void* ff = (e->task.kind == RF_TEST_BRAZIL) ? (void*)k_step_ext<RF_TEST_BRAZIL, 1> : (void*)k_step_ext<RF_TEST_UNIAXIAL, 1>;
-    kp = kparams(ff, e->nblocks, 128);
+    kp = kparams(fire_force_kernel(e), e->ncta, 128);
     kp.sharedMemBytes = step_smem(e);
     RF_CUDA(cudaGraphAddKernelNode(&fnode, body, &inode, 1, &kp));
     kp = kparams((void*)k_fire_update, e->nblocks, 128);
@@ -2513,7 +2772,7 @@ rf_status launch_stream_fire(rf_engine* e, uint64_t max_iter) {
     c.use_graph = 0;
     const unsigned gN = (c.N + 255) / 256, gC = (c.cg_cells + 1 + 255) / 256;
     cudaStream_t s = e->stream;
-    void* ff = (e->task.kind == RF_TEST_BRAZIL) ? (void*)k_step_ext<RF_TEST_BRAZIL, 1> : (void*)k_step_ext<RF_TEST_UNIAXIAL, 1>;
+    void* ff = fire_force_kernel(e);
     void* args[] = {&d, &c};
     for (uint64_t q = 0; q < max_iter + 1;) {
         for (int u = 0; u < 32; ++u, ++q) {
@@ -2523,8 +2782,8 @@ rf_status launch_stream_fire(rf_engine* e, uint64_t max_iter) {
             k_rb_scan_totals<<<1, 32, 0, s>>>(d, c);
             k_rb_scan_apply<<<e->cg_nb, 1024, 0, s>>>(d, c);
             k_rb_scatter<<<gN, 256, 0, s>>>(d, c);
-            k_rb_cand<<<(c.N + 127) / 128, 128, 0, s>>>(d, c);
-            RF_CUDA(cudaLaunchKernel(ff, dim3(e->nblocks), dim3(128), args, step_smem(e), s));
+            k_rb_cand<<<(c.N + RF_RB_CTA - 1) / RF_RB_CTA, RF_RB_CTA, 0, s>>>(d, c);
+            RF_CUDA(cudaLaunchKernel(ff, dim3(e->ncta), dim3(128), args, step_smem(e), s));
             k_fire_update<<<e->nblocks, 128, 0, s>>>(d, c);
         }
         RF_CHECK_LAUNCH("engine stream FIRE");
@@ -2550,9 +2809,9 @@ rf_status launch_stream_steps(rf_engine* e, uint64_t nsteps) {
         k_rb_scan_totals<<<1, 32, 0, s>>>(d, c);
         k_rb_scan_apply<<<e->cg_nb, 1024, 0, s>>>(d, c);
         k_rb_scatter<<<gN, 256, 0, s>>>(d, c);
-        k_rb_cand<<<(c.N + 127) / 128, 128, 0, s>>>(d, c);
+        k_rb_cand<<<(c.N + RF_RB_CTA - 1) / RF_RB_CTA, RF_RB_CTA, 0, s>>>(d, c);
         void* sargs[] = {&d, &c};
-        if (cudaLaunchKernel(step_kernel(e), dim3(e->nblocks), dim3(128), sargs, step_smem(e), s) != cudaSuccess) break;
+        if (cudaLaunchKernel(step_kernel(e), dim3(e->ncta), dim3(128), sargs, step_smem(e), s) != cudaSuccess) break;
         k_stream_ungate<<<1, 32, 0, s>>>(d);
     }
     RF_CHECK_LAUNCH("engine stream steps");
@@ -2705,6 +2964,11 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
     const uint32_t nspec = bin ? (uint32_t)bin->tasks.size() : 1u;
     c.curve_cap = nspec == 1 ? (1u << 20) : std::max(4096u, (1u << 20) / nspec);   // records per specimen
     e->nblocks = (N + 127) / 128;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+    e->pw = particles_per_warp(N, sms);
+    e->ncta = (N + 4 * e->pw - 1) / (4 * e->pw);
+    const size_t nzw = (e->ncta + 31) / 32;
 
     Dev& d = e->d;
     d.n_particles = N;
@@ -2720,8 +2984,9 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
         (st = dalloc(e, &d.cand, (size_t)c.KC * N)) || (st = dalloc(e, &d.cand_n, N)) || (st = dalloc(e, &d.member, N)) ||
         (st = dalloc(e, &d.pos_ref, N)) || (st = dalloc(e, &d.cmargin, N)) || (st = dalloc(e, &d.cbound, N)) || (st = dalloc(e, &d.cg_key, N)) || (st = dalloc(e, &d.cg_count, cells + 1)) ||
         (st = dalloc(e, &d.cg_start, cells + 1)) || (st = dalloc(e, &d.cg_fill, cells + 1)) ||
-        (st = dalloc(e, &d.cg_bsum, e->cg_nb)) || (st = dalloc(e, &d.cg_sorted, N)) ||
-        (st = dalloc(e, &d.partial, e->nblocks)) || (st = dalloc(e, &d.partial2, e->nblocks)) ||
+        (st = dalloc(e, &d.cg_bsum, e->cg_nb)) || (st = dalloc(e, &d.cg_sorted, N)) || (st = dalloc(e, &d.cg_slot, N)) || (st = dalloc(e, &d.cg_pos, N)) ||
+        (st = dalloc(e, &d.partial, e->ncta)) || (st = dalloc(e, &d.partial2, e->ncta)) ||
+        (st = dalloc(e, &d.nz, nzw)) || (st = dalloc(e, &d.nz2, nzw)) ||
         (st = dalloc(e, &d.curve, 3 * (size_t)c.curve_cap * nspec)) ||
         (st = dalloc(e, &d.sc, 1)) || (st = dalloc(e, &e->counters_dev, 4)))
         return fail(st);
@@ -2742,7 +3007,6 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
             G.box_c = ts.S.center; G.box_h = ts.S.spacesized2; G.hp = ts.S.hidenpoint;
             G.p0 = bin ? bin->p0[q] : 0u;
             G.p1 = bin ? bin->p0[q] + bin->n[q] : N;
-            G.b0 = G.p0 / 128; G.b1 = (G.p1 - 1) / 128;
         }
         SpecGeom* dg = nullptr;
         if ((st = dalloc(e, &dg, nspec))) return fail(st);
@@ -2780,6 +3044,7 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
     // the scalar block is read (step parity) by the row import below: start it at zero
     if (cudaMemsetAsync(d.member, 0, N * sizeof(unsigned long long), s) || cudaMemsetAsync(d.cand_n, 0, N * 4, s) ||
         cudaMemsetAsync(d.cmargin, 0, N * sizeof(float), s) ||
+        cudaMemsetAsync(d.nz, 0, nzw * 4, s) || cudaMemsetAsync(d.nz2, 0, nzw * 4, s) ||
         cudaMemsetAsync(d.sc, 0, sizeof(DevScalars), s))
         return fail(RF_ERR_CUDA);
 
@@ -3085,12 +3350,15 @@ rf_status fire_setup(rf_engine* e) {
     if (e->fire_ready) return RF_OK;
     Dev& d = e->d;
     const uint32_t N = e->c.N;
+    const size_t groups = (size_t)d.nspec + e->ncta / FIRE_GROUP + 1;
     rf_status st;
     if ((st = dalloc(e, &d.frc, N)) || (st = dalloc(e, &d.mom, N)) ||
-        (st = dalloc(e, &d.fpart, (size_t)e->nblocks * FIRE_SUMS)) || (st = dalloc(e, &d.rot, N)) ||
-        (d.nspec > 1 && (st = dalloc(e, &d.fpart2, (size_t)e->nblocks * FIRE_SUMS))) ||
+        (st = dalloc(e, &d.fpart, (size_t)e->ncta * FIRE_SUMS)) || (st = dalloc(e, &d.rot, N)) ||
+        (d.nspec > 1 && (st = dalloc(e, &d.fpart2, (size_t)e->ncta * FIRE_SUMS))) ||
+        (st = dalloc(e, &d.fgrp, groups * FIRE_SUMS)) || (st = dalloc(e, &d.fgrp_n, groups)) ||
         (st = dalloc(e, &d.x0, N)) || (st = dalloc(e, &d.bst0, 3 * (size_t)d.QB * N)))
         return st;
+    RF_CUDA(cudaMemsetAsync(d.fgrp_n, 0, groups * sizeof(uint32_t), e->stream));
     e->cf = e->c;
     if (!getenv("RF_ENGINE_NO_GRAPH")) {
         if (build_fire_graph(e) != RF_OK) { cudaGetLastError(); e->cf.use_graph = 0; }
@@ -3265,7 +3533,7 @@ rf_status rf_engine_autotune(rf_engine* e, int steps, int* choice, float* ms_out
     cudaEventCreate(&a0); cudaEventCreate(&a1);
     cudaError_t ce = cudaSuccess;
     for (int v = 0; v < 3 && !ce; ++v) {
-        void* fn = ext_step_variant(e->task.kind == RF_TEST_BRAZIL, variants[v]);
+        void* fn = ext_step_variant(e, variants[v]);
         for (int rep = 0; rep < 2 && !ce; ++rep) {             // first pass warms up
             ce = restore();
             // candidate lists from the current positions (the engine's first step would build them)
@@ -3277,11 +3545,11 @@ rf_status rf_engine_autotune(rf_engine* e, int steps, int* choice, float* ms_out
             k_rb_scan_totals<<<1, 32, 0, s>>>(d, c);
             k_rb_scan_apply<<<e->cg_nb, 1024, 0, s>>>(d, c);
             k_rb_scatter<<<gN, 256, 0, s>>>(d, c);
-            k_rb_cand<<<(c.N + 127) / 128, 128, 0, s>>>(d, c);
+            k_rb_cand<<<(c.N + RF_RB_CTA - 1) / RF_RB_CTA, RF_RB_CTA, 0, s>>>(d, c);
             k_set_target<<<1, 1, 0, s>>>(d.sc, (unsigned long long)steps);
             cudaEventRecord(a0, s);
             for (int q = 0; q < steps && !ce; ++q)
-                ce = cudaLaunchKernel(fn, dim3(e->nblocks), dim3(128), args, step_smem(e), s);
+                ce = cudaLaunchKernel(fn, dim3(e->ncta), dim3(128), args, step_smem(e), s);
             cudaEventRecord(a1, s);
             if (!ce) ce = cudaEventSynchronize(a1);
             float ms = 0.f;

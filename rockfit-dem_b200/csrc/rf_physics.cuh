@@ -490,12 +490,20 @@ __device__ __forceinline__ bool bond_slot_ext_total(const BondExt& b, const f3 r
 }
 
 // Overlapping pair of the extended model. rr = |r|^2 and sr = r_i + r_j in double, with
-// rr < sr^2; the overlap is (sr^2 - rr) / (sr + |r|). mi, mj are the masses. Returns true
-// when the rolling resistance's zero-spin rule cleared the moment sum ms.
-__device__ __forceinline__ bool contact_pair_ext(const ExtParams& p, const f3 r, const double rr, const double sr,
-                                                 const float ri, const float rj, const float mi, const float mj,
-                                                 const f3 vi, const f3 vj, const f3 wi, const f3 wj, f3& Oijt, f3& fs,
-                                                 f3& ms, float& fnabs, float& kt, float& kr) {
+// rr < sr^2; the overlap is (sr^2 - rr) / (sr + |r|). mi, mj are the masses. The terms go to
+// the particle's sums with add_contact, by the lane that keeps them.
+struct ContactTerms {
+    f3 n;                    // normal and force along it (spring and dashpot)
+    float fnd;
+    f3 ft, cr;               // tangential force, n x ft
+    float roll;              // rolling resistance along the spin (rolling), or the zero-spin clear
+    bool rolling, clear;
+    float fn, k1, kt;        // |f_n|, Kn + Kt, Kt (FIRE: force scale and mass scaling)
+};
+__device__ __forceinline__ ContactTerms contact_terms_ext(const ExtParams& p, const f3 r, const double rr, const double sr,
+                                                          const float ri, const float rj, const float mi, const float mj,
+                                                          const f3 vi, const f3 vj, const f3 wi, const f3 wj, f3& Oijt) {
+    ContactTerms t;
     const float rijm = len_from_sq(rr);
     const float delta = (float)fma(sr, sr, -rr) * __frcp_rn((float)sr + rijm);
     const float inv_rm = __frcp_rn(rijm);
@@ -505,8 +513,8 @@ __device__ __forceinline__ bool contact_pair_ext(const ExtParams& p, const f3 r,
     const float c0 = __fsqrt_rn(Rs * delta);
     const float Kn = 2.0f * p.hm_E * c0;
     const float Kt = 8.0f * p.hm_G * c0;
-    kt += Kn + Kt;                                        // contact stiffness (FIRE mass scaling)
-    kr = fm(Kt, ri * ri, kr);
+    t.k1 = Kn + Kt;
+    t.kt = Kt;
     // relative velocity of the contact point: vj - vi + n x (ri wi + rj wj)
     const float ax = fm(ri, wi.x, rj * wj.x), ay = fm(ri, wi.y, rj * wj.y), az = fm(ri, wi.z, rj * wj.z);
     const float vx = fm(ny, az, fm(-nz, ay, vj.x - vi.x));
@@ -514,9 +522,9 @@ __device__ __forceinline__ bool contact_pair_ext(const ExtParams& p, const f3 r,
     const float vz = fm(nx, ay, fm(-ny, ax, vj.z - vi.z));
     const float vn = dot3(nx, ny, nz, vx, vy, vz);
     const float fn = -delta * Kn * RF_2D3_F;
-    fnabs += fabsf(fn);
-    const float fnd = fm(-1.8257f * p.p_A * vn, __fsqrt_rn(Kn * ms_), fn);
-    fs.x = fm(nx, fnd, fs.x); fs.y = fm(ny, fnd, fs.y); fs.z = fm(nz, fnd, fs.z);
+    t.fn = fabsf(fn);
+    t.n = mk3(nx, ny, nz);
+    t.fnd = fm(-1.8257f * p.p_A * vn, __fsqrt_rn(Kn * ms_), fn);
     const float vtx = fm(-nx, vn, vx), vty = fm(-ny, vn, vy), vtz = fm(-nz, vn, vz);
     // old tangential overlap: onto the tangent plane, back to its old length
     const f3 o = Oijt;
@@ -541,21 +549,29 @@ __device__ __forceinline__ bool contact_pair_ext(const ExtParams& p, const f3 r,
         ftx = fm(vtx, c, ftx); fty = fm(vty, c, fty); ftz = fm(vtz, c, ftz);
     }
     Oijt = mk3(ox, oy, oz);
-    fs.x += ftx; fs.y += fty; fs.z += ftz;
-    ms.x = fm(fm(ny, ftz, -(nz * fty)), ri, ms.x);
-    ms.y = fm(fm(nz, ftx, -(nx * ftz)), ri, ms.y);
-    ms.z = fm(fm(nx, fty, -(ny * ftx)), ri, ms.z);
-    if (p.mur != 0.f) {           // rolling resistance, with the reference's zero-spin clear
+    t.ft = mk3(ftx, fty, ftz);
+    t.cr = mk3(fm(ny, ftz, -(nz * fty)), fm(nz, ftx, -(nx * ftz)), fm(nx, fty, -(ny * ftx)));
+    t.rolling = p.mur != 0.f;     // rolling resistance, with the reference's zero-spin clear
+    t.clear = false;
+    t.roll = 0.f;
+    if (t.rolling) {
         const float wim = dot3(wi.x, wi.y, wi.z, wi.x, wi.y, wi.z);
-        if ((double)wim > 1e-18) {
-            const float cr = -p.mur * fabsf(fn) * __frsqrt_rn(wim);
-            ms.x = fm(wi.x, cr, ms.x); ms.y = fm(wi.y, cr, ms.y); ms.z = fm(wi.z, cr, ms.z);
-        } else {
-            ms = mk3(0.f, 0.f, 0.f);
-            return true;
-        }
+        if ((double)wim > 1e-18) t.roll = -p.mur * fabsf(fn) * __frsqrt_rn(wim);
+        else t.clear = true;
     }
-    return false;
+    return t;
+}
+// Adds a contact's terms to its particle's sums (radius ri, spin wi).
+__device__ __forceinline__ void add_contact(const ContactTerms& t, const float ri, const f3 wi, f3& fs, f3& ms,
+                                            float& fnabs, float& kt, float& kr) {
+    kt += t.k1;                                           // contact stiffness (FIRE mass scaling)
+    kr = fm(t.kt, ri * ri, kr);
+    fnabs += t.fn;
+    fs.x = fm(t.n.x, t.fnd, fs.x); fs.y = fm(t.n.y, t.fnd, fs.y); fs.z = fm(t.n.z, t.fnd, fs.z);
+    fs.x += t.ft.x; fs.y += t.ft.y; fs.z += t.ft.z;
+    ms.x = fm(t.cr.x, ri, ms.x); ms.y = fm(t.cr.y, ri, ms.y); ms.z = fm(t.cr.z, ri, ms.z);
+    if (t.clear) ms = mk3(0.f, 0.f, 0.f);
+    else if (t.rolling) { ms.x = fm(wi.x, t.roll, ms.x); ms.y = fm(wi.y, t.roll, ms.y); ms.z = fm(wi.z, t.roll, ms.z); }
 }
 
 }  // namespace rf
