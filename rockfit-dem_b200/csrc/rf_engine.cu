@@ -128,6 +128,9 @@ struct SpecGeom {
     uint32_t p0, p1;
 };
 
+struct __align__(32) F8 { float4 a, b; };
+struct __align__(32) Rec { float4 s0, s1, s2, k; };     // k: (L0 as a double, tensile, shear strength) or (1/L0, 0, 0, 0)
+
 struct Dev {
     // batch of specimens (one specimen: spec == sc, geom[0], blk_spec == nullptr)
     DevScalars* spec;           // [nspec] per-specimen platen / result scalars
@@ -137,11 +140,8 @@ struct Dev {
     uint32_t *nz, *nz2;         // [CTAs / 32] CTAs whose partial / partial2 was written this step
     uint32_t nspec;
     double4* posd[2];   // extended model: x, y, z (FP64) and radius
-    double* bL0;        // extended model: [QB][N] rest length of each bond record
-    float2* bstr;       // extended model: [QB][N] tensile and shear strength of each bond record
     float4* pos[2];
-    float4* vel[2];
-    float4* ang[2];
+    F8* vw[2];          // [N] velocity and spin of a particle (xyz 0 each): one 32-byte sector, one load
     // rows: slot-major, K slots per particle
     uint32_t* ids;      // [N][K] neighbour id of each occupied slot (row-major: a thread walks its own row)
     float* il;          // [K][N] 1/L0 per slot, as the reference layout keeps it (read out only)
@@ -149,12 +149,14 @@ struct Dev {
     uint32_t* live;     // [N] occupied slots
     uint32_t* bond;     // [N] slots holding an intact bond
     uint32_t* cmask;    // [N] type-0 slots whose overlap may be non-zero
-    // bond records: the bonds of particle i in slot order, ordinal-major [q][i]
-    uint32_t* bj;       // [QB][N] partner id
-    uint8_t* bk;        // [QB][N] slot of the record (0xFF: record retired)
-    float* bil;         // [QB][N] 1/L0
-    float4* bst;        // [3][QB][N] (Rij.xyz Oijt.x) (Oijt.yz Mijn.xy) (Mijn.z Mijt.xyz)
-    float4* bst0;       // bst at the start of the current quasi-static increment (FIRE mode)
+    // bond records: the bonds of particle i in slot order, ordinal-major [q][i]. A record is 64
+    // bytes, (Rij.xyz Oijt.x) (Oijt.yz Mijn.xy) (Mijn.z Mijt.xyz) and what does not change: the
+    // FP64 rest length and the two strengths, or 1/L0 in the reference model. It is read and
+    // written as two whole 32-byte pieces: records of broken bonds in between cost nothing, and
+    // no sector is written in part.
+    Rec* rec;           // [QB][N]
+    Rec* rec0;          // rec at the start of the current quasi-static increment (FIRE mode)
+    uint2* bjk;         // [QB][N] partner id and slot of the record (slot 0xFF: record retired)
     uint32_t* nbq;      // [N] records of the particle
     uint32_t* bmask;    // [N] records holding an intact bond
     // Verlet candidates
@@ -181,6 +183,7 @@ struct Dev {
     double* fgrp;       // [groups][FIRE_SUMS] sums over FIRE_GROUP CTAs of a specimen
     uint32_t* fgrp_n;   // [groups] CTAs of the group that have arrived
     double4* rot;       // [N] accumulated rotation of the increment (sum of w dt)
+    double* xax;        // [N] coordinate along the load axis that the last force pass read
     double4* x0;        // [N] positions at the start of the increment
     unsigned long long n_particles;
     uint32_t QB;
@@ -197,9 +200,32 @@ __device__ __forceinline__ float4 posf(const Dev& d, const Consts& c, uint32_t b
     }
     return d.pos[buf][j];
 }
-__device__ __forceinline__ void zero_record(const Dev& d, size_t QN, size_t s) {
+// 32-byte loads and stores (one instruction each on sm_100).
+__device__ __forceinline__ F8 ldg8(const F8* p) {
+    F8 v;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y), "=f"(v.b.z), "=f"(v.b.w)
+        : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void ld8(const void* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st8(void* p, const float4 a, const float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+                 "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ double rec_L0(const float4 k) { return __hiloint2double(__float_as_int(k.y), __float_as_int(k.x)); }
+__device__ __forceinline__ float4 rec_const(double L0, const float2 str) {
+    return make_float4(__int_as_float(__double2loint(L0)), __int_as_float(__double2hiint(L0)), str.x, str.y);
+}
+__device__ __forceinline__ void zero_record(const Dev& d, size_t s) {     // the state; the constants stay
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    d.bst[s] = z; d.bst[s + QN] = z; d.bst[s + 2 * QN] = z;
+    d.rec[s].s0 = z; d.rec[s].s1 = z; d.rec[s].s2 = z;
 }
 
 // ---------------------------------------------------------------------------
@@ -313,7 +339,7 @@ __global__ void k_rb_scatter(Dev d, Consts c) {
 // run of float4 records, nine runs a particle) and the candidates wait in shared memory, as
 // places in that order, until their buckets and the row's members are known; a row member
 // is found by its place. 4M particles: 3.0 ms with an id and a position gathered for
-// every occupant and the list ordered and matched in memory, RB_AFTER ms so.
+// every occupant and the list ordered and matched in memory, 2.5 ms so.
 #define RF_RB_CTA 128
 __global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
     if (gate_closed(d, c)) return;
@@ -405,9 +431,9 @@ __device__ __forceinline__ void retire_record(const Dev& d, const Consts& c, uin
     const uint32_t N = c.N;
     for (uint32_t q = 0; q < nbq; ++q) {
         const size_t s = (size_t)q * N + i;
-        if (d.bk[s] == (uint8_t)k) {
-            d.bk[s] = 0xFF;
-            zero_record(d, (size_t)d.QB * N, s);
+        if (d.bjk[s].y == k) {
+            d.bjk[s].y = 0xFFu;
+            zero_record(d, s);
             bmask &= ~(1u << q);
             return;
         }
@@ -507,10 +533,11 @@ __global__ void k_delete_pending(Dev d, Consts c) {
 // strengths, contacts with equivalent radius and mass; list maintenance compares FP64
 // squared distances. (The reference model's k_step follows below with the same structure.)
 // ===========================================================================
-// Read-only load of a 32-byte particle record (two 16-byte loads of one sector pair).
+// Read-only load of a particle's 32-byte position and radius.
 __device__ __forceinline__ double4 ldg_d4(const double4* p) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ double3 dsub(const double4 a, const double4 b) {
     return make_double3(a.x - b.x, a.y - b.y, a.z - b.z);
@@ -552,7 +579,7 @@ __device__ __forceinline__ double bond_cut2_del(const Consts& c, double ri, doub
 __device__ __forceinline__ double slot_rest_length(const Dev& d, const Consts& c, uint32_t i, uint32_t k, uint32_t nbq) {
     for (uint32_t q = 0; q < nbq; ++q) {
         const size_t s = (size_t)q * c.N + i;
-        if (d.bk[s] == (uint8_t)k) return d.bL0[s];
+        if (d.bjk[s].y == k) return rec_L0(d.rec[s].k);
     }
     return 0.0;
 }
@@ -883,6 +910,22 @@ template <int PW>
 __device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c, double (&acc)[FIRE_SUMS], uint32_t sA,
                                                   bool second, FireSmem& sh);
 
+// A bond record in a FIRE pass: its state at the increment's start (in rij, oijt, mijn, mijt)
+// carried to the current configuration by the pair's motion since then.
+__device__ __forceinline__ bool fire_bond(const Dev& d, const BondExt& b, uint32_t i, uint32_t j, const f3 r, const double3 rd,
+                                          const double rr, f3& rij, f3& oijt, f3& mijn, f3& mijt, f3& fr, f3& mr,
+                                          float& fnr, float& ktr, float& krr) {
+    const double4 xi0 = ldg_d4(&d.x0[i]), ri0 = ldg_d4(&d.rot[i]);
+    const double4 xj0 = ldg_d4(&d.x0[j]), rj0 = ldg_d4(&d.rot[j]);
+    const double hx = 0.5 * (ri0.x + rj0.x), hy = 0.5 * (ri0.y + rj0.y), hz = 0.5 * (ri0.z + rj0.z);
+    const f3 du = mk3((float)(rd.x - (xj0.x - xi0.x) - (hy * rd.z - hz * rd.y)),
+                      (float)(rd.y - (xj0.y - xi0.y) - (hz * rd.x - hx * rd.z)),
+                      (float)(rd.z - (xj0.z - xi0.z) - (hx * rd.y - hy * rd.x)));
+    return bond_slot_ext_total(b, r, rr, du, mk3((float)ri0.x, (float)ri0.y, (float)ri0.z),
+                               mk3((float)rj0.x, (float)rj0.y, (float)rj0.z), rij, oijt, mijn, mijt, rij, oijt, mijn, mijt,
+                               fr, mr, fnr, ktr, krr);
+}
+
 // MODE 0: explicit step (Verlet increments, platen moving at V). MODE 1: force evaluation
 // of one FIRE iteration: the same forces with the FIRE time step, platens at rest; net
 // force and moment are stored for k_fire_update and FP64 sums of the FIRE power, the
@@ -906,8 +949,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     __syncthreads();
     const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
     const double4* __restrict__ P = d.posd[cur];
-    const float4* __restrict__ Vv = d.vel[cur];
-    const float4* __restrict__ Wv = d.ang[cur];
+    const F8* __restrict__ VW = d.vw[cur];
     const uint32_t N = c.N;
     const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
     const uint32_t pl = lane % PW, sub = lane / PW;            // particle of the warp, share of its scans
@@ -928,8 +970,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     const uint32_t FULL = 0xffffffffu;
     if (frozen && mine) {
         d.posd[nxt][i] = P[i];
-        d.vel[nxt][i] = Vv[i];
-        d.ang[nxt][i] = Wv[i];
+        d.vw[nxt][i] = VW[i];
         const float* oi = d.cO[cur] + (size_t)i * c.K * 3;
         float* oo = d.cO[nxt] + (size_t)i * c.K * 3;
         uint32_t m = d.cmask[i];
@@ -951,7 +992,6 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     float fnabs = 0.f, kt = 0.f, kr = 0.f;
     uint32_t npair = 0;
     uint32_t bmask = valid ? d.bmask[i] : 0u;
-    const size_t QN = (size_t)d.QB * N;
     bool dirty = false;          // live, bond, bmask or member changed
     // bond slots whose pair overlaps: their contact (in parallel with the bond) was taken
     // in the bond pass, with its tangential overlap kept in the slot's contact state
@@ -992,7 +1032,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         }
         uint32_t rem = bmask;                          // this particle's records not yet added
         __syncwarp();
-        const float4* src = MODE == 1 ? d.bst0 : d.bst;
+        const Rec* src = MODE == 1 ? d.rec0 : d.rec;
         float* res = s_buf[wp];
         __shared__ uint8_t s_par[4][CH];               // records of the chunk whose pair overlaps
         for (uint32_t base = 0; base < T; base += CH) {
@@ -1005,17 +1045,18 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                     const uint32_t ol = e & 31u, q = e >> 5, io = wbase + ol;
                     const size_t s = (size_t)q * N + io;
                     // every load of the record is issued before the partner's gathers
-                    const uint32_t j = __ldg(&d.bj[s]);
-                    const float4 s0 = src[s], s1 = src[s + QN], s2 = src[s + 2 * QN];
-                    const float2 str = __ldg(&d.bstr[s]);
-                    const double L0 = __ldg(&d.bL0[s]);
-                    const uint32_t k = d.bk[s];
+                    const uint2 jk = d.bjk[s];
+                    float4 s0, s1, s2, kc;
+                    ld8(&src[s].s0, s0, s1);
+                    ld8(&src[s].s2, s2, kc);
+                    const uint32_t j = jk.x;
                     const double4 xo = ldg_d4(&P[io]);
                     const double4 xj = ldg_d4(&P[j]);
-                    const float4 vj = __ldg(&Vv[j]), wj = __ldg(&Wv[j]);
+                    const F8 vwj = ldg8(&VW[j]);
+                    const double L0 = rec_L0(kc);
                     const double3 rd = dsub(xj, xo);
                     const double rr = dlen2(rd);
-                    uint32_t fl = k << 8;
+                    uint32_t fl = jk.y << 8;
                     f3 fr = mk3(0.f, 0.f, 0.f), mr = fr;
                     float fnr = 0.f, ktr = 0.f, krr = 0.f;
                     if (rr > bond_cut2_del(c, xo.w, xj.w, L0) || rr < 1e-10) {
@@ -1031,9 +1072,9 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                         par = MODE == 0 && !c.ref_mode && rr < sr * sr;
                         BondExt b;
                         b.kn = c.kn; b.ks = c.ks; b.br = c.br_lambda * fminf(ro, rj);
-                        b.sc = str.x; b.tc = str.y; b.L0 = L0;
+                        b.sc = kc.z; b.tc = kc.w; b.L0 = L0;
                         if (MODE == 0 && c.ref_mode) {
-                            const float il = __ldg(&d.bil[s]);
+                            const float il = (float)(1.0 / L0);
                             b.kn = c.refE * il; b.ks = c.refG * il; b.br = c.ref_br;
                         }
                         const f3 r = mk3((float)rd.x, (float)rd.y, (float)rd.z);
@@ -1041,22 +1082,17 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                         f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
                         bool broke;
                         if (MODE == 1) {
-                            const double4 xi0 = ldg_d4(&d.x0[io]), ri0 = ldg_d4(&d.rot[io]);
-                            const double4 xj0 = ldg_d4(&d.x0[j]), rj0 = ldg_d4(&d.rot[j]);
-                            const double hx = 0.5 * (ri0.x + rj0.x), hy = 0.5 * (ri0.y + rj0.y), hz = 0.5 * (ri0.z + rj0.z);
-                            const f3 du = mk3((float)(rd.x - (xj0.x - xi0.x) - (hy * rd.z - hz * rd.y)),
-                                              (float)(rd.y - (xj0.y - xi0.y) - (hz * rd.x - hx * rd.z)),
-                                              (float)(rd.z - (xj0.z - xi0.z) - (hx * rd.y - hy * rd.x)));
-                            broke = bond_slot_ext_total(b, r, rr, du, mk3((float)ri0.x, (float)ri0.y, (float)ri0.z),
-                                                        mk3((float)rj0.x, (float)rj0.y, (float)rj0.z), rij, oijt, mijn,
-                                                        mijt, rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr);
+                            broke = fire_bond(d, b, io, j, r, rd, rr, rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr);
                         } else {
-                            broke = bond_slot_ext(ep, b, r, rr, f4to3(__ldg(&Vv[io])), f4to3(vj), f4to3(__ldg(&Wv[io])),
-                                                  f4to3(wj), rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr, c.ref_mode != 0);
+                            const F8 vwo = ldg8(&VW[io]);
+                            broke = bond_slot_ext(ep, b, r, rr, f4to3(vwo.a), f4to3(vwj.a), f4to3(vwo.b), f4to3(vwj.b), rij, oijt, mijn, mijt, fr, mr, fnr, ktr, krr, c.ref_mode != 0);
                         }
-                        d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
-                        d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
-                        d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
+                        // (a FIRE pass reads the increment's start state, so the state it leads to is
+                        // only written when the bond breaks; the relaxed one by k_fire_bond_state)
+                        if (MODE == 0 || broke) {
+                            st8(&d.rec[s].s0, make_float4(rij.x, rij.y, rij.z, oijt.x), make_float4(oijt.y, oijt.z, mijn.x, mijn.y));
+                            st8(&d.rec[s].s2, make_float4(mijn.z, mijt.x, mijt.y, mijt.z), kc);
+                        }
                         if (broke) fl |= RF_REC_BROKE;
                     }
                     res[x] = fr.x; res[CH + x] = fr.y; res[2 * CH + x] = fr.z;
@@ -1076,20 +1112,22 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                     if (t0 + lane < npar) {
                         const uint32_t x = s_par[wp][t0 + lane], e = lst[base + x], io = wbase + (e & 31u);
                         const size_t s = (size_t)(e >> 5) * N + io;
-                        const uint32_t j = __ldg(&d.bj[s]), k = d.bk[s];
-                        const double L0 = __ldg(&d.bL0[s]);
+                        const uint2 jk = d.bjk[s];
+                        const uint32_t j = jk.x, k = jk.y;
+                        const double L0 = rec_L0(d.rec[s].k);
                         const double4 xo = ldg_d4(&P[io]), xj = ldg_d4(&P[j]);
                         const size_t so = ((size_t)io * c.K + k) * 3;
                         const float* oi = d.cO[cur] + so;
                         // (a record's slot is in contact at the step's start until this record is added)
                         f3 o = ((d.cmask[io] >> k) & 1u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
-                        const f3 wo = f4to3(__ldg(&Wv[io]));
+                        const F8 vwo = ldg8(&VW[io]), vwj = ldg8(&VW[j]);
+                        const f3 wo = f4to3(vwo.b);
                         const double3 rd = dsub(xj, xo);
                         const float ro = (float)xo.w, rj = (float)xj.w;
                         const ContactTerms ct = contact_terms_ext(
                             ep, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), fmin(xo.w + xj.w, L0), ro, rj,
-                            c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(__ldg(&Vv[io])), f4to3(__ldg(&Vv[j])), wo,
-                            f4to3(__ldg(&Wv[j])), o);
+                            c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(vwo.a), f4to3(vwj.a), wo,
+                            f4to3(vwj.b), o);
                         float* oo = d.cO[nxt] + so;
                         oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
                         f3 fr = mk3(res[x], res[CH + x], res[2 * CH + x]);
@@ -1142,7 +1180,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         const uint32_t q = __ffs(del) - 1u;
         del &= del - 1u;
         const size_t s = (size_t)q * N + i;
-        delete_slot(d, c, i, d.bk[s], d.bj[s], ncand, nbq, live, bond, cm, bmask, mem);
+        delete_slot(d, c, i, d.bjk[s].y, d.bjk[s].x, ncand, nbq, live, bond, cm, bmask, mem);
     }
 
     // the particle's own position (the bond pass read it through the cache; its velocity
@@ -1164,14 +1202,22 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 all &= all - 1u;
             }
         }
-        while (m) {
-            const uint32_t k = __ffs(m) - 1;
-            m &= m - 1;
-            const double4 xj = ldg_d4(&P[row[k]]);
-            const double rr = dlen2(dsub(xj, xi));
-            if (rr > cut2_del(c, xi.w, xj.w) || rr < 1e-10) { far |= 1u << k; continue; }
-            const double sr = xi.w + xj.w;
-            if (rr < sr * sr) ct |= 1u << k;
+        while (m) {                              // four slots' ids, then their positions, in flight
+            uint32_t bit[4], j[4];
+            double4 xj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { bit[u] = m & (0u - m); m &= m - 1u; }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) j[u] = bit[u] ? row[__ffs(bit[u]) - 1] : i;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = ldg_d4(&P[j[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double rr = dlen2(dsub(xj[u], xi));
+                const double sr = xi.w + xj[u].w;
+                if (rr > cut2_del(c, xi.w, xj[u].w) || rr < 1e-10) far |= bit[u];
+                else if (rr < sr * sr) ct |= bit[u];
+            }
         }
 #pragma unroll
         for (int o = PW; o < 32; o <<= 1) {
@@ -1203,17 +1249,26 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q = sub; scan && q < qlim; q += SUB) {
-                if ((tried >> q) & 1ull) continue;
-                const uint32_t j = __ldg(&d.cand[(size_t)q * N + i]);
-                const double4 xj = ldg_d4(&P[j]);
-                const double rr = dlen2(dsub(xj, xi));
-                if (!(rr < cut2_add(c, xi.w, xj.w) && rr > 1e-10)) continue;
-                if (!have_cells) { oc = octant_of(xif, c.g); have_cells = true; }
-                const int rank = octant_rank(oc, ref_cell(mk3((float)xj.x, (float)xj.y, (float)xj.z), c.g));
-                if (rank < 0) continue;
-                const unsigned long long key = ((unsigned long long)rank << 32) | j;
-                if (key < best) { best = key; best_q = q; }
+            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 4 * SUB) {      // four candidates in flight
+                uint32_t j[4];
+                double4 xj[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const uint32_t q = q0 + u * SUB;
+                    j[u] = q < qlim && !((tried >> q) & 1ull) ? __ldg(&d.cand[(size_t)q * N + i]) : i;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) xj[u] = ldg_d4(&P[j[u]]);
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const double rr = dlen2(dsub(xj[u], xi));
+                    if (j[u] == i || !(rr < cut2_add(c, xi.w, xj[u].w) && rr > 1e-10)) continue;
+                    if (!have_cells) { oc = octant_of(xif, c.g); have_cells = true; }
+                    const int rank = octant_rank(oc, ref_cell(mk3((float)xj[u].x, (float)xj[u].y, (float)xj[u].z), c.g));
+                    if (rank < 0) continue;
+                    const unsigned long long key = ((unsigned long long)rank << 32) | j[u];
+                    if (key < best) { best = key; best_q = q0 + u * SUB; }
+                }
             }
 #pragma unroll
             for (int o = PW; o < 32; o <<= 1) {
@@ -1279,10 +1334,11 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 f3 o = (e & 1024u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
                 const double3 rd = dsub(xj, xo);
                 const float ro = (float)xo.w, rj = (float)xj.w;
+                const F8 vwo = ldg8(&VW[io]), vwj = ldg8(&VW[j]);
                 const ContactTerms t =
                     contact_terms_ext(ep, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), xo.w + xj.w, ro, rj,
-                                      c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(__ldg(&Vv[io])),
-                                      f4to3(__ldg(&Vv[j])), f4to3(__ldg(&Wv[io])), f4to3(__ldg(&Wv[j])), o);
+                                      c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(vwo.a), f4to3(vwj.a),
+                                      f4to3(vwo.b), f4to3(vwj.b), o);
                 float* oo = d.cO[nxt] + 3 * so;
                 oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
                 res[lane] = t.n.x; res[1 * 32 + lane] = t.n.y; res[2 * 32 + lane] = t.n.z;
@@ -1295,7 +1351,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
             }
             __syncwarp();
             if (rem && rk < base + 32u) {
-                const f3 wi = f4to3(__ldg(&Wv[i]));
+                const f3 wi = f4to3(ldg8(&VW[i]).b);
                 while (rem && rk < base + 32u) {
                     const uint32_t x = rk - base;
                     rem &= rem - 1u;
@@ -1330,7 +1386,8 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
 #pragma unroll
     for (int q = 0; q < FIRE_SUMS; ++q) acc[q] = 0.0;
     if (valid) {
-        const f3 vi = f4to3(Vv[i]), wi = f4to3(Wv[i]);
+        const F8 vwi = ldg8(&VW[i]);
+        const f3 vi = f4to3(vwi.a), wi = f4to3(vwi.b);
         const float mi = c.cmass * ri * ri * ri;
         if (dirty) { d.live[i] = live; d.bond[i] = bond; d.member[i] = mem; d.bmask[i] = bmask; }
         if (cm != cm0) d.cmask[i] = cm;
@@ -1356,10 +1413,11 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
             uniaxial_particle_ext(Rx, Ry, Rz, Vx, Vy, Vz, Fx, Fy, Fz, cc, RR, Top, Bottom, TopR, BottomR, vt,
                                   (double)G.zcut, xi.w - c.p_r_d, sfb, sft, MODE == 1);
         if (MODE == 1) {
-            // FIRE: keep the clamped state for the update kernel; reduce the FIRE sums
+            // FIRE: keep the clamped state for the update kernel (and the coordinate the platens
+            // may have clamped, for k_fire_bond_state); reduce the FIRE sums
+            d.xax[i] = KIND == RF_TEST_BRAZIL ? xi.y : xi.z;
             d.posd[nxt][i] = make_double4(Rx, Ry, Rz, xi.w);
-            d.vel[nxt][i] = make_float4(Vx, Vy, Vz, 0.f);
-            d.ang[nxt][i] = make_float4(wi.x, wi.y, wi.z, 0.f);
+            st8(&d.vw[nxt][i], make_float4(Vx, Vy, Vz, 0.f), make_float4(wi.x, wi.y, wi.z, 0.f));
             d.frc[i] = make_float4(Fx, Fy, Fz, kt);
             d.mom[i] = make_float4(Mx, My, Mz, kr);
             acc[0] = (double)Fx * Vx + (double)Fy * Vy + (double)Fz * Vz + (double)Mx * wi.x + (double)My * wi.y +
@@ -1385,8 +1443,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
             Vx = 0.f; Vy = 0.f; Vz = 0.f;
         }
         d.posd[nxt][i] = make_double4(Rx, Ry, Rz, xi.w);
-        d.vel[nxt][i] = make_float4(Vx, Vy, Vz, 0.f);
-        d.ang[nxt][i] = make_float4(Wx, Wy, Wz, 0.f);
+        st8(&d.vw[nxt][i], make_float4(Vx, Vy, Vz, 0.f), make_float4(Wx, Wy, Wz, 0.f));
         const float4 pr = d.pos_ref[i];
         const float ex = (float)Rx - pr.x, ey = (float)Ry - pr.y, ez = (float)Rz - pr.z;
         const float e2 = ex * ex + ey * ey + ez * ez;
@@ -1425,8 +1482,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     __syncthreads();
     const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
     const float4* __restrict__ P = d.pos[cur];
-    const float4* __restrict__ Vv = d.vel[cur];
-    const float4* __restrict__ Wv = d.ang[cur];
+    const F8* __restrict__ VW = d.vw[cur];
     const uint32_t N = c.N;
     const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
     const uint32_t pl = lane % PW, sub = lane / PW;            // particle of the warp, share of its scans
@@ -1445,7 +1501,6 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
         nbq = d.nbq[i]; bmask = d.bmask[i];
     }
     const uint32_t cm0 = cm;
-    const size_t QN = (size_t)d.QB * N;
     bool dirty = false;
     uint32_t nbroken = 0;
 
@@ -1475,12 +1530,16 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                 const uint32_t e = lst[base + lane];
                 const uint32_t q = e >> 5, io = wbase + (e & 31u);
                 const size_t s = (size_t)q * N + io;
-                const uint32_t j = __ldg(&d.bj[s]);
-                const float il = __ldg(&d.bil[s]);
-                const float4 s0 = d.bst[s], s1 = d.bst[s + QN], s2 = d.bst[s + 2 * QN];
-                uint32_t fl = (uint32_t)d.bk[s] << 8;
-                const f3 xo = f4to3(__ldg(&P[io])), vo = f4to3(__ldg(&Vv[io])), wo = f4to3(__ldg(&Wv[io]));
-                const f3 xj = f4to3(__ldg(&P[j])), vj = f4to3(__ldg(&Vv[j])), wj = f4to3(__ldg(&Wv[j]));
+                const uint2 jk = d.bjk[s];
+                float4 s0, s1, s2, kc;
+                ld8(&d.rec[s].s0, s0, s1);
+                ld8(&d.rec[s].s2, s2, kc);
+                const uint32_t j = jk.x;
+                const float il = kc.x;
+                uint32_t fl = jk.y << 8;
+                const f3 xo = f4to3(__ldg(&P[io])), xj = f4to3(__ldg(&P[j]));
+                const F8 vwo = ldg8(&VW[io]), vwj = ldg8(&VW[j]);
+                const f3 vo = f4to3(vwo.a), wo = f4to3(vwo.b), vj = f4to3(vwj.a), wj = f4to3(vwj.b);
                 const float rr = dist2_rn(xo, xj);
                 if (rr > c.aa_farcut || below_1em10(rr)) {
                     fl |= RF_REC_DELETE;
@@ -1491,9 +1550,8 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                     f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w);
                     KeepTerms t;
                     if (bond_slot(c.bp, r, vo, vj, wo, wj, il, rij, oijt, mijn, mijt, t)) fl |= RF_REC_BROKE;
-                    d.bst[s] = make_float4(rij.x, rij.y, rij.z, oijt.x);
-                    d.bst[s + QN] = make_float4(oijt.y, oijt.z, mijn.x, mijn.y);
-                    d.bst[s + 2 * QN] = make_float4(mijn.z, mijt.x, mijt.y, mijt.z);
+                    st8(&d.rec[s].s0, make_float4(rij.x, rij.y, rij.z, oijt.x), make_float4(oijt.y, oijt.z, mijn.x, mijn.y));
+                    st8(&d.rec[s].s2, make_float4(mijn.z, mijt.x, mijt.y, mijt.z), kc);
 #pragma unroll
                     for (int a = 0; a < 2; ++a) {
                         s_res[wp][3 * a][lane] = t.ft[a].x; s_res[wp][3 * a + 1][lane] = t.ft[a].y;
@@ -1550,13 +1608,21 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                 all &= all - 1u;
             }
         }
-        while (m) {
-            const uint32_t k = __ffs(m) - 1;
-            m &= m - 1;
-            const f3 xj = f4to3(__ldg(&P[row[k]]));
-            const float rr = dist2_rn(xi, xj);
-            if (rr > c.aa_farcut || below_1em10(rr)) { far |= 1u << k; continue; }
-            if (norm3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z) < twoR) ct |= 1u << k;
+        while (m) {                              // four slots' ids, then their positions, in flight
+            uint32_t bit[4], j[4];
+            float4 xj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { bit[u] = m & (0u - m); m &= m - 1u; }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) j[u] = bit[u] ? row[__ffs(bit[u]) - 1] : i;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = __ldg(&P[j[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float rr = dist2_rn(xi, f4to3(xj[u]));
+                if (rr > c.aa_farcut || below_1em10(rr)) far |= bit[u];
+                else if (norm3(xj[u].x - xi.x, xj[u].y - xi.y, xj[u].z - xi.z) < twoR) ct |= bit[u];
+            }
         }
 #pragma unroll
         for (int o = PW; o < 32; o <<= 1) {
@@ -1589,17 +1655,26 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q = sub; scan && q < qlim; q += SUB) {
-                if ((tried >> q) & 1ull) continue;
-                const uint32_t j = __ldg(&d.cand[(size_t)q * N + i]);
-                const f3 xj = f4to3(__ldg(&P[j]));
-                const float rr = dist2_rn(xi, xj);
-                if (!(rr < c.aacut && above_1em10(rr))) continue;
-                if (!have_cells) { oc = octant_of(xi, c.g); have_cells = true; }
-                const int rank = octant_rank(oc, ref_cell(xj, c.g));
-                if (rank < 0) continue;
-                const unsigned long long key = ((unsigned long long)rank << 32) | j;
-                if (key < best) { best = key; best_q = q; }
+            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 4 * SUB) {      // four candidates in flight
+                uint32_t j[4];
+                float4 xj[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const uint32_t q = q0 + u * SUB;
+                    j[u] = q < qlim && !((tried >> q) & 1ull) ? __ldg(&d.cand[(size_t)q * N + i]) : i;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) xj[u] = __ldg(&P[j[u]]);
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const float rr = dist2_rn(xi, f4to3(xj[u]));
+                    if (j[u] == i || !(rr < c.aacut && above_1em10(rr))) continue;
+                    if (!have_cells) { oc = octant_of(xi, c.g); have_cells = true; }
+                    const int rank = octant_rank(oc, ref_cell(f4to3(xj[u]), c.g));
+                    if (rank < 0) continue;
+                    const unsigned long long key = ((unsigned long long)rank << 32) | j[u];
+                    if (key < best) { best = key; best_q = q0 + u * SUB; }
+                }
             }
 #pragma unroll
             for (int o = PW; o < 32; o <<= 1) {
@@ -1661,8 +1736,8 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                 f3 o = (e & 1024u) ? mk3(oi[0], oi[1], oi[2]) : mk3(0.f, 0.f, 0.f);
                 const f3 r = mk3(xj.x - xo.x, xj.y - xo.y, xj.z - xo.z);
                 KeepTerms t;
-                contact_pair(c.cp, r, norm3(r.x, r.y, r.z), f4to3(__ldg(&Vv[io])), f4to3(__ldg(&Vv[j])),
-                             f4to3(__ldg(&Wv[io])), f4to3(__ldg(&Wv[j])), o, t);
+                const F8 vwo = ldg8(&VW[io]), vwj = ldg8(&VW[j]);
+                contact_pair(c.cp, r, norm3(r.x, r.y, r.z), f4to3(vwo.a), f4to3(vwj.a), f4to3(vwo.b), f4to3(vwj.b), o, t);
                 float* oo = d.cO[nxt] + 3 * so;
                 oo[0] = o.x; oo[1] = o.y; oo[2] = o.z;
                 if (t.clear) t.mt[1] = mk3(0.f, 0.f, 0.f);
@@ -1706,7 +1781,8 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                     BottomR = (float)sc->BottomR, vt = (float)sc->V, RR = sc->RR;
         rf_float3 cc;
         cc.x = sc->center[0]; cc.y = sc->center[1]; cc.z = sc->center[2];
-        const f3 vi = f4to3(__ldg(&Vv[i])), wi = f4to3(__ldg(&Wv[i]));
+        const F8 vwi = ldg8(&VW[i]);
+        const f3 vi = f4to3(vwi.a), wi = f4to3(vwi.b);
         // F = 0 after the memset, then += _22 sums, then += _21 sums
         float Fx = 0.0f + fsb.x, Fy = 0.0f + fsb.y, Fz = 0.0f + fsb.z;
         Fx += fsc.x; Fy += fsc.y; Fz += fsc.z;
@@ -1727,8 +1803,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
             Vx = 0.f; Vy = 0.f; Vz = 0.f;
         }
         d.pos[nxt][i] = make_float4(Rx, Ry, Rz, 0.f);
-        d.vel[nxt][i] = make_float4(Vx, Vy, Vz, 0.f);
-        d.ang[nxt][i] = make_float4(Wx, Wy, Wz, 0.f);
+        st8(&d.vw[nxt][i], make_float4(Vx, Vy, Vz, 0.f), make_float4(Wx, Wy, Wz, 0.f));
         const float4 pr = d.pos_ref[i];
         const float ex = Rx - pr.x, ey = Ry - pr.y, ez = Rz - pr.z;
         const float e2 = ex * ex + ey * ey + ez * ez;
@@ -1890,6 +1965,46 @@ __device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c,
     }
 }
 
+// State of the intact bond records at the end of an increment: each from its state at the
+// increment's start, at the positions and rotations the specimen's last force pass read (the
+// positions that pass wrote, less the platens' clamp). Once an increment instead of in every
+// pass: 64 bytes a record written were a quarter of a pass's traffic.
+template <int KIND>
+__global__ void __launch_bounds__(128) k_fire_bond_state(Dev d, Consts c) {
+    const uint32_t cur = (uint32_t)(d.sc->steps & 1ull);
+    const double4* __restrict__ P = d.posd[cur];
+    const uint32_t i = blockIdx.x * 128u + threadIdx.x;
+    if (i >= c.N) return;
+    auto read_at = [&](uint32_t q) {
+        double4 x = ldg_d4(&P[q]);
+        (KIND == RF_TEST_BRAZIL ? x.y : x.z) = d.xax[q];
+        return x;
+    };
+    const double4 xi = read_at(i);
+    uint32_t m = d.bmask[i];
+    while (m) {
+        const uint32_t q = __ffs(m) - 1u;
+        m &= m - 1u;
+        const size_t s = (size_t)q * c.N + i;
+        const uint32_t j = d.bjk[s].x;
+        float4 s0, s1, s2, kc;
+        ld8(&d.rec0[s].s0, s0, s1);
+        ld8(&d.rec0[s].s2, s2, kc);
+        const double4 xj = read_at(j);
+        const double3 rd = dsub(xj, xi);
+        const double rr = dlen2(rd);
+        BondExt b;
+        b.kn = c.kn; b.ks = c.ks; b.br = c.br_lambda * fminf((float)xi.w, (float)xj.w);
+        b.sc = kc.z; b.tc = kc.w; b.L0 = rec_L0(kc);
+        f3 rij = mk3(s0.x, s0.y, s0.z), oijt = mk3(s0.w, s1.x, s1.y);
+        f3 mijn = mk3(s1.z, s1.w, s2.x), mijt = mk3(s2.y, s2.z, s2.w), fr = mk3(0.f, 0.f, 0.f), mr = fr;
+        float u0 = 0.f, u1 = 0.f, u2 = 0.f;
+        fire_bond(d, b, i, j, mk3((float)rd.x, (float)rd.y, (float)rd.z), rd, rr, rij, oijt, mijn, mijt, fr, mr, u0, u1, u2);
+        st8(&d.rec[s].s0, make_float4(rij.x, rij.y, rij.z, oijt.x), make_float4(oijt.y, oijt.z, mijn.x, mijn.y));
+        st8(&d.rec[s].s2, make_float4(mijn.z, mijt.x, mijt.y, mijt.z), kc);
+    }
+}
+
 // FIRE update of one iteration, in place on the buffers the force pass wrote:
 // mixing (or, on uphill power, stop), then semi-implicit Euler in FP64
 // positions; the rotation of the increment is accumulated for the warm-start data.
@@ -1906,7 +2021,7 @@ __global__ void k_fire_update(Dev d, Consts c) {
     float e2max = 0.f;
     if (!stop && i < c.N && !S->fstop) {
         double4 x = d.posd[cur][i];
-        float4 v = d.vel[cur][i], w = d.ang[cur][i];
+        float4 v = d.vw[cur][i].a, w = d.vw[cur][i].b;
         const float4 F = d.frc[i], M = d.mom[i];
         const float dt = (float)S->fdt;
         const double dtd = (double)dt;
@@ -1930,8 +2045,7 @@ __global__ void k_fire_update(Dev d, Consts c) {
         r.x += (double)w.x * dtd; r.y += (double)w.y * dtd; r.z += (double)w.z * dtd;
         d.rot[i] = r;
         d.posd[cur][i] = x;
-        d.vel[cur][i] = v;
-        d.ang[cur][i] = w;
+        st8(&d.vw[cur][i], v, w);
         const float4 pr = d.pos_ref[i];
         const float ex = (float)x.x - pr.x, ey = (float)x.y - pr.y, ez = (float)x.z - pr.z;
         const float e2 = ex * ex + ey * ey + ez * ez;
@@ -2070,8 +2184,7 @@ __global__ void k_qs_begin(Dev d, Consts c, const float* __restrict__ warm, int 
             uniaxial_particle_ext(x.x, x.y, x.z, v0, v1, v2, f0, f1, f2, cc, RR, Top, Bottom, TopR, BottomR, 0.f,
                                   zcut, x.w - c.p_r_d, sb, st, false);
         d.posd[cur][i] = x;
-        d.vel[cur][i] = make_float4(v0, v1, v2, 0.f);
-        d.ang[cur][i] = w;
+        st8(&d.vw[cur][i], make_float4(v0, v1, v2, 0.f), w);
         d.rot[i] = rot;
     }
 }
@@ -2104,18 +2217,16 @@ __global__ void k_warm_features(Dev d, Consts c, double sinc, __nv_bfloat16* __r
     f[6] = (float)(p[ax] / (0.5 * sc->size_d[ax]));
     const double o0 = p[ax == 2 ? 0 : 0], o1 = p[ax == 2 ? 1 : 2];
     f[7] = (float)(sqrt(o0 * o0 + o1 * o1) / (0.5 * sc->size_d[0]));
-    const size_t QN = (size_t)d.QB * c.N;
-    (void)QN;
     const uint32_t bm = d.bmask[i], nq = d.nbq[i];
     int nb = 0;
     for (uint32_t q = 0; q < nq && nb < 12; ++q) {
         if (!((bm >> q) & 1u)) continue;
         const size_t s = (size_t)q * c.N + i;
-        const uint32_t j = d.bj[s];
+        const uint32_t j = d.bjk[s].x;
         const double4 xj = d.posd[cur][j], xj0 = d.x0[j];
         const double ex = (xj.x - xj0.x) - dxi, ey = (xj.y - xj0.y) - dyi, ez = (xj.z - xj0.z) - dzi;
         const double rx = xj.x - x.x, ry = xj.y - x.y, rz = xj.z - x.z;
-        const double L0 = d.bL0[s];
+        const double L0 = rec_L0(d.rec[s].k);
         float* g = f + 8 + 4 * nb;
         g[0] = (float)(ex * iD); g[1] = (float)(ey * iD); g[2] = (float)(ez * iD);
         g[3] = (float)((sqrt(rx * rx + ry * ry + rz * rz) - L0) / (L0 * sinc));
@@ -2197,13 +2308,14 @@ __global__ void k_stream_ungate(Dev d) {
 // ---------------------------------------------------------------------------
 // Layout conversion (reference layout <-> engine layout)
 // ---------------------------------------------------------------------------
-__global__ void k_planar_to_f4(const float* __restrict__ R, uint32_t N, float4* __restrict__ out) {
+// (stride: float4 records a particle, 2 for the velocities and spins)
+__global__ void k_planar_to_f4(const float* __restrict__ R, uint32_t N, float4* __restrict__ out, uint32_t stride) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-        out[i] = make_float4(R[i], R[i + N], R[i + 2 * (size_t)N], 0.f);
+        out[(size_t)i * stride] = make_float4(R[i], R[i + N], R[i + 2 * (size_t)N], 0.f);
 }
-__global__ void k_f4_to_planar(const float4* __restrict__ in, uint32_t N, float* __restrict__ R) {
+__global__ void k_f4_to_planar(const float4* __restrict__ in, uint32_t N, float* __restrict__ R, uint32_t stride) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        const float4 v = in[i];
+        const float4 v = in[(size_t)i * stride];
         R[i] = v.x; R[i + N] = v.y; R[i + 2 * (size_t)N] = v.z;
     }
 }
@@ -2236,7 +2348,6 @@ __global__ void k_rows_import(const uint_fast32_t* __restrict__ IL, const uint8_
                               const rf_float3* __restrict__ Mijt, const double* __restrict__ L0x,
                               const float2* __restrict__ strx, Dev d, Consts c) {
     const uint_fast32_t E = empty_id<uint_fast32_t>();
-    const size_t QN = (size_t)d.QB * c.N;
     const uint32_t cur = (uint32_t)(d.sc->steps & 1ull);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
         uint32_t live = 0, bond = 0, cm = 0, nq = 0, bmask = 0;
@@ -2255,21 +2366,20 @@ __global__ void k_rows_import(const uint_fast32_t* __restrict__ IL, const uint8_
             else if (Oijt[r].x != 0.f || Oijt[r].y != 0.f || Oijt[r].z != 0.f) cm |= 1u << k;
             if (needs_record(type[r], Rij[r]) && nq < d.QB) {
                 const size_t b = (size_t)nq * c.N + i;
-                d.bj[b] = (uint32_t)j; d.bk[b] = (uint8_t)k; d.bil[b] = iL[r];
+                d.bjk[b] = make_uint2((uint32_t)j, k);
                 const float ox = t1 ? Oijt[r].x : 0.f, oy = t1 ? Oijt[r].y : 0.f, oz = t1 ? Oijt[r].z : 0.f;
-                d.bst[b] = make_float4(Rij[r].x, Rij[r].y, Rij[r].z, ox);
-                d.bst[b + QN] = make_float4(oy, oz, Mijn[r].x, Mijn[r].y);
-                d.bst[b + 2 * QN] = make_float4(Mijn[r].z, Mijt[r].x, Mijt[r].y, Mijt[r].z);
-                if (L0x) { d.bL0[b] = L0x[r]; d.bstr[b] = strx[r]; }
+                st8(&d.rec[b].s0, make_float4(Rij[r].x, Rij[r].y, Rij[r].z, ox), make_float4(oy, oz, Mijn[r].x, Mijn[r].y));
+                st8(&d.rec[b].s2, make_float4(Mijn[r].z, Mijt[r].x, Mijt[r].y, Mijt[r].z),
+                    L0x ? rec_const(L0x[r], strx[r]) : make_float4(iL[r], 0.f, 0.f, 0.f));
                 if (t1) bmask |= 1u << nq;
                 ++nq;
             }
         }
         for (uint32_t q = nq; q < d.QB; ++q) {          // unused records: retired, zero
             const size_t b = (size_t)q * c.N + i;
-            d.bj[b] = 0; d.bk[b] = 0xFF; d.bil[b] = 0.f;
-            if (L0x) { d.bL0[b] = 1.0; d.bstr[b] = make_float2(0.f, 0.f); }
-            zero_record(d, QN, b);
+            d.bjk[b] = make_uint2(0u, 0xFFu);
+            d.rec[b].k = L0x ? rec_const(1.0, make_float2(0.f, 0.f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            zero_record(d, b);
         }
         d.live[i] = live; d.bond[i] = bond; d.cmask[i] = cm; d.nbq[i] = nq; d.bmask[i] = bmask;
     }
@@ -2279,7 +2389,6 @@ __global__ void k_rows_export(uint_fast32_t* __restrict__ IL, uint8_t* __restric
                               rf_float3* __restrict__ Rij, rf_float3* __restrict__ Oijt, rf_float3* __restrict__ Mijn,
                               rf_float3* __restrict__ Mijt, Dev d, Consts c) {
     const uint_fast32_t E = empty_id<uint_fast32_t>();
-    const size_t QN = (size_t)d.QB * c.N;
     const uint32_t cur = (uint32_t)(d.sc->steps & 1ull);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
         const uint32_t live = d.live[i], bond = d.bond[i], nq = d.nbq[i];
@@ -2296,10 +2405,10 @@ __global__ void k_rows_export(uint_fast32_t* __restrict__ IL, uint8_t* __restric
         }
         for (uint32_t q = 0; q < nq; ++q) {
             const size_t b = (size_t)q * c.N + i;
-            const uint32_t k = d.bk[b];
-            if (k == 0xFF) continue;
+            const uint32_t k = d.bjk[b].y;
+            if (k == 0xFFu) continue;
             const size_t r = (size_t)i * c.K + k;
-            const float4 s0 = d.bst[b], s1 = d.bst[b + QN], s2 = d.bst[b + 2 * QN];
+            const float4 s0 = d.rec[b].s0, s1 = d.rec[b].s1, s2 = d.rec[b].s2;
             Rij[r].x = s0.x; Rij[r].y = s0.y; Rij[r].z = s0.z;
             Mijn[r].x = s1.z; Mijn[r].y = s1.w; Mijn[r].z = s2.x;
             Mijt[r].x = s2.y; Mijt[r].y = s2.z; Mijt[r].z = s2.w;
@@ -2975,7 +3084,7 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
     const size_t NK = (size_t)N * K;
     for (int b = 0; b < 2; ++b) {
         if ((ext ? (st = dalloc(e, &d.posd[b], N)) : (st = dalloc(e, &d.pos[b], N))) ||
-            (st = dalloc(e, &d.vel[b], N)) || (st = dalloc(e, &d.ang[b], N)))
+            (st = dalloc(e, &d.vw[b], N)))
             return fail(st);
     }
     if ((st = dalloc(e, &d.ids, NK)) || (st = dalloc(e, &d.il, NK)) || (st = dalloc(e, &d.cO[0], 3 * NK)) || (st = dalloc(e, &d.cO[1], 3 * NK)) ||
@@ -2992,7 +3101,7 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
         return fail(st);
     cudaStream_t s = e->stream;
     for (int b = 0; b < 2; ++b) {
-        if (cudaMemsetAsync(d.vel[b], 0, N * sizeof(float4), s) || cudaMemsetAsync(d.ang[b], 0, N * sizeof(float4), s))
+        if (cudaMemsetAsync(d.vw[b], 0, N * sizeof(F8), s))
             return fail(cuda_status(cudaGetLastError(), "memset"));
     }
     // specimens: geometry, CTA -> specimen map, per-specimen scalars
@@ -3160,12 +3269,10 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
             if (qb == 0) qb = 1;
             d.QB = qb;
             const size_t QN = (size_t)qb * N;
-            if (!st2 && ((st2 = dalloc(e, &d.bj, QN)) || (st2 = dalloc(e, &d.bk, QN)) || (st2 = dalloc(e, &d.bil, QN)) ||
-                         (st2 = dalloc(e, &d.bst, 3 * QN)))) {}
-            if (!st2 && ext && ((st2 = dalloc(e, &d.bL0, QN)) || (st2 = dalloc(e, &d.bstr, QN)))) {}
+            if (!st2 && ((st2 = dalloc(e, &d.bjk, QN)) || (st2 = dalloc(e, &d.rec, QN)))) {}
         }
         if (!st2) {
-            if (!ext) k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(dR, N, d.pos[0]);
+            if (!ext) k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(dR, N, d.pos[0], 1u);
             k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dIL_f, Rij, Oijt, Mijn, Mijt, dL0, dStr, d, c);
             ce = cudaGetLastError();
             if (ce) st2 = cuda_status(ce, "engine import");
@@ -3356,7 +3463,7 @@ rf_status fire_setup(rf_engine* e) {
         (st = dalloc(e, &d.fpart, (size_t)e->ncta * FIRE_SUMS)) || (st = dalloc(e, &d.rot, N)) ||
         (d.nspec > 1 && (st = dalloc(e, &d.fpart2, (size_t)e->ncta * FIRE_SUMS))) ||
         (st = dalloc(e, &d.fgrp, groups * FIRE_SUMS)) || (st = dalloc(e, &d.fgrp_n, groups)) ||
-        (st = dalloc(e, &d.x0, N)) || (st = dalloc(e, &d.bst0, 3 * (size_t)d.QB * N)))
+        (st = dalloc(e, &d.x0, N)) || (st = dalloc(e, &d.xax, N)) || (st = dalloc(e, &d.rec0, (size_t)d.QB * N)))
         return st;
     RF_CUDA(cudaMemsetAsync(d.fgrp_n, 0, groups * sizeof(uint32_t), e->stream));
     e->cf = e->c;
@@ -3399,7 +3506,7 @@ rf_status load_increment(rf_engine* e, const rf_relax_params* p, const float* wa
     }
     RF_CUDA(cudaMemcpyAsync(d.spec, hs.data(), ns * sizeof(DevScalars), cudaMemcpyHostToDevice, s));
     // the bond records' state at the start of the increment (FIRE mode computes from it)
-    RF_CUDA(cudaMemcpyAsync(d.bst0, d.bst, 3 * (size_t)d.QB * N * sizeof(float4), cudaMemcpyDeviceToDevice, s));
+    RF_CUDA(cudaMemcpyAsync(d.rec0, d.rec, (size_t)d.QB * N * sizeof(Rec), cudaMemcpyDeviceToDevice, s));
     const unsigned nb = (N + 127) / 128;
     if (e->task.kind == RF_TEST_BRAZIL) {
         k_qs_begin_scalars<RF_TEST_BRAZIL><<<1, 32, 0, s>>>(d, e->cf, p->strain_inc);
@@ -3411,6 +3518,9 @@ rf_status load_increment(rf_engine* e, const rf_relax_params* p, const float* wa
     RF_CHECK_LAUNCH("k_qs_begin");
     if (e->cf.use_graph) RF_CUDA(cudaGraphLaunch(e->fexec, s));
     else if (rf_status st = launch_stream_fire(e, p->max_iter)) return st;
+    if (e->task.kind == RF_TEST_BRAZIL) k_fire_bond_state<RF_TEST_BRAZIL><<<nb, 128, 0, s>>>(d, e->cf);
+    else k_fire_bond_state<RF_TEST_UNIAXIAL><<<nb, 128, 0, s>>>(d, e->cf);
+    RF_CHECK_LAUNCH("k_fire_bond_state");
     DevScalars g;
     RF_CUDA(cudaMemcpyAsync(hs.data(), d.spec, ns * sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
     RF_CUDA(cudaMemcpyAsync(&g, d.sc, sizeof(g), cudaMemcpyDeviceToHost, s));
@@ -3696,12 +3806,12 @@ rf_status rf_engine_export(rf_engine* e, float* R, float* V, float* W, uint_fast
     if (e->c.ext) k_delete_pending_ext<<<(N + 127) / 128, 128, 0, s>>>(e->d, e->c);
     else k_delete_pending<<<(N + 127) / 128, 128, 0, s>>>(e->d, e->c);
     RF_CHECK_LAUNCH("k_delete_pending");
-    const float4* vecs[3] = {e->d.pos[cur], e->d.vel[cur], e->d.ang[cur]};
+    const float4* vecs[3] = {e->d.pos[cur], &e->d.vw[cur]->a, &e->d.vw[cur]->b};
     float* outs[3] = {R, V, W};
     for (int q = 0; q < 3; ++q) {
         if (!outs[q]) continue;
         if (q == 0 && e->c.ext) k_posd_to_planar_f<<<(N + 255) / 256, 256, 0, s>>>(e->d.posd[cur], N, e->staging);
-        else k_f4_to_planar<<<(N + 255) / 256, 256, 0, s>>>(vecs[q], N, e->staging);
+        else k_f4_to_planar<<<(N + 255) / 256, 256, 0, s>>>(vecs[q], N, e->staging, q ? 2u : 1u);
         RF_CHECK_LAUNCH("k_f4_to_planar");
         RF_CUDA(cudaMemcpyAsync(outs[q], e->staging, 3 * (size_t)N * sizeof(float), cudaMemcpyDeviceToHost, s));
         RF_CUDA(cudaStreamSynchronize(s));
@@ -3749,10 +3859,10 @@ rf_status rf_engine_import(rf_engine* e, const float* R, const float* V, const f
     const int cur = (int)(h.steps & 1ull);
     if (!e->staging) RF_CUDA(cudaMalloc(&e->staging, 3 * (size_t)N * sizeof(float)));
     const float* ins[3] = {R, V, W};
-    float4* vecs[3] = {e->d.pos[cur], e->d.vel[cur], e->d.ang[cur]};
+    float4* vecs[3] = {e->d.pos[cur], &e->d.vw[cur]->a, &e->d.vw[cur]->b};
     for (int q = 0; q < 3; ++q) {
         RF_CUDA(cudaMemcpyAsync(e->staging, ins[q], 3 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, s));
-        k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(e->staging, N, vecs[q]);
+        k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(e->staging, N, vecs[q], q ? 2u : 1u);
         RF_CHECK_LAUNCH("k_planar_to_f4");
         RF_CUDA(cudaStreamSynchronize(s));
     }
