@@ -336,9 +336,10 @@ __global__ void k_rb_scatter(Dev d, Consts c) {
 // scan needs no candidate of a bucket whose lower bound the displacements since this build
 // cannot have closed, see scan_limit), which of them sit in i's row, and the margin of the
 // nearest that does not. Positions are read in cell order (three x-neighbouring cells are one
-// run of float4 records, nine runs a particle) and the candidates wait in shared memory, as
-// places in that order, until their buckets and the row's members are known; a row member
-// is found by its place. 4M particles: 3.0 ms with an id and a position gathered for
+// run of float4 records, nine runs a particle). A particle first only collects, in shared memory,
+// the places of its candidates in that order (what else a candidate needs would be run by the
+// whole warp for each of its lanes' hits in turn); the buckets and the row's members, found by
+// their places, follow. 4M particles: 3.0 ms with an id and a position gathered for
 // every occupant and the list ordered and matched in memory, 2.5 ms so.
 #define RF_RB_CTA 128
 __global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
@@ -351,7 +352,6 @@ __global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
         d.pos_ref[i] = xi;
         auto cut_of = [&](const float4 xj) { return c.lgap_f > 0.f ? fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) : c.acut_f; };
         uint32_t n = 0;
-        unsigned long long k0 = 0ull, k1 = 0ull;           // bits 0 and 1 of the candidates' buckets
         if (key < c.cg_cells) {
             const int ix = key % c.cg_nx, iy = (key / c.cg_nx) % c.cg_ny, iz = key / (c.cg_nx * c.cg_ny);
             const uint32_t xa = ix > 0 ? ix - 1 : 0, xb = ix + 1 < (int)c.cg_nx ? ix + 1 : ix;
@@ -364,25 +364,25 @@ __global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
                         const float4 xj = __ldg(&d.cg_pos[q]);
                         const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
                         const float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                        if (!(d2 < c.rc2) || q == mine) continue;
-                        const float cut = cut_of(xj);
-                        const float reach = cut + c.skin_f;
-                        if (c.lgap_f > 0.f && !(d2 < reach * reach)) continue;
-                        if (n < c.KC) {
-                            const float mg = sqrtf(d2) - cut;
-                            const uint32_t b = mg < RF_CB1 * c.skin_f ? 0u : mg < RF_CB2 * c.skin_f ? 1u : mg < RF_CB3 * c.skin_f ? 2u : 3u;
-                            s_c[n][tid] = q;
-                            k0 |= (unsigned long long)(b & 1u) << n;
-                            k1 |= (unsigned long long)(b >> 1) << n;
-                        } else {
-                            raise_status(&d.sc->err, RF_ERR_CAPACITY);
-                        }
-                        ++n;
+                        // (with one cutoff for all, reach is rc up to rounding: rc2 alone decides)
+                        const float reach = c.lgap_f > 0.f ? fminf(c.acut_f, (xi.w + xj.w) + c.lgap_f) + c.skin_f : 3.0e18f;
+                        if (!(d2 < c.rc2) || !(d2 < reach * reach) || q == mine) continue;
+                        if (n < c.KC) s_c[n++][tid] = q;
+                        else raise_status(&d.sc->err, RF_ERR_CAPACITY);
                     }
                 }
             }
         }
-        if (n > c.KC) n = c.KC;
+        unsigned long long k0 = 0ull, k1 = 0ull;           // bits 0 and 1 of the candidates' buckets
+#pragma unroll 4
+        for (uint32_t q = 0; q < n; ++q) {
+            const float4 xj = __ldg(&d.cg_pos[s_c[q][tid]]);
+            const float ddx = xj.x - xi.x, ddy = xj.y - xi.y, ddz = xj.z - xi.z;
+            const float mg = sqrtf(ddx * ddx + ddy * ddy + ddz * ddz) - cut_of(xj);
+            const uint32_t b = mg < RF_CB1 * c.skin_f ? 0u : mg < RF_CB2 * c.skin_f ? 1u : mg < RF_CB3 * c.skin_f ? 2u : 3u;
+            k0 |= (unsigned long long)(b & 1u) << q;
+            k1 |= (unsigned long long)(b >> 1) << q;
+        }
         d.cand_n[i] = n;
         unsigned long long in_row = 0ull;                  // candidates already in the row
         uint32_t live = d.live[i];
