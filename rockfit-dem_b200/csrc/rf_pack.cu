@@ -1,10 +1,11 @@
 // Seeded polydisperse specimen generator: random positions in a cylindrical container,
 // overlaps removed by FIRE with a repulsive (frictionless, undamped) Hertz contact, radii
 // grown in stages from a loose start to their targets. FP64 throughout (a one-time
-// generator, not the hot path). Neighbour search: a cell grid rebuilt every iteration
-// (histogram, scan, scatter). Each FIRE iteration is two fused kernels (forces with the
-// power and norm partials; then the per-particle FIRE update), the scalar FIRE state
-// lives on the device and batches of iterations are captured in a CUDA graph.
+// generator, not the hot path). Neighbour search: a cell grid rebuilt every iteration. A
+// small specimen's iteration is a chain of launches and memory latencies, so it is as few
+// kernels as the grid's dependencies allow, captured in batches in a CUDA graph: scan of the
+// cell counts, scatter, per-cell order with the positions gathered into it, forces with the
+// FIRE decision by the last block, and the FIRE update with the next grid's cell counts.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -18,7 +19,7 @@ struct Scal {
     double dt, alpha, fdotv, ff, vv, maxov;
     double scale;          // current radius scale g
     unsigned long long npos, iters;
-    uint32_t counter, pad;
+    uint32_t counter, arrived;
 };
 
 struct Par {
@@ -33,7 +34,8 @@ struct Dev {
     double4* x;       // x, y, z, target radius
     double4* v;       // velocity (w unused)
     double4* f;       // force (w unused)
-    uint32_t *key, *count, *start, *fill, *sorted, *bsum;
+    double4* xs;      // x in cell order
+    uint32_t *key, *count, *start, *sorted, *bsum;
     double4* part;    // per-block (F.v, |F|^2, |v|^2, max overlap)
     Scal* s;
 };
@@ -47,11 +49,6 @@ __device__ __forceinline__ uint32_t cell_of(const double4 p, const Par& c) {
     return (uint32_t)(ix + c.nx * (iy + c.ny * iz));
 }
 
-__global__ void k_zero(Dev d, Par c) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < c.cells; q += gridDim.x * blockDim.x) {
-        d.count[q] = 0; d.fill[q] = 0;
-    }
-}
 __global__ void k_bin(Dev d, Par c) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
         const uint32_t k = cell_of(d.x[i], c);
@@ -59,11 +56,11 @@ __global__ void k_bin(Dev d, Par c) {
         atomicAdd(&d.count[k], 1u);
     }
 }
-// single-block exclusive scan of the cell counts (cells are few: N / ~2)
-// Exclusive scan of the cell counts into cell starts, in three kernels: per-chunk sums
-// (SCAN_CHUNK cells per block), a one-block scan of the chunk sums, and the chunks'
-// own scans offset by their sums.
+// Exclusive scan of the cell counts into cell starts (start[cells] = N), SCAN_CHUNK cells per
+// block. Up to SCAN_SELF chunks each block adds up the counts before its chunk itself, one
+// kernel instead of three; beyond that the chunk sums and their scan are kernels of their own.
 constexpr uint32_t SCAN_CHUNK = 4096;
+constexpr uint32_t SCAN_SELF = 32;
 
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* wsum, uint32_t* total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -115,11 +112,22 @@ __global__ void k_scan_chunks(Dev d, uint32_t nb) {
     }
 }
 
-__global__ void k_scan_apply(Dev d, Par c) {
+__global__ void k_scan_apply(Dev d, Par c, int self) {
     __shared__ uint32_t wsum[32];
     __shared__ uint32_t total;
     const size_t base = (size_t)blockIdx.x * SCAN_CHUNK;
-    uint32_t carry = d.bsum[blockIdx.x];
+    uint32_t carry = 0;
+    if (self) {
+        uint32_t v = 0;
+        const uint4* c4 = reinterpret_cast<const uint4*>(d.count);
+#pragma unroll 4
+        for (size_t q = threadIdx.x; q < base / 4; q += blockDim.x) { const uint4 u = c4[q]; v += (u.x + u.y) + (u.z + u.w); }
+        block_excl_scan(v, wsum, &total);
+        carry = total;
+        __syncthreads();
+    } else {
+        carry = d.bsum[blockIdx.x];
+    }
     for (uint32_t off = 0; off < SCAN_CHUNK; off += blockDim.x) {
         const size_t q = base + off + threadIdx.x;
         const uint32_t v = q < c.cells ? d.count[q] : 0;
@@ -128,33 +136,39 @@ __global__ void k_scan_apply(Dev d, Par c) {
         carry += total;
         __syncthreads();
     }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) d.start[c.cells] = carry;
 }
+// The counts run back to zero as the cells fill: the update counts the next grid into them.
 __global__ void k_scatter(Dev d, Par c) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
         const uint32_t k = d.key[i];
-        d.sorted[d.start[k] + atomicAdd(&d.fill[k], 1u)] = i;
+        d.sorted[d.start[k] + atomicSub(&d.count[k], 1u) - 1u] = i;
     }
 }
 
 // Occupants of each cell in id order (the scatter's atomics leave them in arrival
-// order), so the force sums below, and with them the whole packing, are deterministic.
+// order), so the force sums below, and with them the whole packing, are deterministic; and
+// their positions in that order, so that the forces read the cells' runs straight through.
 __global__ void k_cellsort(Dev d, Par c) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < c.cells; q += gridDim.x * blockDim.x) {
-        uint32_t* a = d.sorted + d.start[q];
-        const uint32_t n = d.count[q];
+        const uint32_t s0 = d.start[q], n = d.start[q + 1] - s0;
+        uint32_t* a = d.sorted + s0;
         for (uint32_t u = 1; u < n; ++u) {
             const uint32_t v = a[u];
             uint32_t w = u;
             while (w > 0 && a[w - 1] > v) { a[w] = a[w - 1]; --w; }
             a[w] = v;
         }
+        for (uint32_t u = 0; u < n; ++u) d.xs[s0 + u] = d.x[a[u]];
     }
 }
 
 // Forces: repulsive Hertz between overlapping spheres and against the container wall,
 // f = 4/3 sqrt(R*) delta^1.5 (unit modulus, unit masses). Partials of F.v, |F|^2,
-// |v|^2 and the largest overlap (relative to the smaller radius).
-__global__ void k_force(Dev d, Par c) {
+// |v|^2 and the largest overlap (relative to the smaller radius); the last block to finish
+// makes the FIRE decision.
+__device__ __forceinline__ void fire_decide(Dev d, Par c, int nblocks);
+__global__ void __launch_bounds__(256) k_force(Dev d, Par c) {
     const double g = d.s->scale;
     double fv = 0, ff = 0, vv = 0, mo = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
@@ -163,31 +177,23 @@ __global__ void k_force(Dev d, Par c) {
         double fx = 0, fy = 0, fz = 0;
         const uint32_t key = d.key[i];
         const int ix = key % c.nx, iy = (key / c.nx) % c.ny, iz = key / (c.nx * c.ny);
-        for (int dz = -1; dz <= 1; ++dz) {
-            const int z = iz + dz;
-            if (z < 0 || z >= (int)c.nz) continue;
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int y = iy + dy;
-                if (y < 0 || y >= (int)c.ny) continue;
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int x = ix + dx;
-                    if (x < 0 || x >= (int)c.nx) continue;
-                    const uint32_t cell = x + c.nx * (y + c.ny * z);
-                    const uint32_t s0 = d.start[cell], e0 = s0 + d.count[cell];
-                    for (uint32_t q = s0; q < e0; ++q) {
-                        const uint32_t j = d.sorted[q];
-                        if (j == i) continue;
-                        const double4 xj = d.x[j];
-                        const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
-                        const double rj = g * xj.w;
-                        const double r2 = rx * rx + ry * ry + rz * rz, sr = ri + rj;
-                        if (r2 >= sr * sr || r2 <= 0) continue;
-                        const double r = sqrt(r2), dl = sr - r;
-                        const double Rs = ri * rj / sr;
-                        const double fn = (4.0 / 3.0) * sqrt(Rs) * dl * sqrt(dl);
-                        fx -= fn * rx / r; fy -= fn * ry / r; fz -= fn * rz / r;
-                        mo = fmax(mo, dl / fmin(ri, rj));
-                    }
+        // (three x-neighbouring cells are one run of the cell order)
+        const uint32_t xa = ix > 0 ? ix - 1 : 0, xb = ix + 1 < (int)c.nx ? ix + 1 : ix;
+        for (int z = max(iz - 1, 0); z <= min(iz + 1, (int)c.nz - 1); ++z) {
+            for (int y = max(iy - 1, 0); y <= min(iy + 1, (int)c.ny - 1); ++y) {
+                const uint32_t line = c.nx * (y + c.ny * z);
+                const uint32_t e0 = d.start[line + xb + 1];
+                for (uint32_t q = d.start[line + xa]; q < e0; ++q) {
+                    const double4 xj = d.xs[q];
+                    const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
+                    const double rj = g * xj.w;
+                    const double r2 = rx * rx + ry * ry + rz * rz, sr = ri + rj;
+                    if (r2 >= sr * sr || r2 <= 0) continue;        // (the particle itself: r2 = 0)
+                    const double r = sqrt(r2), dl = sr - r;
+                    const double Rs = ri * rj / sr;
+                    const double fn = (4.0 / 3.0) * sqrt(Rs) * dl * sqrt(dl);
+                    fx -= fn * rx / r; fy -= fn * ry / r; fz -= fn * rz / r;
+                    mo = fmax(mo, dl / fmin(ri, rj));
                 }
             }
         }
@@ -209,6 +215,7 @@ __global__ void k_force(Dev d, Par c) {
         vv += vi.x * vi.x + vi.y * vi.y + vi.z * vi.z;
     }
     __shared__ double sh[4][32];
+    __shared__ bool s_last;
     for (int o = 16; o; o >>= 1) {
         fv += __shfl_xor_sync(0xffffffffu, fv, o);
         ff += __shfl_xor_sync(0xffffffffu, ff, o);
@@ -222,32 +229,41 @@ __global__ void k_force(Dev d, Par c) {
         double a = 0, b = 0, e = 0, m = 0;
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) { a += sh[0][q]; b += sh[1][q]; e += sh[2][q]; m = fmax(m, sh[3][q]); }
         d.part[blockIdx.x] = make_double4(a, b, e, m);
+        __threadfence();
+        s_last = atomicAdd(&d.s->arrived, 1u) == gridDim.x - 1u;
     }
+    __syncthreads();
+    if (s_last) { __threadfence(); fire_decide(d, c, (int)gridDim.x); }
 }
 
-// FIRE step decision (one block): sums of the block partials in a fixed order (thread t
-// adds partials t, t + blockDim, ...; then a fixed tree), then power, time step and
-// mixing factor on thread 0.
-__global__ void k_fire_decide(Dev d, Par c, int nblocks) {
+// FIRE step decision (256 threads): sums of the block partials in a fixed order -- 1024
+// strided shares, four a thread, then a fixed tree over their 32 groups -- then power, time
+// step and mixing factor on thread 0.
+__device__ __forceinline__ void fire_decide(Dev d, Par c, int nblocks) {
     __shared__ double sh[4][32];
-    double fv = 0, ff = 0, vv = 0, mo = 0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-        const double4 p = d.part[b];
-        fv += p.x; ff += p.y; vv += p.z; mo = fmax(mo, p.w);
-    }
-    for (int o = 16; o; o >>= 1) {
-        fv += __shfl_xor_sync(0xffffffffu, fv, o);
-        ff += __shfl_xor_sync(0xffffffffu, ff, o);
-        vv += __shfl_xor_sync(0xffffffffu, vv, o);
-        mo = fmax(mo, __shfl_xor_sync(0xffffffffu, mo, o));
-    }
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { sh[0][w] = fv; sh[1][w] = ff; sh[2][w] = vv; sh[3][w] = mo; }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        double fv = 0, ff = 0, vv = 0, mo = 0;
+        for (int b = threadIdx.x + 256 * u; b < nblocks; b += 1024) {
+            const double2 p = __ldcg(reinterpret_cast<const double2*>(&d.part[b]));
+            const double2 q = __ldcg(reinterpret_cast<const double2*>(&d.part[b]) + 1);
+            fv += p.x; ff += p.y; vv += q.x; mo = fmax(mo, q.y);
+        }
+        for (int o = 16; o; o >>= 1) {
+            fv += __shfl_xor_sync(0xffffffffu, fv, o);
+            ff += __shfl_xor_sync(0xffffffffu, ff, o);
+            vv += __shfl_xor_sync(0xffffffffu, vv, o);
+            mo = fmax(mo, __shfl_xor_sync(0xffffffffu, mo, o));
+        }
+        if (l == 0) { sh[0][w + 8 * u] = fv; sh[1][w + 8 * u] = ff; sh[2][w + 8 * u] = vv; sh[3][w + 8 * u] = mo; }
+    }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    fv = 0; ff = 0; vv = 0; mo = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) { fv += sh[0][q]; ff += sh[1][q]; vv += sh[2][q]; mo = fmax(mo, sh[3][q]); }
+    double fv = 0, ff = 0, vv = 0, mo = 0;
+    for (int q = 0; q < 32; ++q) { fv += sh[0][q]; ff += sh[1][q]; vv += sh[2][q]; mo = fmax(mo, sh[3][q]); }
     Scal* s = d.s;
+    s->arrived = 0;
     s->fdotv = fv; s->ff = ff; s->vv = vv; s->maxov = mo;
     if (fv > 0) {
         s->npos += 1;
@@ -281,6 +297,9 @@ __global__ void k_fire_update(Dev d, Par c) {
         }
         x.x += v.x * s.dt; x.y += v.y * s.dt; x.z += v.z * s.dt;
         d.x[i] = x; d.v[i] = v;
+        const uint32_t k = cell_of(x, c);        // the next iteration's grid
+        d.key[i] = k;
+        atomicAdd(&d.count[k], 1u);
     }
 }
 
@@ -360,8 +379,8 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
     if (!e) e = al((void**)&d.key, N * 4);
     if (!e) e = al((void**)&d.sorted, N * 4);
     if (!e) e = al((void**)&d.count, (size_t)c.cells * 4);
-    if (!e) e = al((void**)&d.start, (size_t)c.cells * 4);
-    if (!e) e = al((void**)&d.fill, (size_t)c.cells * 4);
+    if (!e) e = al((void**)&d.start, ((size_t)c.cells + 1) * 4);
+    if (!e) e = al((void**)&d.xs, N * sizeof(double4));
     if (!e) e = al((void**)&d.part, nb * sizeof(double4));
     const uint32_t nchunks = (c.cells + SCAN_CHUNK - 1) / SCAN_CHUNK;
     if (!e) e = al((void**)&d.bsum, (size_t)nchunks * sizeof(uint32_t));
@@ -373,6 +392,9 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
     if (!e) e = cudaMemcpyAsync(d.x, hx.data(), N * sizeof(double4), cudaMemcpyHostToDevice, st);
     if (!e) e = cudaMemsetAsync(d.v, 0, N * sizeof(double4), st);
     if (!e) e = cudaMemcpyAsync(d.s, &hs, sizeof(hs), cudaMemcpyHostToDevice, st);
+    // the first iteration's grid; every update counts the next one's
+    if (!e) e = cudaMemsetAsync(d.count, 0, (size_t)c.cells * 4, st);
+    if (!e) { k_bin<<<nb, 256, 0, st>>>(d, c); e = cudaGetLastError(); }
     // one batch of FIRE iterations, captured once and relaunched
     const int BATCH = 50;
     cudaGraph_t graph = nullptr;
@@ -380,15 +402,16 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
     if (!e) e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (!e) {
         for (int it = 0; it < BATCH; ++it) {
-            k_zero<<<(c.cells + 255) / 256, 256, 0, st>>>(d, c);
-            k_bin<<<nb, 256, 0, st>>>(d, c);
-            k_scan_sums<<<nchunks, 256, 0, st>>>(d, c);
-            k_scan_chunks<<<1, 1024, 0, st>>>(d, nchunks);
-            k_scan_apply<<<nchunks, 1024, 0, st>>>(d, c);
+            if (nchunks <= SCAN_SELF) {
+                k_scan_apply<<<nchunks, 1024, 0, st>>>(d, c, 1);
+            } else {
+                k_scan_sums<<<nchunks, 256, 0, st>>>(d, c);
+                k_scan_chunks<<<1, 1024, 0, st>>>(d, nchunks);
+                k_scan_apply<<<nchunks, 1024, 0, st>>>(d, c, 0);
+            }
             k_scatter<<<nb, 256, 0, st>>>(d, c);
             k_cellsort<<<(c.cells + 255) / 256, 256, 0, st>>>(d, c);
             k_force<<<nb, 256, 0, st>>>(d, c);
-            k_fire_decide<<<1, 1024, 0, st>>>(d, c, nb);
             k_fire_update<<<nb, 256, 0, st>>>(d, c);
         }
         e = cudaStreamEndCapture(st, &graph);
