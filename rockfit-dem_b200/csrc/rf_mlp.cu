@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 #include <cstring>
 #include <cmath>
+#include <algorithm>
 #include <vector>
 #include "rf_common.cuh"
 
@@ -317,9 +318,9 @@ extern "C" rf_status rf_gemm_status(rf_stream stream) {
 // Both directions are one kernel each: a tile of 128 rows goes through every layer inside
 // one CTA, its activations never leave shared memory, and a training step's weight
 // gradients stay in tensor memory until the CTA has seen all its tiles. What a step must
-// move is then the features and targets (152 B a row) and the arithmetic is about 235
-// kFLOP a row (0.31 ms at the measured tensor rate for 2M rows). Measured on a B200: a
-// training step on 2M rows 0.97 ms, inference of 300k rows 67 us with the host's wait;
+// move is then the features and targets (152 B a row) and, for the bias sums, dZ (800 B a
+// row, written and read); the arithmetic is about 235 kFLOP a row (0.31 ms at the measured
+// tensor rate for 2M rows). Measured on a B200: a training step on 2M rows 2.3 ms, inference of 300k rows 67 us with the host's wait;
 // layer-by-layer GEMMs with the activations and their transposes in memory took 58 ms and
 // 1.59 ms. What bounds both is the chain of a tile (GEMM, accumulator read, conversion,
 // shared-memory write, barrier, seven times over in training): the tensor cores idle in it.
@@ -349,30 +350,31 @@ static const int NOUT = 6;
 #define MLP_W4 (MLP_W3 + 128 * 128 * 2)
 #define MLP_BIAS (MLP_W4 + 16 * 128 * 2)
 #define MLP_DATA (MLP_BIAS + (3 * 128 + 16) * 4)
-#define MLP_ONES (2 * MLP_CS)               // 16 columns of ones after a tile: the bias gradient's operand
+#define MLP_T_WARPS 16                      // of a training CTA, and the one that issues the MMAs
+#define MLP_T_THREADS (32 * MLP_T_WARPS + 32)
+#define MLP_SPLITS 64                       // splits of a training step's rows (CTAs)
 
 // Shared memory of a training CTA: features, activations H1..H3 (the gradients dZ1..dZ3
-// replace them in place), dZ4; X, H1 and H2 are followed by 16 columns of ones.
+// replace them in place), dZ4.
 #define MLP_T_X MLP_DATA
-#define MLP_T_H1 (MLP_T_X + 8 * MLP_CS + MLP_ONES)
-#define MLP_T_H2 (MLP_T_H1 + 16 * MLP_CS + MLP_ONES)
-#define MLP_T_H3 (MLP_T_H2 + 16 * MLP_CS + MLP_ONES)
+#define MLP_T_H1 (MLP_T_X + 8 * MLP_CS)
+#define MLP_T_H2 (MLP_T_H1 + 16 * MLP_CS)
+#define MLP_T_H3 (MLP_T_H2 + 16 * MLP_CS)
 #define MLP_T_D4 (MLP_T_H3 + 16 * MLP_CS)
 #define MLP_T_SMEM (MLP_T_D4 + 2 * MLP_CS)
 // Shared memory of an inference CTA: one 32 KB activation buffer per warpgroup.
 #define MLP_F_GROUPS 4
 #define MLP_F_SMEM (MLP_DATA + MLP_F_GROUPS * 16 * MLP_CS)
 
-// Tensor memory columns of a training CTA (all 512): the working accumulator, then the
-// gradients dW1^T.. with lane = output, column = input (W4: lane = input, column = output),
-// each of the first three followed by 16 equal columns of the bias gradient.
+// Tensor memory columns of a training CTA: the working accumulator, then the gradients
+// dW1^T.. with lane = output, column = input (W4: lane = input, column = output).
 #define MLP_C_ACC 0
 #define MLP_C_D1 128
-#define MLP_C_D2 (MLP_C_D1 + 80)
-#define MLP_C_D3 (MLP_C_D2 + 144)
-#define MLP_C_D4 (MLP_C_D3 + 144)
-#define MLP_GCOLS 384                       // gradient columns (MLP_C_D1 .. 512)
-static_assert(MLP_C_D4 + 16 == 512, "tensor memory columns");
+#define MLP_C_D2 (MLP_C_D1 + 64)
+#define MLP_C_D3 (MLP_C_D2 + 128)
+#define MLP_C_D4 (MLP_C_D3 + 128)
+#define MLP_GCOLS 336                       // gradient columns
+static_assert(MLP_C_D1 + MLP_GCOLS == MLP_C_D4 + 16 && MLP_C_D4 + 16 <= 512, "tensor memory columns");
 static_assert(MLP_T_SMEM <= 227 * 1024 && MLP_F_SMEM <= 227 * 1024, "shared memory of an SM");
 
 struct MlpWeights {
@@ -380,10 +382,14 @@ struct MlpWeights {
     const float* b[NL];
 };
 
-// Per-CTA sums of a training step besides the gradient columns.
-struct StepSums {
-    double loss;
-    float gb4[NOUT];
+// What a training step leaves for its bias gradients: the rows' output gradients (outputs
+// 0..3 and 4..5) and dZ1..dZ3 in bf16, in the order in which k_mlp_bias adds them: by 8-column
+// group and 32-row share of every 256 rows, so that each of its warps reads one contiguous stream.
+struct BiasRows {
+    float4* dy;              // [8 shares][nk][32 rows]
+    float2* dy2;
+    uint4* dz[3];            // [16 column groups][8 shares][nk][32 rows]
+    long nk;                 // 256-row blocks
 };
 
 __device__ __forceinline__ uint64_t mlp_desc(uint32_t saddr, uint32_t lead, uint32_t stride) {
@@ -441,9 +447,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-// b's halves where h's are positive, else zero (h: activations after ReLU, never negative).
+// b's halves where h's are positive, else zero. h are activations after ReLU (+0 to +inf): adding
+// 0x7FFF sets a half's top bit, with no carry out of it, exactly if the half is not zero, and
+// the byte permutation spreads the two top bits over their halves.
 __device__ __forceinline__ uint32_t mask_bf16(uint32_t b, uint32_t h) {
-    return ((h & 0x7FFFu) ? b & 0xFFFFu : 0u) | ((h & 0x7FFF0000u) ? b & 0xFFFF0000u : 0u);
+    uint32_t m;
+    asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(m) : "r"(h + 0x7FFF7FFFu));
+    return b & m;
+}
+// bf16 of max(a + bias, 0), a pair at once: rounded first, so the larger of the rounded sum and +0
+// (a NaN sum gives 0, as fmaxf does in FP32).
+__device__ __forceinline__ uint32_t relu_pair(uint32_t a0, uint32_t a1, float b0, float b1) {
+    const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(__uint_as_float(a0) + b0, __uint_as_float(a1) + b1),
+                                     __floats2bfloat162_rn(0.f, 0.f));
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // Weights (bf16 [out][in]) and biases into shared memory.
@@ -464,14 +481,13 @@ __device__ __forceinline__ void load_weights(uint8_t* smem, const MlpWeights& w)
 
 // 32 accumulator columns of a row -> bias, ReLU -> four 16-byte pieces of the activations.
 __device__ __forceinline__ void hidden_piece(const uint32_t (&r)[32], const float* bias, uint8_t* dst) {
+    const float4* b4 = reinterpret_cast<const float4*>(bias);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        uint32_t p[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-            p[t] = pack_bf16(fmaxf(__uint_as_float(r[8 * q + 2 * t]) + bias[8 * q + 2 * t], 0.f),
-                             fmaxf(__uint_as_float(r[8 * q + 2 * t + 1]) + bias[8 * q + 2 * t + 1], 0.f));
-        *reinterpret_cast<uint4*>(dst + q * MLP_CS) = make_uint4(p[0], p[1], p[2], p[3]);
+        const float4 u = b4[2 * q], v = b4[2 * q + 1];
+        *reinterpret_cast<uint4*>(dst + q * MLP_CS) =
+            make_uint4(relu_pair(r[8 * q], r[8 * q + 1], u.x, u.y), relu_pair(r[8 * q + 2], r[8 * q + 3], u.z, u.w),
+                       relu_pair(r[8 * q + 4], r[8 * q + 5], v.x, v.y), relu_pair(r[8 * q + 6], r[8 * q + 7], v.z, v.w));
     }
 }
 
@@ -580,21 +596,25 @@ k_mlp_forward(MlpWeights w, const __nv_bfloat16* __restrict__ X, int rows, float
     }
 }
 
-// One training step's forward and backward pass over the CTA's tiles. Eight warps: warp w
-// owns rows 32 (w % 4) .. + 31 of the tile and columns 64 (w / 4) .. + 63 of each layer.
-// The chain of a tile is seven GEMMs, each followed by its epilogue; the weight gradients
-// are issued behind the GEMM the chain waits for and run under its epilogue. part: the
-// CTA's gradient columns [384][128]; sums: its loss and output-bias gradient.
-__global__ void __launch_bounds__(256, 1)
-k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, int rows, int residual,
-            float* __restrict__ part, StepSums* __restrict__ sums, uint32_t* err) {
+// One training step's forward and backward pass over a CTA's split of the rows (`split` rows, a
+// multiple of 64; up to 64 splits). Warp w < 16 owns rows 32 (w % 4) .. + 31 of the tile and
+// columns 32 (w / 4) .. + 31 of each layer; warp 16 issues the MMAs (an issuing thread is held
+// about as long as its MMAs run). The chain of a tile is seven GEMMs, each followed by its
+// epilogue; the weight gradients are issued behind the GEMM the chain waits for and run under
+// its epilogue, as do the stores to memory. part: the CTA's gradient columns [336][128].
+// A split's weight gradients are one tensor-memory accumulation over its rows in order, the
+// splits those of a split-K GEMM over 64-row chunks: the FP32 accumulator's rounding over tens
+// of thousands of rows is the largest error of a step, and with other splits (one per SM, every
+// 148th tile: 0.97 ms a step at 2M rows against 2.3 ms) the gradients moved by 5e-5.
+__global__ void __launch_bounds__(MLP_T_THREADS, 1)
+k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, int rows, long split,
+            int residual, float* __restrict__ part, double* __restrict__ loss_part, BiasRows out_rows, uint32_t* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t s_taddr, s_fail;
     __shared__ double s_loss[4];
-    __shared__ float s_gb[4][NOUT];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+    const int row = (warp & 3) * 32 + lane, quart = warp >> 2;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_taddr)),
                      "r"(512)
@@ -608,11 +628,6 @@ k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __re
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     load_weights(smem, w);
-    for (int q = threadIdx.x; q < 3 * MLP_ONES / 16; q += blockDim.x) {
-        const int b = q / (MLP_ONES / 16), o = q % (MLP_ONES / 16);
-        uint8_t* base = smem + (b == 0 ? MLP_T_X + 8 * MLP_CS : b == 1 ? MLP_T_H1 + 16 * MLP_CS : MLP_T_H2 + 16 * MLP_CS);
-        *reinterpret_cast<uint4*>(base + o * 16) = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-    }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -620,23 +635,20 @@ k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __re
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t sm = smem_u32(smem);
     const float* sb = reinterpret_cast<const float*>(smem + MLP_BIAS);
-    const long ntiles = ((long)rows + MLP_TILE - 1) / MLP_TILE;
+    const long row0 = (long)blockIdx.x * split, row1 = min((long)rows, row0 + split);
     const float inv = 2.0f / ((float)rows * (float)NOUT);
     uint32_t pa = 0, pg = 0;
     bool ok = true;
     double loss = 0.0;
-    float gb4[NOUT];
+    // features of a tile: warp w loads rows 8 w .. + 7, 64 bytes of each at a time
+    const int lr = warp * 8 + (lane & 7), lk = lane >> 3;
+    uint4 xv[2];
+    auto fetch = [&](long first_row) {
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) gb4[c] = 0.f;
-    // features of a tile: warp w loads rows 16 w .. + 15, 8 rows x 64 bytes at a time
-    const int lr = warp * 16 + (lane & 7), lk = lane >> 3;
-    uint4 xv[4];
-    auto fetch = [&](long tile) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const long r = tile * MLP_TILE + lr + (q >> 1) * 8;
+        for (int q = 0; q < 2; ++q) {
+            const long r = first_row + lr;
             xv[q] = make_uint4(0u, 0u, 0u, 0u);
-            if (r < rows) xv[q] = __ldg(reinterpret_cast<const uint4*>(X + (size_t)r * 64) + (q & 1) * 4 + lk);
+            if (r < row1) xv[q] = __ldg(reinterpret_cast<const uint4*>(X + (size_t)r * 64) + q * 4 + lk);
         }
     };
     // shared-memory writes and tensor-memory reads of the stage done: the next MMAs may follow
@@ -656,141 +668,151 @@ k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __re
         pg ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     };
-    fetch(blockIdx.x);
     bool first = true;
-    for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        if (!first) wait_g();                          // the last tile's dW1 has read X
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            *reinterpret_cast<uint4*>(smem + MLP_T_X + ((q & 1) * 4 + lk) * MLP_CS + (lr + (q >> 1) * 8) * 16) = xv[q];
-        stage_sync();
-        ok = s_fail == 0;
-        if (!ok) break;
-        if (threadIdx.x == 0) { mma_forward(tm + MLP_C_ACC, sm + MLP_T_X, sm + MLP_W1, 128, 4); mlp_commit(bar_a); }
-        if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
-        const long gr = tile * MLP_TILE + row;
-        float t[NOUT];
-#pragma unroll
-        for (int c = 0; c < NOUT; ++c) t[c] = (half == 0 && gr < rows) ? __ldg(&T[(size_t)gr * NOUT + c]) : 0.f;
-        // forward: H1, H2, H3
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-            uint8_t* H = smem + (l == 0 ? MLP_T_H1 : l == 1 ? MLP_T_H2 : MLP_T_H3) + half * 8 * MLP_CS + row * 16;
-            wait_a();
-            uint32_t r0[32], r1[32];
-            tmem_ld32(tm + lanes + MLP_C_ACC + half * 64, r0);
-            tmem_ld32(tm + lanes + MLP_C_ACC + half * 64 + 32, r1);
-            tmem_ld_wait();
-            hidden_piece(r0, sb + l * 128 + half * 64, H);
-            hidden_piece(r1, sb + l * 128 + half * 64 + 32, H + 4 * MLP_CS);
+    if (warp == MLP_T_WARPS) {
+        // the MMAs of a tile, each batch after the barrier that its operands' writers reach
+        for (long r0 = row0; r0 < row1; r0 += MLP_TILE) {
             stage_sync();
-            if (threadIdx.x == 0) {
-                if (l == 0) mma_forward(tm + MLP_C_ACC, sm + MLP_T_H1, sm + MLP_W2, 128, 8);
-                if (l == 1) mma_forward(tm + MLP_C_ACC, sm + MLP_T_H2, sm + MLP_W3, 128, 8);
-                if (l == 2) mma_forward(tm + MLP_C_ACC, sm + MLP_T_H3, sm + MLP_W4, 16, 8);
+            ok = s_fail == 0;
+            if (!ok) break;
+            const bool issue = lane == 0;
+            if (issue) { mma_forward(tm + MLP_C_ACC, sm + MLP_T_X, sm + MLP_W1, 128, 4); mlp_commit(bar_a); }
+            stage_sync();
+            if (issue) { mma_forward(tm + MLP_C_ACC, sm + MLP_T_H1, sm + MLP_W2, 128, 8); mlp_commit(bar_a); }
+            stage_sync();
+            if (issue) { mma_forward(tm + MLP_C_ACC, sm + MLP_T_H2, sm + MLP_W3, 128, 8); mlp_commit(bar_a); }
+            stage_sync();
+            if (issue) { mma_forward(tm + MLP_C_ACC, sm + MLP_T_H3, sm + MLP_W4, 16, 8); mlp_commit(bar_a); }
+            stage_sync();
+            if (issue) {
+                mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_D4, sm + MLP_W4, 16);
                 mlp_commit(bar_a);
+                mma_weight_grad(tm + MLP_C_D4, sm + MLP_T_H3, sm + MLP_T_D4, 16, !first);
+                mlp_commit(bar_g);
             }
+            stage_sync();
+            if (issue) {
+                mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_H3, sm + MLP_W3, 128);
+                mlp_commit(bar_a);
+                mma_weight_grad(tm + MLP_C_D3, sm + MLP_T_H3, sm + MLP_T_H2, 128, !first);
+                mlp_commit(bar_g);
+            }
+            stage_sync();
+            if (issue) {
+                mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_H2, sm + MLP_W2, 128);
+                mlp_commit(bar_a);
+                mma_weight_grad(tm + MLP_C_D2, sm + MLP_T_H2, sm + MLP_T_H1, 128, !first);
+                mlp_commit(bar_g);
+            }
+            stage_sync();
+            if (issue) {
+                mma_weight_grad(tm + MLP_C_D1, sm + MLP_T_H1, sm + MLP_T_X, 64, !first);
+                mlp_commit(bar_g);
+            }
+            __syncwarp();
+            first = false;
         }
-        // output, loss and its gradient
-        wait_a();
-        if (half == 0) {
-            float v[16];
-            tmem_ld<16>(tm + lanes + MLP_C_ACC, v);
-            float g[8];
+    } else {
+        fetch(row0);
+        for (long r0 = row0; r0 < row1; r0 += MLP_TILE) {
+            if (!first) wait_g();                          // the last tile's dW1 has read X
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<uint4*>(smem + MLP_T_X + (q * 4 + lk) * MLP_CS + lr * 16) = xv[q];
+            stage_sync();
+            ok = s_fail == 0;
+            if (!ok) break;
+            if (r0 + MLP_TILE < row1) fetch(r0 + MLP_TILE);
+            const long gr = r0 + row;
+            float t[NOUT];
+#pragma unroll
+            for (int c = 0; c < NOUT; ++c) t[c] = (quart == 0 && gr < row1) ? __ldg(&T[(size_t)gr * NOUT + c]) : 0.f;
+            // forward: H1, H2, H3
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                uint8_t* H = smem + (l == 0 ? MLP_T_H1 : l == 1 ? MLP_T_H2 : MLP_T_H3) + quart * 4 * MLP_CS + row * 16;
+                wait_a();
+                uint32_t r[32];
+                tmem_ld32(tm + lanes + MLP_C_ACC + quart * 32, r);
+                tmem_ld_wait();
+                hidden_piece(r, sb + l * 128 + quart * 32, H);
+                stage_sync();
+            }
+            // output, loss and its gradient
+            wait_a();
+            float e[NOUT], g[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) g[c] = 0.f;
-            if (gr < rows) {
+            if (quart == 0) {
+                float v[16];
+                tmem_ld<16>(tm + lanes + MLP_C_ACC, v);
 #pragma unroll
                 for (int c = 0; c < NOUT; ++c) {
                     float y = v[c] + sb[3 * 128 + c];
                     if (residual) y += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(smem + MLP_T_X + row * 16)[c]);
-                    const float e = y - t[c];
-                    loss += (double)e * e;
-                    g[c] = inv * e;
-                    gb4[c] += g[c];
+                    e[c] = y - t[c];
+                    if (gr < row1) g[c] = inv * e[c];
                 }
+                *reinterpret_cast<uint4*>(smem + MLP_T_D4 + row * 16) =
+                    make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), pack_bf16(g[4], g[5]), 0u);
+                *reinterpret_cast<uint4*>(smem + MLP_T_D4 + MLP_CS + row * 16) = make_uint4(0u, 0u, 0u, 0u);
             }
-            *reinterpret_cast<uint4*>(smem + MLP_T_D4 + row * 16) =
-                make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), pack_bf16(g[4], g[5]), pack_bf16(g[6], g[7]));
-            *reinterpret_cast<uint4*>(smem + MLP_T_D4 + MLP_CS + row * 16) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        stage_sync();
-        if (threadIdx.x == 0) {
-            mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_D4, sm + MLP_W4, 16);
-            mlp_commit(bar_a);
-            mma_weight_grad(tm + MLP_C_D4, sm + MLP_T_H3, sm + MLP_T_D4, 16, !first);
-            mlp_commit(bar_g);
-        }
-        // backward: dZ3, dZ2, dZ1 over H3, H2, H1
-#pragma unroll
-        for (int l = 2; l >= 0; --l) {
-            uint8_t* H = smem + (l == 0 ? MLP_T_H1 : l == 1 ? MLP_T_H2 : MLP_T_H3) + half * 8 * MLP_CS + row * 16;
-            wait_a();
-            uint32_t r0[32], r1[32];
-            tmem_ld32(tm + lanes + MLP_C_ACC + half * 64, r0);
-            tmem_ld32(tm + lanes + MLP_C_ACC + half * 64 + 32, r1);
-            tmem_ld_wait();
-            uint4 z[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const uint4 h = *reinterpret_cast<const uint4*>(H + q * MLP_CS);
-                const uint32_t* r = q < 4 ? &r0[8 * q] : &r1[8 * (q - 4)];
-                z[q].x = mask_bf16(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), h.x);
-                z[q].y = mask_bf16(pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])), h.y);
-                z[q].z = mask_bf16(pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), h.z);
-                z[q].w = mask_bf16(pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])), h.w);
-            }
-            wait_g();                                  // the weight gradient has read this buffer
-#pragma unroll
-            for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(H + q * MLP_CS) = z[q];
             stage_sync();
-            if (threadIdx.x == 0) {
-                if (l == 2) {
-                    mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_H3, sm + MLP_W3, 128);
-                    mlp_commit(bar_a);
-                    mma_weight_grad(tm + MLP_C_D3, sm + MLP_T_H3, sm + MLP_T_H2, 144, !first);
-                } else if (l == 1) {
-                    mma_input_grad(tm + MLP_C_ACC, sm + MLP_T_H2, sm + MLP_W2, 128);
-                    mlp_commit(bar_a);
-                    mma_weight_grad(tm + MLP_C_D2, sm + MLP_T_H2, sm + MLP_T_H1, 144, !first);
-                } else {
-                    mma_weight_grad(tm + MLP_C_D1, sm + MLP_T_H1, sm + MLP_T_X, 80, !first);
-                }
-                mlp_commit(bar_g);
-            }
-        }
-        first = false;
-    }
-    if (ok) wait_g();
-    __syncthreads();
-    if (s_fail == 0) {
-        float* out = part + (size_t)blockIdx.x * MLP_GCOLS * 128;
-        for (int cb = half * 32; cb < MLP_GCOLS; cb += 64) {
-            uint32_t r[32];
-            tmem_ld32(tm + lanes + MLP_C_D1 + cb, r);
-            tmem_ld_wait();
+            const size_t at = (((gr >> 5) & 7) * out_rows.nk + (gr >> 8)) * 32 + (gr & 31);     // in a stream
+            if (quart == 0 && gr < row1) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) out[(size_t)(cb + c) * 128 + row] = __uint_as_float(r[c]);
+                for (int c = 0; c < NOUT; ++c) loss += (double)e[c] * e[c];
+                out_rows.dy[at] = make_float4(g[0], g[1], g[2], g[3]);
+                out_rows.dy2[at] = make_float2(g[4], g[5]);
+            }
+            // backward: dZ3, dZ2, dZ1 over H3, H2, H1
+#pragma unroll
+            for (int l = 2; l >= 0; --l) {
+                uint8_t* H = smem + (l == 0 ? MLP_T_H1 : l == 1 ? MLP_T_H2 : MLP_T_H3) + quart * 4 * MLP_CS + row * 16;
+                wait_a();
+                uint32_t r[32];
+                tmem_ld32(tm + lanes + MLP_C_ACC + quart * 32, r);
+                tmem_ld_wait();
+                uint4 z[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint4 h = *reinterpret_cast<const uint4*>(H + q * MLP_CS);
+                    z[q].x = mask_bf16(pack_bf16(__uint_as_float(r[8 * q]), __uint_as_float(r[8 * q + 1])), h.x);
+                    z[q].y = mask_bf16(pack_bf16(__uint_as_float(r[8 * q + 2]), __uint_as_float(r[8 * q + 3])), h.y);
+                    z[q].z = mask_bf16(pack_bf16(__uint_as_float(r[8 * q + 4]), __uint_as_float(r[8 * q + 5])), h.z);
+                    z[q].w = mask_bf16(pack_bf16(__uint_as_float(r[8 * q + 6]), __uint_as_float(r[8 * q + 7])), h.w);
+                }
+                wait_g();                                  // the weight gradient has read this buffer
+#pragma unroll
+                for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(H + q * MLP_CS) = z[q];
+                stage_sync();
+                if (gr < row1) {
+                    uint4* dz = out_rows.dz[l] + (size_t)quart * 4 * 8 * out_rows.nk * 32 + at;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) dz[(size_t)q * 8 * out_rows.nk * 32] = z[q];
+                }
+            }
+            first = false;
         }
-    } else if (threadIdx.x == 0) {
+    }
+    if (ok && warp < MLP_T_WARPS) wait_g();
+    __syncthreads();
+    if (s_fail == 0 && warp < MLP_T_WARPS) {
+        float* out = part + (size_t)blockIdx.x * MLP_GCOLS * 128;
+        for (int cb = quart * 16; cb < MLP_GCOLS; cb += 64) {
+            float v[16];
+            tmem_ld<16>(tm + lanes + MLP_C_D1 + cb, v);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) out[(size_t)(cb + c) * 128 + row] = v[c];
+        }
+    } else if (s_fail && threadIdx.x == 0) {
         atomicOr(err, 1u);
     }
-    for (int o = 16; o; o >>= 1) {
-        loss += __shfl_xor_sync(0xffffffffu, loss, o);
-#pragma unroll
-        for (int c = 0; c < NOUT; ++c) gb4[c] += __shfl_xor_sync(0xffffffffu, gb4[c], o);
-    }
-    if (half == 0 && lane == 0) {
-        s_loss[warp] = loss;
-#pragma unroll
-        for (int c = 0; c < NOUT; ++c) s_gb[warp][c] = gb4[c];
-    }
+    for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (quart == 0 && lane == 0) s_loss[warp] = loss;
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0) sums[blockIdx.x].loss = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
-    if (threadIdx.x < NOUT)
-        sums[blockIdx.x].gb4[threadIdx.x] =
-            (s_gb[0][threadIdx.x] + s_gb[1][threadIdx.x]) + (s_gb[2][threadIdx.x] + s_gb[3][threadIdx.x]);
+    if (threadIdx.x == 0) loss_part[blockIdx.x] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tm), "r"(512) : "memory");
     }
@@ -828,42 +850,95 @@ __device__ __forceinline__ void adam(float* p, float* m, float* v, float g, floa
     *p -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
 }
 
-// Gradients of the step from the CTAs' partials (added in CTA order), then with lr > 0 an
-// Adam step of every weight and bias and the BF16 copies. One thread per gradient column
+// Column sums of a lane's n rows (a stream of 32-row lines) in row order, DEPTH loads in flight.
+template <int DEPTH, typename V, typename F>
+__device__ __forceinline__ void sum_stream(const V* z, int n, F add) {
+    V v[DEPTH];
+#pragma unroll
+    for (int q = 0; q < DEPTH; ++q)
+        if (q < n) v[q] = __ldcs(z + (size_t)q * 32);
+    int k = 0;
+    for (; k + DEPTH <= n; k += DEPTH) {
+#pragma unroll
+        for (int q = 0; q < DEPTH; ++q) {
+            add(v[q]);
+            if (k + DEPTH + q < n) v[q] = __ldcs(z + (size_t)(k + DEPTH + q) * 32);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < DEPTH; ++q)
+        if (k + q < n) add(v[q]);
+}
+
+// Bias gradients: column sums of dY (FP32) and dZ1..dZ3 (bf16) over the rows in FP32, share t of
+// 256 adding rows t, t + 256, ..., then trees over 32 shares (a warp each), then the eight warps'
+// sums in order (k_mlp_update): the order fixes the parallelism at 256 chains a column. One warp
+// a block, eight columns (one 16-byte piece a row) of a hidden layer or up to four of the output
+// layer; 400 warps have to keep the memory busy, so each has 32 rows a lane in flight (2M rows:
+// 0.27 ms, 5.9 TB/s; with 16 rows loaded, then added, and dY in one stream 0.75 ms).
+__global__ void __launch_bounds__(32) k_mlp_bias(BiasRows r, int rows, float* __restrict__ bias_part) {
+    const int b = blockIdx.x >> 3, w = blockIdx.x & 7, l = threadIdx.x, t = w * 32 + l;
+    const int n = (rows - t + 255) / 256;                // rows of this share
+    const size_t at = (size_t)w * r.nk * 32 + l;
+    float s[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) s[c] = 0.f;
+    if (b < 48) {
+        sum_stream<32>(r.dz[b >> 4] + (size_t)(b & 15) * 8 * r.nk * 32 + at, n, [&](const uint4& v) {
+            s[0] += __uint_as_float(v.x << 16); s[1] += __uint_as_float(v.x & 0xFFFF0000u);
+            s[2] += __uint_as_float(v.y << 16); s[3] += __uint_as_float(v.y & 0xFFFF0000u);
+            s[4] += __uint_as_float(v.z << 16); s[5] += __uint_as_float(v.z & 0xFFFF0000u);
+            s[6] += __uint_as_float(v.w << 16); s[7] += __uint_as_float(v.w & 0xFFFF0000u);
+        });
+    } else if (b == 48) {
+        sum_stream<32>(r.dy + at, n, [&](const float4& v) { s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w; });
+    } else {
+        sum_stream<32>(r.dy2 + at, n, [&](const float2& v) { s[4] += v.x; s[5] += v.y; });
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        for (int o = 16; o; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    if (l < 8 && (b < 48 || (l < 4) == (b == 48))) {     // the last two blocks of eight share a group
+        float v = s[0];
+#pragma unroll
+        for (int c = 1; c < 8; ++c) v = l == c ? s[c] : v;
+        bias_part[((size_t)min(b, 48) * 8 + l) * 8 + w] = v;
+    }
+}
+
+// Weight gradients of the step from the CTAs' partials (added in CTA order), then with lr > 0
+// an Adam step of every weight and bias and the BF16 copies. One thread per gradient column
 // entry: consecutive threads read consecutive lanes of each partial.
-__global__ void k_mlp_update(MlpParams p, const float* __restrict__ part, const StepSums* __restrict__ sums, int ncta,
+__global__ void k_mlp_update(MlpParams p, const float* __restrict__ part, const float* __restrict__ bias_part, int ncta,
                              float lr, float b1, float b2, float eps, float c1, float c2) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int col = q >> 7, lane = q & 127;
-    if (col >= MLP_GCOLS) return;
+    if (col >= MLP_GCOLS) {                      // the last block: biases
+        for (int l = 0; l < NL; ++l) {
+            if (l == 3 && lane >= 16) break;
+            float g = 0.f;
+            if (l < 3 || lane < NOUT)
+                for (int w = 0; w < 8; ++w) g += bias_part[((size_t)(l * 16 + (lane >> 3)) * 8 + (lane & 7)) * 8 + w];
+            p.gb[l][lane] = g;
+            if (lr > 0.f && (l < 3 || lane < NOUT))
+                adam(&p.b[l][lane], &p.mb[l][lane], &p.vb[l][lane], g, lr, b1, b2, eps, c1, c2);
+        }
+        return;
+    }
     int l, in, out;
-    bool bias = false;
-    if (col < 80) { l = 0; in = col; out = lane; bias = col == 64; if (col > 64) return; }
-    else if (col < 224) { l = 1; in = col - 80; out = lane; bias = in == 128; if (in > 128) return; }
-    else if (col < 368) { l = 2; in = col - 224; out = lane; bias = in == 128; if (in > 128) return; }
-    else { l = 3; in = lane; out = col - 368; }
+    if (col < 64) { l = 0; in = col; out = lane; }
+    else if (col < 192) { l = 1; in = col - 64; out = lane; }
+    else if (col < 320) { l = 2; in = col - 192; out = lane; }
+    else { l = 3; in = lane; out = col - 320; }
     float g = 0.f;
 #pragma unroll 8
     for (int b = 0; b < ncta; ++b) g += __ldg(&part[((size_t)b * MLP_GCOLS + col) * 128 + lane]);
     const int nin = l == 0 ? 64 : 128, nout = l == 3 ? 16 : 128, nreal = l == 3 ? NOUT : 128;
-    if (bias) {
-        p.gb[l][out] = g;
-        if (lr > 0.f) adam(&p.b[l][out], &p.mb[l][out], &p.vb[l][out], g, lr, b1, b2, eps, c1, c2);
-        return;
-    }
     p.gT[l][(size_t)in * nout + out] = g;
     if (lr > 0.f && out < nreal) {
         const size_t s = (size_t)out * nin + in;
         adam(&p.W[l][s], &p.mW[l][s], &p.vW[l][s], g, lr, b1, b2, eps, c1, c2);
         p.Wb[l][s] = __float2bfloat16_rn(p.W[l][s]);
-    }
-    if (l == 3 && lane == 0) {                   // the output layer's bias
-        float gb = 0.f;
-        if (out < NOUT) {
-            for (int b = 0; b < ncta; ++b) gb += sums[b].gb4[out];
-            if (lr > 0.f) adam(&p.b[3][out], &p.mb[3][out], &p.vb[3][out], gb, lr, b1, b2, eps, c1, c2);
-        }
-        p.gb[3][out] = gb;
     }
 }
 
@@ -873,7 +948,11 @@ __global__ void k_mlp_update(MlpParams p, const float* __restrict__ part, const 
 struct rf_mlp {
     rf::mlp::MlpParams p = {};
     float* part = nullptr;                       // gradient partials of the training CTAs (first training step)
-    rf::mlp::StepSums* sums = nullptr;
+    double* loss_part = nullptr;
+    float* bias_part = nullptr;
+    rf::mlp::BiasRows rows = {};                 // as many rows as the largest step so far
+    void* rows_mem = nullptr;
+    size_t rows_cap = 0;
     __nv_bfloat16* xcopy = nullptr;              // features given at an address that is not 16-byte aligned
     size_t xcopy_rows = 0;
     int sms = 0;
@@ -948,6 +1027,7 @@ rf_status rf_mlp_destroy(rf_mlp* m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     for (void* p : m->allocs) cudaFree(p);
     if (m->xcopy) cudaFree(m->xcopy);
+    if (m->rows_mem) cudaFree(m->rows_mem);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return RF_OK;
@@ -987,8 +1067,23 @@ rf_status rf_mlp_train_step(rf_mlp* m, const void* X, const float* T, int rows, 
     if (!err) { set_error("rf_mlp_train_step: no status word"); return RF_ERR_CUDA; }
     if (!m->part) {
         rf_status st;
-        if ((st = mlp_alloc(m, &m->sums, m->sms)) || (st = mlp_alloc(m, &m->part, (size_t)m->sms * MLP_GCOLS * 128)))
+        if ((st = mlp_alloc(m, &m->loss_part, MLP_SPLITS)) || (st = mlp_alloc(m, &m->bias_part, 49 * 64)) ||
+            (st = mlp_alloc(m, &m->part, (size_t)MLP_SPLITS * MLP_GCOLS * 128)))
             return st;
+    }
+    const size_t rp = ((size_t)rows + 255) / 256 * 256;
+    if (m->rows_cap < rp) {
+        if (m->rows_mem) cudaFree(m->rows_mem);  // (waits for what still uses it)
+        m->rows_mem = nullptr; m->rows_cap = 0;
+        RF_CUDA(cudaMalloc(&m->rows_mem, rp * (24 + 3 * 256)));
+        m->rows_cap = rp;
+    }
+    {
+        char* q = (char*)m->rows_mem;
+        m->rows.dy = (float4*)q;
+        m->rows.dy2 = (float2*)(q + rp * 16);
+        m->rows.nk = (long)(rp / 256);
+        for (int l = 0; l < 3; ++l) m->rows.dz[l] = (uint4*)(q + rp * (24 + l * 256));
     }
     const void* x = X;
     if ((uintptr_t)X % 16 != 0) {                // the kernel's loads take 16 bytes: a copy where they cannot
@@ -1001,9 +1096,12 @@ rf_status rf_mlp_train_step(rf_mlp* m, const void* X, const float* T, int rows, 
         RF_CUDA(cudaMemcpyAsync(m->xcopy, X, (size_t)rows * 64 * 2, cudaMemcpyDeviceToDevice, cs));
         x = m->xcopy;
     }
-    const int ncta = mlp_grid(m, rows);
-    k_mlp_train<<<ncta, 256, MLP_T_SMEM, cs>>>(mlp_weights(m), (const __nv_bfloat16*)x, T, rows, m->residual, m->part,
-                                               m->sums, err);
+    // the rows in splits of whole 64-row chunks, one per 2048 rows up to MLP_SPLITS
+    const long chunks = ((long)rows + 127) / 128 * 2;
+    const long splits = std::max(1l, std::min((long)MLP_SPLITS, chunks / 32)), per = (chunks + splits - 1) / splits;
+    const int ncta = (int)((((long)rows + 63) / 64 + per - 1) / per);    // (the last chunk can be padding alone)
+    k_mlp_train<<<ncta, MLP_T_THREADS, MLP_T_SMEM, cs>>>(mlp_weights(m), (const __nv_bfloat16*)x, T, rows, per * 64, m->residual,
+                                               m->part, m->loss_part, m->rows, err);
     RF_CHECK_LAUNCH("k_mlp_train");
     float c1 = 1.f, c2 = 1.f;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -1012,14 +1110,16 @@ rf_status rf_mlp_train_step(rf_mlp* m, const void* X, const float* T, int rows, 
         c1 = 1.f - std::pow(b1, (float)m->steps);
         c2 = 1.f - std::pow(b2, (float)m->steps);
     }
-    k_mlp_update<<<MLP_GCOLS * 128 / 256, 256, 0, cs>>>(m->p, m->part, m->sums, ncta, lr, b1, b2, 1e-8f, c1, c2);
+    k_mlp_bias<<<50 * 8, 32, 0, cs>>>(m->rows, rows, m->bias_part);
+    RF_CHECK_LAUNCH("k_mlp_bias");
+    k_mlp_update<<<MLP_GCOLS + 1, 128, 0, cs>>>(m->p, m->part, m->bias_part, ncta, lr, b1, b2, 1e-8f, c1, c2);
     RF_CHECK_LAUNCH("k_mlp_update");
-    std::vector<StepSums> h(ncta);
-    RF_CUDA(cudaMemcpyAsync(h.data(), m->sums, ncta * sizeof(StepSums), cudaMemcpyDeviceToHost, cs));
+    std::vector<double> h(ncta);
+    RF_CUDA(cudaMemcpyAsync(h.data(), m->loss_part, ncta * sizeof(double), cudaMemcpyDeviceToHost, cs));
     if (rf_status st = rf_gemm_status((rf_stream)cs)) return st;      // (synchronises the stream)
     if (loss) {
         double t = 0.0;
-        for (const StepSums& q : h) t += q.loss;
+        for (double q : h) t += q;
         *loss = t / ((double)rows * NOUT);
     }
     return RF_OK;

@@ -1,5 +1,5 @@
-"""The fused MLP kernels at the edges of their tiling (128-row tiles, one CTA an SM): row
-counts around a tile and around one and two tiles a CTA, unaligned features, every output
+"""The fused MLP kernels at the edges of their tiling (128-row tiles, up to 64 splits): row
+counts around a tile and a split (133000: the last split would be padding alone), unaligned features, every output
 stride and column count, the residual mode; against the CPU restatement (oracle/mlp_ref.py)
 with the bound of the existing MLP test (BF16 roundings: 2 % of the largest output, 2 %
 relative norm of the gradients)."""
@@ -47,7 +47,8 @@ def _check(torch, rows, offset=0, residual=False):
     m.close()
 
 
-@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128, 148 * 128 + 1, 2 * 148 * 128 + 65, 4 * 148 * 128 + 3])
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128, 148 * 128 + 1, 2 * 148 * 128 + 65, 4 * 148 * 128 + 3,
+                                  133000, 133057])
 def test_mlp_row_counts(cuda, rows):
     _check(cuda, rows)
 
