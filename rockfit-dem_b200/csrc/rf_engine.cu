@@ -1202,17 +1202,17 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 all &= all - 1u;
             }
         }
-        while (m) {                              // four slots' ids, then their positions, in flight
-            uint32_t bit[4], j[4];
-            double4 xj[4];
+        while (m) {                              // two slots' ids, then their positions, in flight
+            uint32_t bit[2], j[2];
+            double4 xj[2];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) { bit[u] = m & (0u - m); m &= m - 1u; }
+            for (int u = 0; u < 2; ++u) { bit[u] = m & (0u - m); m &= m - 1u; }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) j[u] = bit[u] ? row[__ffs(bit[u]) - 1] : i;
+            for (int u = 0; u < 2; ++u) j[u] = bit[u] ? row[__ffs(bit[u]) - 1] : i;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) xj[u] = ldg_d4(&P[j[u]]);
+            for (int u = 0; u < 2; ++u) xj[u] = ldg_d4(&P[j[u]]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 2; ++u) {
                 const double rr = dlen2(dsub(xj[u], xi));
                 const double sr = xi.w + xj[u].w;
                 if (rr > cut2_del(c, xi.w, xj[u].w) || rr < 1e-10) far |= bit[u];
@@ -1249,18 +1249,18 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 4 * SUB) {      // four candidates in flight
-                uint32_t j[4];
-                double4 xj[4];
+            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 2 * SUB) {      // two candidates in flight
+                uint32_t j[2];
+                double4 xj[2];
 #pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) {
+                for (uint32_t u = 0; u < 2; ++u) {
                     const uint32_t q = q0 + u * SUB;
                     j[u] = q < qlim && !((tried >> q) & 1ull) ? __ldg(&d.cand[(size_t)q * N + i]) : i;
                 }
 #pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) xj[u] = ldg_d4(&P[j[u]]);
+                for (uint32_t u = 0; u < 2; ++u) xj[u] = ldg_d4(&P[j[u]]);
 #pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) {
+                for (uint32_t u = 0; u < 2; ++u) {
                     const double rr = dlen2(dsub(xj[u], xi));
                     if (j[u] == i || !(rr < cut2_add(c, xi.w, xj[u].w) && rr > 1e-10)) continue;
                     if (!have_cells) { oc = octant_of(xif, c.g); have_cells = true; }
