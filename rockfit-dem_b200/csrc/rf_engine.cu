@@ -34,6 +34,7 @@
 #include <fstream>
 #include <vector>
 #include <algorithm>
+#include <utility>
 #include <cuda_bf16.h>
 #include "rf_physics.cuh"
 
@@ -2345,8 +2346,7 @@ __global__ void k_count_records(const uint_fast32_t* __restrict__ IL, const uint
 __global__ void k_rows_import(const uint_fast32_t* __restrict__ IL, const uint8_t* __restrict__ type,
                               const float* __restrict__ iL, const rf_float3* __restrict__ Rij,
                               const rf_float3* __restrict__ Oijt, const rf_float3* __restrict__ Mijn,
-                              const rf_float3* __restrict__ Mijt, const double* __restrict__ L0x,
-                              const float2* __restrict__ strx, Dev d, Consts c) {
+                              const rf_float3* __restrict__ Mijt, Dev d, Consts c) {
     const uint_fast32_t E = empty_id<uint_fast32_t>();
     const uint32_t cur = (uint32_t)(d.sc->steps & 1ull);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
@@ -2370,7 +2370,7 @@ __global__ void k_rows_import(const uint_fast32_t* __restrict__ IL, const uint8_
                 const float ox = t1 ? Oijt[r].x : 0.f, oy = t1 ? Oijt[r].y : 0.f, oz = t1 ? Oijt[r].z : 0.f;
                 st8(&d.rec[b].s0, make_float4(Rij[r].x, Rij[r].y, Rij[r].z, ox), make_float4(oy, oz, Mijn[r].x, Mijn[r].y));
                 st8(&d.rec[b].s2, make_float4(Mijn[r].z, Mijt[r].x, Mijt[r].y, Mijt[r].z),
-                    L0x ? rec_const(L0x[r], strx[r]) : make_float4(iL[r], 0.f, 0.f, 0.f));
+                    make_float4(iL[r], 0.f, 0.f, 0.f));
                 if (t1) bmask |= 1u << nq;
                 ++nq;
             }
@@ -2378,7 +2378,7 @@ __global__ void k_rows_import(const uint_fast32_t* __restrict__ IL, const uint8_
         for (uint32_t q = nq; q < d.QB; ++q) {          // unused records: retired, zero
             const size_t b = (size_t)q * c.N + i;
             d.bjk[b] = make_uint2(0u, 0xFFu);
-            d.rec[b].k = L0x ? rec_const(1.0, make_float2(0.f, 0.f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            d.rec[b].k = make_float4(0.f, 0.f, 0.f, 0.f);
             zero_record(d, b);
         }
         d.live[i] = live; d.bond[i] = bond; d.cmask[i] = cm; d.nbq[i] = nq; d.bmask[i] = bmask;
@@ -2441,75 +2441,163 @@ struct BondSpec {
     int ref_mode;               // reference constants: bonds below the centre distance bd, strengths sig, tau
     double bd;
 };
-// Initial rows of the extended model with a list gap g: the reference's construction
-// (md_interaction_list_construct.cu:13-98: the 8 octant cells in visiting order, their
-// occupants in cell order, slots filled in order) with the pair test
-// rr < min(a_farcut, r_i + r_j + g)^2 on the FP64 positions. IL is preset to empty.
-__global__ void k_list_ext(const float* __restrict__ R, const double4* __restrict__ P, uint32_t N,
-                           const uint_fast32_t* __restrict__ CIs, const uint_fast32_t* __restrict__ pnC,
-                           uint_fast32_t* __restrict__ IL, uint32_t K, RefGrid g, double a_farcut, double gap,
-                           uint32_t* err) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        int64_t cells[8];
-        octant_cells(mk3(R[i], R[i + N], R[i + 2 * (size_t)N]), g, cells);
-        const double4 xi = P[i];
-        uint32_t n = 0;
-        for (int c = 0; c < 8; ++c) {
-            if (cells[c] < 0 || (uint64_t)cells[c] >= g.CN) { raise_status(err, RF_ERR_CELL_RANGE); continue; }
-            const uint64_t s = (uint64_t)pnC[cells[c]], cnt = (uint64_t)pnC[cells[c] + g.CN];
-            for (uint64_t m = 0; m < cnt; ++m) {
-                if (s + m >= N) break;
-                const uint_fast32_t j = CIs[s + m + N];
-                if (j >= N) continue;
-                const double4 xj = P[j];
-                const double rr = dlen2(dsub(xj, xi));
-                const double q = fmin(a_farcut, (xi.w + xj.w) + gap);
-                if (rr < q * q && j != i) {
-                    if (n < K) IL[(size_t)i * K + n] = j;
-                    else raise_status(err, RF_ERR_ROW_OVERFLOW);
-                    ++n;
+// Initial rows of an engine, in the reference's construction order (md_interaction_list_
+// construct.cu:13-98: the 8 octant cells in visiting order, their occupants in cell order, slots
+// filled in order), by eight lanes a particle as md_InteractionListConstruct builds them, but
+// straight into the engine's rows. gap < 0: pairs with float |r|^2 < aacut (the reference's
+// test); else the extended model's pair test |r| < min(a_farcut, r_i + r_j + gap) on the FP64
+// positions. Nothing of a row exists in the reference layout in between: seven FP32 triples a
+// slot, their zeroing and about 60 allocations were most of a creation. Creation, an affine
+// strain, 100 steps and the read-back of 200k particles: 42 -> 18 ms.
+__global__ void __launch_bounds__(128) k_rows_list(const float* __restrict__ R, Dev d, Consts c,
+                                                   const uint_fast32_t* __restrict__ CIs,
+                                                   const uint_fast32_t* __restrict__ pnC, double a_farcut, double gap,
+                                                   uint32_t* err) {
+    const size_t N = c.N;
+    const int sub = threadIdx.x & 7;
+    const size_t i = (size_t)blockIdx.x * 16 + (threadIdx.x >> 3);
+    const bool valid = i < N;
+    f3 xi = mk3(0.f, 0.f, 0.f);
+    double4 xd = make_double4(0, 0, 0, 0);
+    uint64_t s = 0, cnt = 0;
+    if (valid) {
+        xi = mk3(R[i], R[i + N], R[i + 2 * N]);
+        if (gap >= 0.0) xd = d.posd[0][i];
+        const int64_t cell = octant_cell(octant_of(xi, c.g), sub);
+        if (cell < 0 || (uint64_t)cell >= c.g.CN) raise_status(err, RF_ERR_CELL_RANGE);
+        else { s = (uint64_t)pnC[cell]; cnt = (uint64_t)pnC[cell + c.g.CN]; }
+        if (s > N) s = N;
+        if (cnt > N - s) cnt = N - s;
+    }
+    auto hit = [&](uint64_t m, uint32_t& j) {
+        const uint_fast32_t id = CIs[s + m + N];
+        if (id >= N || id == i) return false;
+        j = (uint32_t)id;
+        if (gap >= 0.0) {
+            const double4 xj = ldg_d4(&d.posd[0][j]);
+            const double q = fmin(a_farcut, (xd.w + xj.w) + gap);
+            return dlen2(dsub(xj, xd)) < q * q;
+        }
+        return dist2_rn(xi, mk3(R[j], R[j + N], R[j + 2 * N])) < c.aacut;
+    };
+    uint32_t n = 0, j = 0;
+    for (uint64_t m = 0; m < cnt; ++m) n += hit(m, j) ? 1u : 0u;
+    uint32_t at = n;
+    for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, at, o, 8);
+        if (sub >= o) at += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, at, 7, 8);
+    at -= n;
+    if (!valid) return;
+    uint32_t* row = d.ids + i * c.K;
+    if (n && at + n > c.K) raise_status(err, RF_ERR_ROW_OVERFLOW);
+    for (uint64_t m = 0; n && m < cnt; ++m)
+        if (hit(m, j)) {
+            if (at < c.K) row[at] = j;
+            ++at; --n;
+        }
+    for (uint32_t k = total + sub; k < c.K; k += 8) row[k] = EMPTY32;
+    if (sub == 0) d.live[i] = total >= 32u ? 0xffffffffu : (1u << total) - 1u;
+}
+
+// Bonds of the rows, a warp a particle and a lane a slot. Reference model: pairs below the
+// squared length aa_create, 1/L0 = rsqrt(|r|^2) (md_boundinteractions_construct.cu). Extended
+// model: gap below gap_frac * min(r_i, r_j) (or, in the reference-constants mode, centre
+// distance below b_d), with the FP64 rest length and the pair's strengths. aa_far > 0: then
+// DeleteFarLinks on the float positions, as the drivers run it before their first step.
+// PASS 0 finds the rows' bonds and the most of any row (the record planes to allocate); PASS 1
+// writes the records, the per-slot 1/L0 and the particles' masks.
+template <int PASS>
+__global__ void __launch_bounds__(128) k_rows_bonds(const float* __restrict__ R, Dev d, Consts c, float aa_create, float aa_far,
+                                                    const BondSpec* __restrict__ bs, uint32_t nspec, uint32_t* maxq) {
+    __shared__ float s_il[32][33];
+    const uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
+    const size_t N = c.N, i0 = (size_t)blockIdx.x * 32;
+    uint32_t most = 0;
+    for (uint32_t u = wp; u < 32u; u += 4u) {
+        const size_t i = i0 + u;
+        float il = 0.f;
+        if (i < N) {
+            const f3 xi = mk3(R[i], R[i + N], R[i + 2 * N]);
+            uint32_t live = d.live[i];
+            const bool occ = lane < c.K && ((live >> lane) & 1u);
+            const uint32_t j = occ ? d.ids[i * c.K + lane] : 0u;
+            bool bond = false, far = false;
+            double L = 1.0;
+            float2 str = make_float2(0.f, 0.f);
+            if (occ) {
+                const f3 xj = mk3(R[j], R[j + N], R[j + 2 * N]);
+                if (c.ext) {
+                    uint32_t sp = 0;
+                    while (sp + 1 < nspec && i >= bs[sp].p1) ++sp;
+                    const BondSpec& B = bs[sp];
+                    const double4 a = ldg_d4(&d.posd[0][i]), b = ldg_d4(&d.posd[0][j]);
+                    const double dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+                    const double len = sqrt(dx * dx + dy * dy + dz * dz);
+                    // md_boundinteractions_construct.cu:62 on the FP64 distance in the reference-constants mode
+                    bond = (B.ref_mode ? len < B.bd : len - a.w - b.w < B.gap_frac * fmin(a.w, b.w)) && len > 0;
+                    if (bond) {
+                        il = (float)(1.0 / len);
+                        L = len;
+                        if (PASS == 1) {
+                            if (B.ref_mode) {
+                                str = make_float2((float)B.sig, (float)B.tau);
+                            } else {
+                                // strengths keyed on specimen-local ids
+                                const double inv_m = 1.0 / B.wm;
+                                const uint32_t li = (uint32_t)i - B.p0, lj = j - B.p0;
+                                const double us = pair_uniform(B.seed, li, lj, 0), ut = pair_uniform(B.seed, li, lj, 1);
+                                str = make_float2((float)(B.sig * pow(-log(us), inv_m)), (float)(B.tau * pow(-log(ut), inv_m)));
+                            }
+                        }
+                    }
+                } else {
+                    const float rm2 = rm2_bond(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z);
+                    bond = rm2 < aa_create && (double)rm2 > 1e-18;
+                    if (bond) il = __frsqrt_rn(rm2);
+                }
+                if (aa_far > 0.f) {
+                    const float rr = dist2_rn(xi, xj);
+                    far = rr > aa_far || below_1em10(rr);
+                }
+            }
+            const uint32_t bm = __ballot_sync(FULL, bond && !far), fm = __ballot_sync(FULL, far);
+            const uint32_t nq = __popc(bm);
+            most = max(most, nq);
+            if (PASS == 1) {
+                if (far) d.ids[i * c.K + lane] = EMPTY32;
+                if ((bm >> lane) & 1u) {
+                    const size_t b = (size_t)__popc(bm & ((1u << lane) - 1u)) * N + i;
+                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                    d.bjk[b] = make_uint2(j, lane);
+                    st8(&d.rec[b].s0, z, z);
+                    st8(&d.rec[b].s2, z, c.ext ? rec_const(L, str) : make_float4(il, 0.f, 0.f, 0.f));
+                }
+                for (uint32_t q = nq + lane; q < d.QB; q += 32u) {         // unused records: retired, zero
+                    const size_t b = (size_t)q * N + i;
+                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                    d.bjk[b] = make_uint2(0u, 0xFFu);
+                    st8(&d.rec[b].s0, z, z);
+                    st8(&d.rec[b].s2, z, c.ext ? rec_const(1.0, make_float2(0.f, 0.f)) : z);
+                }
+                if (lane == 0) {
+                    live &= ~fm;
+                    d.live[i] = live; d.bond[i] = bm; d.cmask[i] = 0u; d.nbq[i] = nq;
+                    d.bmask[i] = nq >= 32u ? 0xffffffffu : (1u << nq) - 1u;
                 }
             }
         }
+        if (PASS == 1) s_il[u][lane] = il;
     }
-}
-
-__global__ void k_bond_ext(const double4* __restrict__ P, const uint_fast32_t* __restrict__ IL,
-                           uint8_t* __restrict__ type, float* __restrict__ iL, double* __restrict__ L0x,
-                           float2* __restrict__ strx, uint32_t N, uint32_t K, const BondSpec* __restrict__ bs,
-                           uint32_t nspec) {
-    const uint_fast32_t E = empty_id<uint_fast32_t>();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        uint32_t sp = 0;
-        while (sp + 1 < nspec && i >= bs[sp].p1) ++sp;
-        const double gap_frac = bs[sp].gap_frac, sig = bs[sp].sig, tau = bs[sp].tau;
-        const double inv_m = 1.0 / bs[sp].wm;
-        const uint64_t seed = bs[sp].seed;
-        const uint32_t pbase = bs[sp].p0;       // strengths keyed on specimen-local ids
-        const double4 xi = P[i];
-        for (uint32_t k = 0; k < K; ++k) {
-            const size_t r = (size_t)i * K + k;
-            const uint_fast32_t j = IL[r];
-            type[r] = 0; iL[r] = 0.f; L0x[r] = 1.0; strx[r] = make_float2(0.f, 0.f);
-            if (j == E || j >= N) continue;
-            const double4 xj = P[j];
-            const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            const double L = sqrt(dx * dx + dy * dy + dz * dz);
-            if (bs[sp].ref_mode) {
-                // md_boundinteractions_construct.cu:62 (on the FP64 distance), global strengths
-                if (!(L < bs[sp].bd) || !(L > 0)) continue;
-            } else if (!(L - xi.w - xj.w < gap_frac * fmin(xi.w, xj.w)) || !(L > 0)) {
-                continue;
-            }
-            type[r] = 1;
-            iL[r] = (float)(1.0 / L);
-            L0x[r] = L;
-            if (bs[sp].ref_mode) { strx[r] = make_float2((float)sig, (float)tau); continue; }
-            const uint32_t li = i - pbase, lj = (uint32_t)j - pbase;
-            const double us = pair_uniform(seed, li, lj, 0), ut = pair_uniform(seed, li, lj, 1);
-            strx[r] = make_float2((float)(sig * pow(-log(us), inv_m)), (float)(tau * pow(-log(ut), inv_m)));
-        }
+    if (PASS == 0) {
+        if (lane == 0 && most > *(volatile uint32_t*)maxq) atomicMax(maxq, most);
+        return;
     }
+    __syncthreads();
+    for (uint32_t k = wp; k < c.K; k += 4u)
+        if (i0 + lane < N) d.il[(size_t)k * N + i0 + lane] = s_il[lane][k];
 }
 __global__ void k_posd_from_planar(const double* __restrict__ R, const double* __restrict__ rad, uint32_t N,
                                    double4* __restrict__ out, float* __restrict__ Rf) {
@@ -2533,14 +2621,17 @@ __global__ void k_posd_to_planar_f(const double4* __restrict__ in, uint32_t N, f
 }
 
 __global__ void k_counters(Dev d, Consts c, unsigned long long* out) {
-    unsigned long long nb = 0, nc = 0, nl = 0;
+    uint32_t nb = 0, nc = 0, nl = 0;              // (a warp's share: below 2^32)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
-        const uint32_t l = d.live[i], b = d.bond[i];
-        nl += __popc(l); nb += __popc(b); nc += __popc(d.cmask[i]);
+        nl += __popc(d.live[i]); nb += __popc(d.bond[i]); nc += __popc(d.cmask[i]);
     }
-    atomicAdd(&out[0], nb); atomicAdd(&out[1], nc); atomicAdd(&out[2], nl);
+    nb = __reduce_add_sync(0xffffffffu, nb); nc = __reduce_add_sync(0xffffffffu, nc); nl = __reduce_add_sync(0xffffffffu, nl);
+    if ((threadIdx.x & 31) == 0) {
+        if (nb) atomicAdd(&out[0], (unsigned long long)nb);
+        if (nc) atomicAdd(&out[1], (unsigned long long)nc);
+        if (nl) atomicAdd(&out[2], (unsigned long long)nl);
+    }
 }
-
 
 __global__ void k_set_target(DevScalars* sc, unsigned long long n) { sc->target = sc->steps + n; }
 __global__ void k_force_rebuild(DevScalars* sc) { sc->rebuild = 1u; }
@@ -2655,12 +2746,28 @@ struct rf_engine {
 
 namespace {
 
-template <class T> rf_status dalloc(rf_engine* e, T** p, size_t n) {
+// A set of device arrays in one allocation, each on a 256-byte boundary: an allocation and its
+// free cost about 0.1 ms each, and an engine has some sixty arrays.
+struct Arrays {
+    std::vector<std::pair<void**, size_t>> list;
+    size_t bytes = 0;
+    template <class T> void add(T** p, size_t n) {
+        list.push_back({(void**)p, bytes});
+        bytes += ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+    }
+    cudaError_t alloc(void** base) const {
+        *base = nullptr;
+        const cudaError_t ce = cudaMalloc(base, bytes);
+        if (!ce) for (auto& a : list) *a.first = (char*)*base + a.second;
+        return ce;
+    }
+};
+// ... owned by an engine
+rf_status dalloc(rf_engine* e, const Arrays& a) {
     void* q = nullptr;
-    RF_CUDA(cudaMalloc(&q, (n ? n : 1) * sizeof(T)));
+    RF_CUDA(a.alloc(&q));
     e->allocs.push_back(q);
-    e->alloc_bytes.push_back((n ? n : 1) * sizeof(T));
-    *p = (T*)q;
+    e->alloc_bytes.push_back(a.bytes);
     return RF_OK;
 }
 
@@ -3082,23 +3189,27 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
     Dev& d = e->d;
     d.n_particles = N;
     const size_t NK = (size_t)N * K;
-    for (int b = 0; b < 2; ++b) {
-        if ((ext ? (st = dalloc(e, &d.posd[b], N)) : (st = dalloc(e, &d.pos[b], N))) ||
-            (st = dalloc(e, &d.vw[b], N)))
-            return fail(st);
+    SpecGeom* dgeom = nullptr;
+    uint16_t* dblk = nullptr;
+    {
+        Arrays A;
+        for (int b = 0; b < 2; ++b) {
+            if (ext) A.add(&d.posd[b], N); else A.add(&d.pos[b], N);
+            A.add(&d.vw[b], N);
+            A.add(&d.cO[b], 3 * NK);
+        }
+        A.add(&d.ids, NK); A.add(&d.il, NK);
+        A.add(&d.live, N); A.add(&d.bond, N); A.add(&d.cmask, N); A.add(&d.nbq, N); A.add(&d.bmask, N); A.add(&e->maxq_dev, 1);
+        A.add(&d.cand, (size_t)c.KC * N); A.add(&d.cand_n, N); A.add(&d.member, N);
+        A.add(&d.pos_ref, N); A.add(&d.cmargin, N); A.add(&d.cbound, N); A.add(&d.cg_key, N);
+        A.add(&d.cg_count, cells + 1); A.add(&d.cg_start, cells + 1); A.add(&d.cg_fill, cells + 1);
+        A.add(&d.cg_bsum, e->cg_nb); A.add(&d.cg_sorted, N); A.add(&d.cg_slot, N); A.add(&d.cg_pos, N);
+        A.add(&d.partial, e->ncta); A.add(&d.partial2, e->ncta); A.add(&d.nz, nzw); A.add(&d.nz2, nzw);
+        A.add(&d.curve, 3 * (size_t)c.curve_cap * nspec); A.add(&d.sc, 1); A.add(&e->counters_dev, 4);
+        A.add(&dgeom, nspec);
+        if (nspec > 1) { A.add(&dblk, e->nblocks); A.add(&d.spec, nspec); }
+        if ((st = dalloc(e, A))) return fail(st);
     }
-    if ((st = dalloc(e, &d.ids, NK)) || (st = dalloc(e, &d.il, NK)) || (st = dalloc(e, &d.cO[0], 3 * NK)) || (st = dalloc(e, &d.cO[1], 3 * NK)) ||
-        (st = dalloc(e, &d.live, N)) || (st = dalloc(e, &d.bond, N)) || (st = dalloc(e, &d.cmask, N)) ||
-        (st = dalloc(e, &d.nbq, N)) || (st = dalloc(e, &d.bmask, N)) || (st = dalloc(e, &e->maxq_dev, 1)) ||
-        (st = dalloc(e, &d.cand, (size_t)c.KC * N)) || (st = dalloc(e, &d.cand_n, N)) || (st = dalloc(e, &d.member, N)) ||
-        (st = dalloc(e, &d.pos_ref, N)) || (st = dalloc(e, &d.cmargin, N)) || (st = dalloc(e, &d.cbound, N)) || (st = dalloc(e, &d.cg_key, N)) || (st = dalloc(e, &d.cg_count, cells + 1)) ||
-        (st = dalloc(e, &d.cg_start, cells + 1)) || (st = dalloc(e, &d.cg_fill, cells + 1)) ||
-        (st = dalloc(e, &d.cg_bsum, e->cg_nb)) || (st = dalloc(e, &d.cg_sorted, N)) || (st = dalloc(e, &d.cg_slot, N)) || (st = dalloc(e, &d.cg_pos, N)) ||
-        (st = dalloc(e, &d.partial, e->ncta)) || (st = dalloc(e, &d.partial2, e->ncta)) ||
-        (st = dalloc(e, &d.nz, nzw)) || (st = dalloc(e, &d.nz2, nzw)) ||
-        (st = dalloc(e, &d.curve, 3 * (size_t)c.curve_cap * nspec)) ||
-        (st = dalloc(e, &d.sc, 1)) || (st = dalloc(e, &e->counters_dev, 4)))
-        return fail(st);
     cudaStream_t s = e->stream;
     for (int b = 0; b < 2; ++b) {
         if (cudaMemsetAsync(d.vw[b], 0, N * sizeof(F8), s))
@@ -3117,10 +3228,8 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
             G.p0 = bin ? bin->p0[q] : 0u;
             G.p1 = bin ? bin->p0[q] + bin->n[q] : N;
         }
-        SpecGeom* dg = nullptr;
-        if ((st = dalloc(e, &dg, nspec))) return fail(st);
-        if (cudaMemcpyAsync(dg, hg.data(), nspec * sizeof(SpecGeom), cudaMemcpyHostToDevice, s)) return fail(RF_ERR_CUDA);
-        d.geom = dg;
+        if (cudaMemcpyAsync(dgeom, hg.data(), nspec * sizeof(SpecGeom), cudaMemcpyHostToDevice, s)) return fail(RF_ERR_CUDA);
+        d.geom = dgeom;
         d.blk_spec = nullptr;
         if (nspec > 1) {
             std::vector<uint16_t> hb(e->nblocks);
@@ -3129,12 +3238,9 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
                 while (q + 1 < nspec && hg[q].p1 <= b * 128u) ++q;
                 hb[b] = (uint16_t)q;
             }
-            uint16_t* db = nullptr;
-            if ((st = dalloc(e, &db, e->nblocks))) return fail(st);
-            if (cudaMemcpyAsync(db, hb.data(), e->nblocks * sizeof(uint16_t), cudaMemcpyHostToDevice, s))
+            if (cudaMemcpyAsync(dblk, hb.data(), e->nblocks * sizeof(uint16_t), cudaMemcpyHostToDevice, s))
                 return fail(RF_ERR_CUDA);
-            d.blk_spec = db;
-            if ((st = dalloc(e, &d.spec, nspec))) return fail(st);
+            d.blk_spec = dblk;
             std::vector<DevScalars> hs(nspec);
             for (uint32_t k = 0; k < nspec; ++k) {
                 fill_scalars(hs[k], bin->tasks[k]);
@@ -3157,129 +3263,99 @@ rf_status engine_create_impl(const rf_task* t, const float* h_R, const double* h
         cudaMemsetAsync(d.sc, 0, sizeof(DevScalars), s))
         return fail(RF_ERR_CUDA);
 
-    // Initial rows exactly as the drivers build them (md_calculationbraziltest.cu:132-144),
-    // with the md_* kernels on temporary reference-layout buffers.
+    // Initial rows exactly as the drivers build them (md_calculationbraziltest.cu:132-144): the
+    // binning of md_CellDistribution, then lists, bonds and DeleteFarLinks straight into the
+    // engine's rows and records; or rows given in the reference layout.
     {
-        float *dR = nullptr, *dV = nullptr, *dIL_f = nullptr;
+        float* dR = nullptr;
         uint_fast32_t *dCI = nullptr, *dCIs = nullptr, *dpnC = nullptr, *dIL = nullptr;
         uint8_t* dT = nullptr;
+        float* dIL_f = nullptr;
         rf_float3* dS = nullptr;
-        double *dRd = nullptr, *dRad = nullptr, *dL0 = nullptr;
-        float2* dStr = nullptr;
-        void* scratch = nullptr;
+        double *dRd = nullptr, *dRad = nullptr;
+        BondSpec* dbs = nullptr;
+        char* scratch = nullptr;
         const size_t sb = md_CellDistributionScratchBytes(N, t->C.N);
-        cudaError_t ce = cudaSuccess;
-        ce = cudaMalloc(&dR, 3 * (size_t)N * sizeof(float));
-        if (!ce) ce = cudaMalloc(&dV, 3 * (size_t)N * sizeof(float));
-        if (!ce) ce = cudaMalloc(&dCI, N * sizeof(uint_fast32_t));
-        if (!ce) ce = cudaMalloc(&dCIs, 2 * (size_t)N * sizeof(uint_fast32_t));
-        if (!ce) ce = cudaMalloc(&dpnC, 2 * t->C.N * sizeof(uint_fast32_t));
-        if (!ce) ce = cudaMalloc(&dIL, NK * sizeof(uint_fast32_t));
-        if (!ce) ce = cudaMalloc(&dT, NK);
-        if (!ce) ce = cudaMalloc(&dIL_f, NK * sizeof(float));
-        if (!ce) ce = cudaMalloc(&dS, 7 * NK * sizeof(rf_float3));
-        if (!ce) ce = cudaMalloc(&scratch, sb);
-        if (ext) {
-            if (!ce) ce = cudaMalloc(&dRd, 3 * (size_t)N * sizeof(double));
-            if (!ce) ce = cudaMalloc(&dRad, (size_t)N * sizeof(double));
-            if (!ce) ce = cudaMalloc(&dL0, NK * sizeof(double));
-            if (!ce) ce = cudaMalloc(&dStr, NK * sizeof(float2));
-            if (!ce) ce = cudaMemcpyAsync(dRd, h_Rd, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice, s);
+        Arrays A;
+        A.add(&dR, 3 * (size_t)N); A.add(&dCI, N); A.add(&dCIs, 2 * (size_t)N); A.add(&dpnC, 2 * t->C.N);
+        A.add(&scratch, sb); A.add(&dbs, nspec);
+        if (ext) { A.add(&dRd, 3 * (size_t)N); A.add(&dRad, N); }
+        if (rows) { A.add(&dIL, NK); A.add(&dT, NK); A.add(&dIL_f, NK); A.add(&dS, 4 * NK); }
+        void* tmp = nullptr;
+        cudaError_t ce = A.alloc(&tmp);
+        if (!ce && ext) {
+            ce = cudaMemcpyAsync(dRd, h_Rd, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice, s);
             if (!ce) ce = cudaMemcpyAsync(dRad, h_rad, (size_t)N * sizeof(double), cudaMemcpyHostToDevice, s);
             if (!ce) { k_posd_from_planar<<<(N + 255) / 256, 256, 0, s>>>(dRd, dRad, N, d.posd[0], dR); ce = cudaGetLastError(); }
         } else if (!ce) {
             ce = cudaMemcpyAsync(dR, h_R, 3 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, s);
+            if (!ce) { k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(dR, N, d.pos[0], 1u); ce = cudaGetLastError(); }
         }
-        if (!ce) ce = cudaMemsetAsync(dV, 0, 3 * (size_t)N * sizeof(float), s);
-        if (!ce) ce = cudaMemsetAsync(dT, 0, NK, s);
-        if (!ce) ce = cudaMemsetAsync(dIL_f, 0, NK * sizeof(float), s);
-        if (!ce) ce = cudaMemsetAsync(dS, 0, 7 * NK * sizeof(rf_float3), s);
         rf_status st2 = ce ? cuda_status(ce, "engine init buffers") : RF_OK;
-        rf_float3 *Rij = dS, *Oijt = dS + NK, *Fijn = dS + 2 * NK, *Fijt = dS + 3 * NK, *Mijn = dS + 4 * NK,
-                  *Mijt = dS + 5 * NK, *Mijadd = dS + 6 * NK;
         rf_status init_dev = RF_OK;
         if (!st2) {
             rf_status a = md_CellDistribution(dR, N, dCI, dCIs, dpnC, t->C.N, t->C._1d_a, t->C.Nr, scratch, sb, s);
             if (a != RF_OK && a != RF_ERR_CELL_RANGE && a != RF_ERR_ROW_OVERFLOW) st2 = a; else if (a) init_dev = a;
         }
         const bool pair_cut = ext && x->list_gap > 0.0;
+        uint32_t qb = 0;
+        std::vector<BondSpec> hbs(nspec);
         if (!st2 && rows) {
             ce = cudaMemcpyAsync(dIL, rows->IL, NK * sizeof(uint_fast32_t), cudaMemcpyHostToDevice, s);
             if (!ce) ce = cudaMemcpyAsync(dT, rows->ILtype, NK, cudaMemcpyHostToDevice, s);
             if (!ce) ce = cudaMemcpyAsync(dIL_f, rows->iL, NK * sizeof(float), cudaMemcpyHostToDevice, s);
             const rf_float3* src[4] = {rows->Rij, rows->Oijt, rows->Mijn, rows->Mijt};
-            rf_float3* dst[4] = {Rij, Oijt, Mijn, Mijt};
             for (int q = 0; q < 4 && !ce; ++q)
-                ce = cudaMemcpyAsync(dst[q], src[q], NK * sizeof(rf_float3), cudaMemcpyHostToDevice, s);
+                ce = cudaMemcpyAsync(dS + q * NK, src[q], NK * sizeof(rf_float3), cudaMemcpyHostToDevice, s);
+            if (!ce) ce = cudaMemsetAsync(e->maxq_dev, 0, sizeof(uint32_t), s);
+            if (!ce) { k_count_records<<<148 * 4, 256, 0, s>>>(dIL, dT, dS, N, K, e->maxq_dev); ce = cudaGetLastError(); }
+            if (!ce) ce = cudaMemcpyAsync(&qb, e->maxq_dev, sizeof(qb), cudaMemcpyDeviceToHost, s);
+            if (!ce) ce = cudaStreamSynchronize(s);
             if (ce) st2 = cuda_status(ce, "engine rows");
         }
-        if (!st2 && !pair_cut && !rows) {
-            rf_status a = md_InteractionListConstruct(dR, N, dCIs, dpnC, dIL, K, t->C.a, t->C._1d_a, t->aacut,
-                                                      t->C.Nr, t->C.N, s);
-            if (a != RF_OK && a != RF_ERR_CELL_RANGE && a != RF_ERR_ROW_OVERFLOW) st2 = a; else if (a && !init_dev) init_dev = a;
-        }
-        if (!st2 && pair_cut) {
-            uint32_t w = 0;
-            ce = cudaMemsetAsync(dIL, 0xFF, NK * sizeof(uint_fast32_t), s);
-            if (!ce) ce = cudaMemsetAsync(e->maxq_dev, 0, sizeof(uint32_t), s);
-            if (!ce) {
-                k_list_ext<<<(N + 127) / 128, 128, 0, s>>>(dR, d.posd[0], N, dCIs, dpnC, dIL, K, c.g, P.a_farcut,
-                                                           x->list_gap, e->maxq_dev);
-                ce = cudaGetLastError();
-            }
-            if (!ce) ce = cudaMemcpyAsync(&w, e->maxq_dev, sizeof(w), cudaMemcpyDeviceToHost, s);
-            if (!ce) ce = cudaStreamSynchronize(s);
-            if (ce) st2 = cuda_status(ce, "k_list_ext");
-            else if (w && !init_dev) init_dev = (rf_status)w;
-        }
-        if (!st2 && !ext && !rows) st2 = md_ConstructBoundInteractions(dR, dV, dV, dIL, dT, dIL_f, Rij, Oijt, Fijn, Fijt, Mijn, Mijt,
-                                                              Mijadd, N, K, (float)P.b_dd, (float)P.b_r, s);
-        if (!st2 && ext) {
-            std::vector<BondSpec> hbs(nspec);
+        // (with a list gap every listed pair is within its cutoff: nothing to delete)
+        const float aa_create = (float)P.b_dd, aa_far = pair_cut ? 0.f : (float)P.aa_farcut;
+        if (!st2 && !rows) {
+            uint32_t w[2] = {0, 0};                  // status of the lists, most bonds of a row
             for (uint32_t q = 0; q < nspec; ++q) {
+                if (!ext) { hbs[q] = BondSpec{}; continue; }
                 const rf_ext_params& xq = bin ? bin->xs[q] : *x;
                 const rf_task& tq = bin ? bin->tasks[q] : *t;
                 hbs[q] = BondSpec{xq.gap_frac, xq.weibull_m, xq.sigma_c, xq.tau_c, xq.seed, bin ? bin->p0[q] : 0u,
                                   bin ? bin->p0[q] + bin->n[q] : N, xq.ref_mode, tq.Po.b_d};
                 if (xq.ref_mode) { hbs[q].sig = tq.Po.m_Ec; hbs[q].tau = tq.Po.m_Gc; hbs[q].wm = 1.0; }
             }
-            BondSpec* dbs = nullptr;
-            ce = cudaMalloc(&dbs, nspec * sizeof(BondSpec));
-            if (!ce) ce = cudaMemcpyAsync(dbs, hbs.data(), nspec * sizeof(BondSpec), cudaMemcpyHostToDevice, s);
+            uint32_t* dw = (uint32_t*)e->counters_dev;
+            ce = cudaMemcpyAsync(dbs, hbs.data(), nspec * sizeof(BondSpec), cudaMemcpyHostToDevice, s);
+            if (!ce) ce = cudaMemsetAsync(dw, 0, 2 * sizeof(uint32_t), s);
             if (!ce) {
-                k_bond_ext<<<(N + 127) / 128, 128, 0, s>>>(d.posd[0], dIL, dT, dIL_f, dL0, dStr, N, K, dbs, nspec);
+                k_rows_list<<<(N + 15) / 16, 128, 0, s>>>(dR, d, c, dCIs, dpnC, P.a_farcut, pair_cut ? x->list_gap : -1.0, dw);
+                k_rows_bonds<0><<<(N + 31) / 32, 128, 0, s>>>(dR, d, c, aa_create, aa_far, dbs, nspec, dw + 1);
                 ce = cudaGetLastError();
             }
+            if (!ce) ce = cudaMemcpyAsync(w, dw, sizeof(w), cudaMemcpyDeviceToHost, s);
             if (!ce) ce = cudaStreamSynchronize(s);
-            cudaFree(dbs);
-            if (ce) st2 = cuda_status(ce, "k_bond_ext");
+            if (ce) st2 = cuda_status(ce, "engine lists");
+            else if (w[0] && !init_dev) init_dev = (rf_status)w[0];
+            qb = w[1];
         }
-        // (with a list gap every listed pair is within its cutoff: nothing to delete)
-        if (!st2 && !pair_cut && !rows)
-            st2 = md_DeleteFarLinks(dR, N, dIL, dT, dIL_f, Rij, Oijt, Fijn, Fijt, Mijn, Mijt, Mijadd, K,
-                                    (float)P.aa_farcut, s);
         if (!st2) {
             // bond records: as many per particle as its row holds bonds (bonds are never created later)
-            uint32_t qb = 0;
-            ce = cudaMemsetAsync(e->maxq_dev, 0, sizeof(uint32_t), s);
-            if (!ce) { k_count_records<<<148 * 4, 256, 0, s>>>(dIL, dT, Rij, N, K, e->maxq_dev); ce = cudaGetLastError(); }
-            if (!ce) ce = cudaMemcpyAsync(&qb, e->maxq_dev, sizeof(qb), cudaMemcpyDeviceToHost, s);
-            if (!ce) ce = cudaStreamSynchronize(s);
-            if (ce) st2 = cuda_status(ce, "engine bond count");
-            if (qb == 0) qb = 1;
-            d.QB = qb;
-            const size_t QN = (size_t)qb * N;
-            if (!st2 && ((st2 = dalloc(e, &d.bjk, QN)) || (st2 = dalloc(e, &d.rec, QN)))) {}
+            d.QB = qb ? qb : 1u;
+            Arrays B;
+            B.add(&d.bjk, (size_t)d.QB * N); B.add(&d.rec, (size_t)d.QB * N);
+            st2 = dalloc(e, B);
         }
         if (!st2) {
-            if (!ext) k_planar_to_f4<<<(N + 255) / 256, 256, 0, s>>>(dR, N, d.pos[0], 1u);
-            k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dIL_f, Rij, Oijt, Mijn, Mijt, dL0, dStr, d, c);
+            if (rows)
+                k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dIL_f, dS, dS + NK, dS + 2 * NK, dS + 3 * NK, d, c);
+            else
+                k_rows_bonds<1><<<(N + 31) / 32, 128, 0, s>>>(dR, d, c, aa_create, aa_far, dbs, nspec, nullptr);
             ce = cudaGetLastError();
-            if (ce) st2 = cuda_status(ce, "engine import");
+            if (!ce) ce = cudaStreamSynchronize(s);
+            if (ce) st2 = cuda_status(ce, "engine init");
         }
-        if (!st2) { ce = cudaStreamSynchronize(s); if (ce) st2 = cuda_status(ce, "engine init"); }
-        cudaFree(dR); cudaFree(dV); cudaFree(dCI); cudaFree(dCIs); cudaFree(dpnC); cudaFree(dIL); cudaFree(dT);
-        cudaFree(dIL_f); cudaFree(dS); cudaFree(scratch); cudaFree(dRd); cudaFree(dRad); cudaFree(dL0); cudaFree(dStr);
+        cudaFree(tmp);
         if (st2) return fail(st2);
         st = init_dev;
     }
@@ -3459,12 +3535,13 @@ rf_status fire_setup(rf_engine* e) {
     const uint32_t N = e->c.N;
     const size_t groups = (size_t)d.nspec + e->ncta / FIRE_GROUP + 1;
     rf_status st;
-    if ((st = dalloc(e, &d.frc, N)) || (st = dalloc(e, &d.mom, N)) ||
-        (st = dalloc(e, &d.fpart, (size_t)e->ncta * FIRE_SUMS)) || (st = dalloc(e, &d.rot, N)) ||
-        (d.nspec > 1 && (st = dalloc(e, &d.fpart2, (size_t)e->ncta * FIRE_SUMS))) ||
-        (st = dalloc(e, &d.fgrp, groups * FIRE_SUMS)) || (st = dalloc(e, &d.fgrp_n, groups)) ||
-        (st = dalloc(e, &d.x0, N)) || (st = dalloc(e, &d.xax, N)) || (st = dalloc(e, &d.rec0, (size_t)d.QB * N)))
-        return st;
+    Arrays A;
+    A.add(&d.frc, N); A.add(&d.mom, N); A.add(&d.rot, N); A.add(&d.x0, N); A.add(&d.xax, N);
+    A.add(&d.fpart, (size_t)e->ncta * FIRE_SUMS);
+    if (d.nspec > 1) A.add(&d.fpart2, (size_t)e->ncta * FIRE_SUMS);
+    A.add(&d.fgrp, groups * FIRE_SUMS); A.add(&d.fgrp_n, groups);
+    A.add(&d.rec0, (size_t)d.QB * N);
+    if ((st = dalloc(e, A))) return st;
     RF_CUDA(cudaMemsetAsync(d.fgrp_n, 0, groups * sizeof(uint32_t), e->stream));
     e->cf = e->c;
     if (!getenv("RF_ENGINE_NO_GRAPH")) {
@@ -3888,8 +3965,7 @@ rf_status rf_engine_import(rf_engine* e, const float* R, const float* V, const f
         return RF_ERR_CAPACITY;
     }
     if (!ce) {
-        k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dL, dS, dS + NK, dS + 2 * NK, dS + 3 * NK, nullptr,
-                                                      nullptr, e->d, e->c);
+        k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dL, dS, dS + NK, dS + 2 * NK, dS + 3 * NK, e->d, e->c);
         ce = cudaGetLastError();
     }
     if (!ce) {

@@ -183,11 +183,6 @@ __global__ void k_cell_last_run(size_t N, uint64_t CN, mid_t* __restrict__ CIs, 
 constexpr int LIST_GROUP = 8;            // lanes a particle
 constexpr int LIST_PARTICLES = 16;       // particles a 128-thread CTA
 
-// Cell of lane `sub` of a particle's group, in the reference's visiting order (own, +x, +y,
-// +z, +xy, +xz, +yz, +xyz).
-__device__ __forceinline__ int64_t octant_cell(const Octant& o, int sub) {
-    return o.b + ((0xB2 >> sub) & 1 ? o.ox : 0) + ((0xD4 >> sub) & 1 ? o.oy : 0) + ((0xE8 >> sub) & 1 ? o.oz : 0);
-}
 // First occupant and count of a cell's run; out-of-grid cells are empty and reported.
 __device__ __forceinline__ void cell_run(const mid_t* pnC, uint64_t CN, int64_t cell, uint64_t& s, uint64_t& n,
                                          uint32_t* err) {
@@ -374,11 +369,6 @@ __global__ void __launch_bounds__(128) k_delete_far_links(const float* __restric
             st3(Mijn, k, z); st3(Mijt, k, z); st3(Mijadd, k, z);
         }
     }
-}
-
-// rm2 with the contraction nvcc gives r.x*r.x + r.y*r.y + r.z*r.z in the reference build.
-__device__ __forceinline__ float rm2_bond(float x, float y, float z) {
-    return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
 }
 
 __global__ void __launch_bounds__(128) k_construct_bonds(const float* __restrict__ R, size_t N, const mid_t* __restrict__ IL,

@@ -203,6 +203,11 @@ __device__ __forceinline__ float dist2_rn(const f3 a, const f3 b) {
 __device__ __forceinline__ bool above_1em10(float rr) { return rr >= 1e-10f; }
 __device__ __forceinline__ bool below_1em10(float rr) { return rr < 1e-10f; }
 
+// rm2 with the contraction nvcc gives r.x*r.x + r.y*r.y + r.z*r.z in the reference build.
+__device__ __forceinline__ float rm2_bond(float x, float y, float z) {
+    return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y)));
+}
+
 // Cell grid of the reference (cell_data): cell edge a, 1/a, Nr.
 struct RefGrid {
     float a, inv_a;
@@ -221,23 +226,8 @@ __device__ __forceinline__ uint32_t ref_cell(const f3 x, const RefGrid& g, uint3
     return ix + iy * g.nx + iz * g.ny * g.nx;
 }
 
-// The 8 octant cells in the reference's visiting order
-// (md_interaction_list_reconstructbpm.cu:91-118): own cell, +x, +y, +z, +xy, +xz, +yz, +xyz,
-// each step towards the half of the cell the particle sits in.
-__device__ __forceinline__ void octant_cells(const f3 x, const RefGrid& g, int64_t cells[8]) {
-    uint32_t ix, iy, iz;
-    const uint32_t c = ref_cell(x, g, &ix, &iy, &iz);
-    const float hx = __fadd_rn((float)ix, 0.5f), hy = __fadd_rn((float)iy, 0.5f), hz = __fadd_rn((float)iz, 0.5f);
-    const int sx = signbit(x.x - __fmul_rn(hx, g.a)) ? -1 : 1;
-    const int sy = signbit(x.y - __fmul_rn(hy, g.a)) ? -1 : 1;
-    const int sz = signbit(x.z - __fmul_rn(hz, g.a)) ? -1 : 1;
-    const int64_t ox = sx, oy = (int64_t)sy * g.nx, oz = (int64_t)sz * g.ny * g.nx;
-    const int64_t b = (int64_t)c;
-    cells[0] = b;           cells[1] = b + ox;           cells[2] = b + oy;      cells[3] = b + oz;
-    cells[4] = b + ox + oy; cells[5] = b + ox + oz;      cells[6] = b + oy + oz; cells[7] = b + ox + oy + oz;
-}
-
-// The same 8 cells as base + offsets (compact form for register-tight kernels).
+// The 8 octant cells (md_interaction_list_reconstructbpm.cu:91-118), own cell and its neighbours
+// towards the half of the cell the particle sits in per axis, as base + offsets.
 struct Octant {
     int64_t b, ox, oy, oz;
 };
@@ -266,15 +256,11 @@ __device__ __forceinline__ int octant_rank(const Octant& o, uint32_t cj) {
     return -1;
 }
 
-// Rank (0..7) of cell cj among the octant cells of a particle at x, or -1.
-__device__ __forceinline__ int octant_rank(const int64_t cells[8], uint32_t cj) {
-    const int64_t c = (int64_t)cj;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-        if (cells[r] == c) return r;
-    return -1;
+// Cell of lane `sub` of a particle's group, in the reference's visiting order (own, +x, +y,
+// +z, +xy, +xz, +yz, +xyz).
+__device__ __forceinline__ int64_t octant_cell(const Octant& o, int sub) {
+    return o.b + ((0xB2 >> sub) & 1 ? o.ox : 0) + ((0xD4 >> sub) & 1 ? o.oy : 0) + ((0xE8 >> sub) & 1 ? o.oz : 0);
 }
-
 // d_braziltest_simple2 per particle (md_braziltest_simple2.cu:28-92); returns contributions.
 __device__ __forceinline__ void brazil_particle(float& Rx, float& Ry, float& Rz, float& Vx, float& Vy, float& Vz,
                                                 float& Fx, float& Fy, float& Fz, const rf_float3 c, float RR, float Yt,
