@@ -128,15 +128,14 @@ __global__ void k_scan_apply(Dev d, Par c, int self) {
     } else {
         carry = d.bsum[blockIdx.x];
     }
-    for (uint32_t off = 0; off < SCAN_CHUNK; off += blockDim.x) {
-        const size_t q = base + off + threadIdx.x;
-        const uint32_t v = q < c.cells ? d.count[q] : 0;
-        const uint32_t ex = block_excl_scan(v, wsum, &total);
-        if (q < c.cells) d.start[q] = carry + ex;
-        carry += total;
-        __syncthreads();
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) d.start[c.cells] = carry;
+    const size_t q = base + 4 * threadIdx.x;             // (SCAN_CHUNK: four cells a thread)
+    uint32_t v[4], sum = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { v[u] = q + u < c.cells ? d.count[q + u] : 0u; sum += v[u]; }
+    uint32_t run = carry + block_excl_scan(sum, wsum, &total);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { if (q + u < c.cells) d.start[q + u] = run; run += v[u]; }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) d.start[c.cells] = carry + total;
 }
 // The counts run back to zero as the cells fill: the update counts the next grid into them.
 __global__ void k_scatter(Dev d, Par c) {
@@ -146,20 +145,20 @@ __global__ void k_scatter(Dev d, Par c) {
     }
 }
 
-// Occupants of each cell in id order (the scatter's atomics leave them in arrival
-// order), so the force sums below, and with them the whole packing, are deterministic; and
-// their positions in that order, so that the forces read the cells' runs straight through.
+// The positions in cell order, a cell's occupants in id order (the scatter's atomics leave them in
+// arrival order), so the force sums below, and with them the whole packing, are deterministic,
+// and the forces read the cells' runs straight through. A thread a particle finds its place among
+// its cell's occupants (a thread a cell sorted them one load after another: 11 us a launch at 20k
+// particles, cold, against 4.4).
 __global__ void k_cellsort(Dev d, Par c) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < c.cells; q += gridDim.x * blockDim.x) {
-        const uint32_t s0 = d.start[q], n = d.start[q + 1] - s0;
-        uint32_t* a = d.sorted + s0;
-        for (uint32_t u = 1; u < n; ++u) {
-            const uint32_t v = a[u];
-            uint32_t w = u;
-            while (w > 0 && a[w - 1] > v) { a[w] = a[w - 1]; --w; }
-            a[w] = v;
-        }
-        for (uint32_t u = 0; u < n; ++u) d.xs[s0 + u] = d.x[a[u]];
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < c.N; q += gridDim.x * blockDim.x) {
+        const uint32_t i = d.sorted[q], k = d.key[i];
+        const double4 x = d.x[i];
+        const uint32_t s0 = d.start[k], s1 = d.start[k + 1];
+        uint32_t at = s0;
+#pragma unroll 4
+        for (uint32_t u = s0; u < s1; ++u) at += d.sorted[u] < i ? 1u : 0u;
+        d.xs[at] = x;
     }
 }
 
@@ -167,36 +166,128 @@ __global__ void k_cellsort(Dev d, Par c) {
 // f = 4/3 sqrt(R*) delta^1.5 (unit modulus, unit masses). Partials of F.v, |F|^2,
 // |v|^2 and the largest overlap (relative to the smaller radius); the last block to finish
 // makes the FIRE decision.
+// The candidates of a particle are the occupants of nine runs of cells (three x-neighbouring cells
+// are one run of the cell order). Eight lanes a particle test them and list the overlapping ones in
+// run order; the warp's listed pairs are then evaluated a lane a pair (about one tested pair in six
+// overlaps, and one evaluation is some 300 instructions of FP64 roots and quotients), and the
+// particle's first lane adds its pairs' forces in list order, the order of a plain loop. A thread
+// a particle ran a chain of some 40 candidates, on 79 CTAs for 20k particles: 43 us a launch
+// (cold), 25 us so; the packing of 3k particles 185 -> 80 ms, of 20k 178 -> 105 ms. Two and four
+// lanes were slower at every size (20k: 125 ms); one lane was 7 % faster at 1M only.
+#define PACK_LANES 8
+#define PACK_HITS 32                         // listed pairs of a particle before they are evaluated
 __device__ __forceinline__ void fire_decide(Dev d, Par c, int nblocks);
 __global__ void __launch_bounds__(256) k_force(Dev d, Par c) {
+    constexpr uint32_t LANES = PACK_LANES, G = 32 / LANES, CAP = PACK_HITS;     // G: particles of a warp
+    __shared__ uint32_t s_hit[8][G][CAP], s_run[8][G][9], s_off[8][G][9];
+    __shared__ uint16_t s_pair[8][G * CAP];
+    __shared__ double s_res[8][3][32];
+    const uint32_t FULL = 0xffffffffu;
+    const uint32_t wp = threadIdx.x >> 5, lane = threadIdx.x & 31u, sub = lane % LANES, grp = lane / LANES;
+    const uint32_t lower = (1u << sub) - 1u;
     const double g = d.s->scale;
     double fv = 0, ff = 0, vv = 0, mo = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.N; i += gridDim.x * blockDim.x) {
-        const double4 xi = d.x[i];
-        const double ri = g * xi.w;
+    for (uint32_t i0 = (blockIdx.x * 8u + wp) * G; i0 < c.N; i0 += gridDim.x * 8u * G) {
+        const uint32_t i = i0 + grp;
+        const bool in = i < c.N;
+        double4 xi = make_double4(0, 0, 0, 0);
         double fx = 0, fy = 0, fz = 0;
-        const uint32_t key = d.key[i];
+        if (in) xi = d.x[i];
+        const double ri = g * xi.w;
+        const uint32_t key = in ? d.key[i] : 0u;
         const int ix = key % c.nx, iy = (key / c.nx) % c.ny, iz = key / (c.nx * c.ny);
-        // (three x-neighbouring cells are one run of the cell order)
         const uint32_t xa = ix > 0 ? ix - 1 : 0, xb = ix + 1 < (int)c.nx ? ix + 1 : ix;
-        for (int z = max(iz - 1, 0); z <= min(iz + 1, (int)c.nz - 1); ++z) {
-            for (int y = max(iy - 1, 0); y <= min(iy + 1, (int)c.ny - 1); ++y) {
-                const uint32_t line = c.nx * (y + c.ny * z);
-                const uint32_t e0 = d.start[line + xb + 1];
-                for (uint32_t q = d.start[line + xa]; q < e0; ++q) {
-                    const double4 xj = d.xs[q];
-                    const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
-                    const double rj = g * xj.w;
-                    const double r2 = rx * rx + ry * ry + rz * rz, sr = ri + rj;
-                    if (r2 >= sr * sr || r2 <= 0) continue;        // (the particle itself: r2 = 0)
-                    const double r = sqrt(r2), dl = sr - r;
-                    const double Rs = ri * rj / sr;
-                    const double fn = (4.0 / 3.0) * sqrt(Rs) * dl * sqrt(dl);
-                    fx -= fn * rx / r; fy -= fn * ry / r; fz -= fn * rz / r;
-                    mo = fmax(mo, dl / fmin(ri, rj));
-                }
+        auto run_of = [&](int r, uint32_t& s0) -> uint32_t {         // occupants of run r
+            const int z = iz + r / 3 - 1, y = iy + r % 3 - 1;
+            s0 = 0;
+            if (!in || z < 0 || z >= (int)c.nz || y < 0 || y >= (int)c.ny) return 0u;
+            const uint32_t line = c.nx * (y + c.ny * z);
+            s0 = d.start[line + xa];
+            return d.start[line + xb + 1] - s0;
+        };
+        auto pair = [&](double rx, double ry, double rz, double ra, double rb) -> double3 {
+            const double r2 = rx * rx + ry * ry + rz * rz, sr = ra + rb;
+            const double r = sqrt(r2), dl = sr - r;
+            const double Rs = ra * rb / sr;
+            const double fn = (4.0 / 3.0) * sqrt(Rs) * dl * sqrt(dl);
+            mo = fmax(mo, dl / fmin(ra, rb));
+            return make_double3(fn * rx / r, fn * ry / r, fn * rz / r);
+        };
+        uint32_t cnt = 0;                                // the particle's listed pairs
+        // evaluates the warp's listed pairs and adds them up
+        auto flush = [&]() {
+            uint32_t all = sub == 0 ? cnt : 0u;
+#pragma unroll
+            for (uint32_t o = LANES; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, all, o);
+                if (lane >= o) all += y;
             }
+            const uint32_t first = __shfl_sync(FULL, all, grp * LANES) - cnt;
+            all = __shfl_sync(FULL, all, 32 - LANES);
+            for (uint32_t t = sub; t < cnt; t += LANES) s_pair[wp][first + t] = (uint16_t)(grp | (t << 5));
+            __syncwarp();
+            uint32_t added = 0;
+            for (uint32_t b = 0; b < all; b += 32u) {
+                const uint32_t x = b + lane, e = x < all ? s_pair[wp][x] : 0u, u = e & 31u;
+                const double px = __shfl_sync(FULL, xi.x, u * LANES), py = __shfl_sync(FULL, xi.y, u * LANES),
+                             pz = __shfl_sync(FULL, xi.z, u * LANES), pr = __shfl_sync(FULL, ri, u * LANES);
+                if (x < all) {
+                    const double4 xj = d.xs[s_hit[wp][u][e >> 5]];
+                    const double3 t = pair(xj.x - px, xj.y - py, xj.z - pz, pr, g * xj.w);
+                    s_res[wp][0][lane] = t.x; s_res[wp][1][lane] = t.y; s_res[wp][2][lane] = t.z;
+                }
+                __syncwarp();
+                if (sub == 0)
+                    for (; added < cnt && first + added < b + 32u; ++added) {
+                        const uint32_t k = first + added - b;
+                        fx -= s_res[wp][0][k]; fy -= s_res[wp][1][k]; fz -= s_res[wp][2][k];
+                    }
+                __syncwarp();
+            }
+            cnt = 0;
+        };
+        auto overlaps = [&](uint32_t q) -> bool {
+            const double4 xj = d.xs[q];
+            const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
+            const double rj = g * xj.w;
+            const double r2 = rx * rx + ry * ry + rz * rz, sr = ri + rj;
+            return !(r2 >= sr * sr || r2 <= 0);          // (the particle itself: r2 = 0)
+        };
+        uint32_t total = 0;
+#pragma unroll
+        for (uint32_t t = 0; t < (9 + LANES - 1) / LANES; ++t) {      // runs sub, sub + LANES, ...
+            const int r = (int)(sub + LANES * t);
+            uint32_t s0 = 0;
+            const uint32_t n = r < 9 ? run_of(r, s0) : 0u;
+            uint32_t at = n;
+#pragma unroll
+            for (uint32_t o = 1; o < LANES; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, at, o, LANES);
+                if (sub >= o) at += v;
+            }
+            if (r < 9) { s_run[wp][grp][r] = s0; s_off[wp][grp][r] = total + at - n; }   // candidates before run r
+            total += __shfl_sync(FULL, at, LANES - 1, LANES);
         }
+        __syncwarp();
+        const uint32_t most = __reduce_max_sync(FULL, total);
+        for (uint32_t base = 0; base < most; base += LANES) {
+            const uint32_t f = base + sub;
+            bool hit = false;
+            uint32_t q = 0;
+            if (f < total) {
+                uint32_t r = 0;
+#pragma unroll
+                for (uint32_t t = 1; t < 9; ++t) r = f >= s_off[wp][grp][t] ? t : r;
+                q = s_run[wp][grp][r] + (f - s_off[wp][grp][r]);
+                hit = overlaps(q);
+            }
+            const uint32_t bal = (__ballot_sync(FULL, hit) >> (grp * LANES)) & ((1u << LANES) - 1u);
+            if (hit) s_hit[wp][grp][cnt + __popc(bal & lower)] = q;
+            cnt += __popc(bal);
+            if (__any_sync(FULL, cnt > CAP - LANES) || base + LANES >= most) { __syncwarp(); flush(); }
+        }
+        __syncwarp();
+        if (!in || sub != 0) continue;
         // container wall (cylinder side and end caps)
         const double rho = sqrt(xi.x * xi.x + xi.y * xi.y);
         const double dw = rho + ri - c.Rc;
@@ -372,6 +463,7 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
     std::vector<void*> allocs;
     auto al = [&](void** p, size_t bytes) { cudaError_t e = cudaMalloc(p, bytes); if (!e) allocs.push_back(*p); return e; };
     const int nb = (int)((N + 255) / 256) < 148 * 8 ? (int)((N + 255) / 256) : 148 * 8;
+    const int per = 256 / PACK_LANES, nbf = (int)((N + per - 1) / per) < 148 * 8 ? (int)((N + per - 1) / per) : 148 * 8;
     cudaError_t e = cudaSuccess;
     if (!e) e = al((void**)&d.x, N * sizeof(double4));
     if (!e) e = al((void**)&d.v, N * sizeof(double4));
@@ -381,7 +473,7 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
     if (!e) e = al((void**)&d.count, (size_t)c.cells * 4);
     if (!e) e = al((void**)&d.start, ((size_t)c.cells + 1) * 4);
     if (!e) e = al((void**)&d.xs, N * sizeof(double4));
-    if (!e) e = al((void**)&d.part, nb * sizeof(double4));
+    if (!e) e = al((void**)&d.part, nbf * sizeof(double4));
     const uint32_t nchunks = (c.cells + SCAN_CHUNK - 1) / SCAN_CHUNK;
     if (!e) e = al((void**)&d.bsum, (size_t)nchunks * sizeof(uint32_t));
     if (!e) e = al((void**)&d.s, sizeof(Scal));
@@ -410,8 +502,8 @@ extern "C" rf_status rf_pack_cylinder_dist(uint64_t seed, uint64_t N, double r0,
                 k_scan_apply<<<nchunks, 1024, 0, st>>>(d, c, 0);
             }
             k_scatter<<<nb, 256, 0, st>>>(d, c);
-            k_cellsort<<<(c.cells + 255) / 256, 256, 0, st>>>(d, c);
-            k_force<<<nb, 256, 0, st>>>(d, c);
+            k_cellsort<<<(c.N + 127) / 128, 128, 0, st>>>(d, c);
+            k_force<<<nbf, 256, 0, st>>>(d, c);
             k_fire_update<<<nb, 256, 0, st>>>(d, c);
         }
         e = cudaStreamEndCapture(st, &graph);
