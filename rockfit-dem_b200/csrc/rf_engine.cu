@@ -105,6 +105,7 @@ struct Consts {
     unsigned long long curve_cap;
     cudaGraphConditionalHandle h_loop, h_rebuild;
     int use_graph;
+    int fire_skip;             // FIRE loop: the kernels of the body's later iterations leave if a rebuild is due
     // extended model (ext != 0): FP64 positions with radii, per-bond strengths
     int ext;
     ExtParams ep;
@@ -500,12 +501,6 @@ __device__ __forceinline__ uint32_t scan_limit(const Dev& d, const Consts& c, ui
     return n;
 }
 
-// Largest squared displacement (since the last build) of the positions a step writes.
-__device__ __forceinline__ void note_displacement(const Dev& d, float e2) {
-    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(e2));
-    if ((threadIdx.x & 31) == 0 && w) atomicMax(&d.sc->d2max_next, w);
-}
-
 // The delete pass of the last step, applied before the state is read out: the step
 // kernel defers each step's DeleteFarLinks to the start of the next step (same
 // positions), so a snapshot taken between steps applies it first. Idempotent.
@@ -723,6 +718,30 @@ __device__ __forceinline__ void spec_platen_sums(const Dev& d, const SpecGeom& G
     const uint32_t b0 = spec_first_cta(G, n), b1 = spec_last_cta(G, n), w0 = b0 >> 5, w1 = b1 >> 5;
     const bool shared0 = b0 * n < G.p0;              // the first CTA's first specimen is the one before
     pb = 0.0; pt = 0.0;
+    if (w1 - w0 < 8u) {
+        // a small specimen: bits and partials are asked for together, and a partial counts if its
+        // bit is set (the bits first, then the partials behind them, were two latencies of the
+        // chain that ends every step)
+        uint32_t m[8];
+        double2 v[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            m[u] = 0u;
+            v[u] = make_double2(0.0, 0.0);
+            if (w0 + u > w1) continue;
+            m[u] = __ldcg(&d.nz[w0 + u]);
+            const uint32_t b = (w0 + u) * 32u + lane;
+            if (b >= b0 && b <= b1) v[u] = __ldcg(&d.partial[b]);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            const uint32_t w = w0 + u;
+            if (w == w0) m[u] &= (0xffffffffu << (b0 & 31u)) & (shared0 ? ~(1u << (b0 & 31u)) : 0xffffffffu);
+            if (w == w1) m[u] &= 0xffffffffu >> (31u - (b1 & 31u));
+            if (m[u] && lane == 0) atomicAnd(&d.nz[w], ~m[u]);
+            if ((m[u] >> lane) & 1u) { pb += v[u].x; pt += v[u].y; }
+        }
+    } else
     for (uint32_t wb = w0; wb <= w1; wb += 256u) {
         uint32_t m[8];
 #pragma unroll
@@ -766,41 +785,71 @@ __device__ __forceinline__ void spec_platen_sums(const Dev& d, const SpecGeom& G
     }
 }
 
+// What a specimen's scalar step reads, taken while its platen sums are on the way.
+struct SpecIn {
+    double VLoad, Top, FractureStress, MinStress, ZeroStress, MaxStrain, Size0, size_d, size_z, center_d, sz0, keep_frac;
+    float Area;
+    int32_t Loading, Fracture;
+    unsigned long long steps, curve_n;
+};
+template <int KIND>
+__device__ __forceinline__ SpecIn spec_read(const DevScalars* S) {
+    constexpr int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
+    SpecIn q;
+    q.VLoad = S->VLoad; q.Top = S->Top; q.FractureStress = S->FractureStress;
+    q.MinStress = S->MinStress; q.ZeroStress = S->ZeroStress; q.MaxStrain = S->MaxStrain; q.Size0 = S->Size0;
+    q.size_d = S->size_d[ax]; q.size_z = S->size_d[2]; q.center_d = S->center_d[ax]; q.sz0 = S->sz0; q.keep_frac = S->keep_frac;
+    q.Area = S->_1d_Area; q.Loading = S->Loading; q.Fracture = S->Fracture;
+    q.steps = S->steps; q.curve_n = S->curve_n;
+    return q;
+}
+
 // A specimen's scalar step (one thread): SumForcesULoading (md_results.cu:34-74), the
 // fracture test and CompressB/U (md_data_types.h:223-293) from its platen sums; true while
-// the specimen runs on.
+// the specimen runs on. (Every field is read before the first is written: a load behind a store
+// that may be to the same place waits for it, one memory latency after another.)
 template <int KIND>
-__device__ __forceinline__ bool spec_scalars(const Dev& d, const Consts& c, DevScalars* S, uint32_t s, double sfb_all,
-                                             double sft_all) {
-    const double a1 = (double)S->_1d_Area;
-    if (S->curve_n < c.curve_cap) {
-        double* rec = d.curve + 3 * ((size_t)s * c.curve_cap + S->curve_n);
-        rec[0] = (S->size_d[2] - S->sz0) / S->sz0;
+__device__ __forceinline__ bool spec_scalars(const Dev& d, const Consts& c, DevScalars* S, uint32_t s, const SpecIn& in,
+                                             double sfb_all, double sft_all) {
+    constexpr int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
+    const double a1 = (double)in.Area;
+    const double strain = (in.size_z - in.sz0) / in.sz0;
+    const double stress = 0.5 * (fabs(sfb_all) + fabs(sft_all)) * a1;
+    const bool loading = in.Loading || stress > in.MinStress;
+    const bool peak = in.FractureStress < stress;
+    const double fstress = peak ? stress : in.FractureStress;
+    const bool fracture = in.Fracture || (loading && stress < in.ZeroStress) ||
+                          (loading && stress < in.keep_frac * fstress);
+    const double V = (stress < 1e-9) ? 10.0 * in.VLoad : in.VLoad;
+    const double size = in.size_d + V * c.dt_d, top = in.Top + V * c.dt_d, center = in.center_d + V * c.dt_d;
+    const float half = (float)(0.5 * size);
+    const double total = (size - in.Size0) / in.Size0;
+    const bool running = (total < in.MaxStrain) && !fracture;
+    if (in.curve_n < c.curve_cap) {
+        double* rec = d.curve + 3 * ((size_t)s * c.curve_cap + in.curve_n);
+        rec[0] = strain;
         rec[1] = sfb_all * a1;
         rec[2] = sft_all * a1;
     }
-    S->curve_n += 1;
-    S->Stress = 0.5 * (fabs(sfb_all) + fabs(sft_all)) * a1;
-    if (!S->Loading && S->Stress > S->MinStress) S->Loading = 1;
-    if (S->FractureStress < S->Stress) {
-        S->FractureStress = S->Stress;
-        S->FractureStrain = (S->sz0 - S->size_d[2]) / S->sz0;
+    S->curve_n = in.curve_n + 1;
+    S->Stress = stress;
+    if (loading && !in.Loading) S->Loading = 1;
+    if (peak) {
+        S->FractureStress = stress;
+        S->FractureStrain = (in.sz0 - in.size_z) / in.sz0;
     }
-    if (S->Loading && S->Stress < S->ZeroStress) S->Fracture = 1;
-    if (S->Loading && S->Stress < S->keep_frac * S->FractureStress) S->Fracture = 1;
-    const int ax = (KIND == RF_TEST_BRAZIL) ? 1 : 2;
-    S->V = (S->Stress < 1e-9) ? 10.0 * S->VLoad : S->VLoad;
-    S->size_d[ax] += S->V * c.dt_d;
-    S->Top += S->V * c.dt_d;
-    S->TopR = S->Top - 2.0 * c.p_r_d;
-    S->size[ax] = (float)S->size_d[ax];
-    S->sized2[ax] = (float)(0.5 * S->size_d[ax]);
-    S->center_d[ax] += S->V * c.dt_d;
-    S->center[ax] = (float)S->center_d[ax];
-    S->Hd2 = S->sized2[ax];
-    S->Strain = (S->size_d[ax] - S->Size0) / S->Size0;
-    S->steps += 1;                                    // the specimen's own step count
-    const bool running = (S->Strain < S->MaxStrain) && !S->Fracture;
+    if (fracture && !in.Fracture) S->Fracture = 1;
+    S->V = V;
+    S->size_d[ax] = size;
+    S->Top = top;
+    S->TopR = top - 2.0 * c.p_r_d;
+    S->size[ax] = (float)size;
+    S->sized2[ax] = half;
+    S->center_d[ax] = center;
+    S->center[ax] = (float)center;
+    S->Hd2 = half;
+    S->Strain = total;
+    S->steps = in.steps + 1;                          // the specimen's own step count
     S->done = running ? 0u : 1u;
     return running;
 }
@@ -808,12 +857,12 @@ __device__ __forceinline__ bool spec_scalars(const Dev& d, const Consts& c, DevS
 // Shared memory of the end of a step: the warps' sums and their arrivals.
 struct FinishSmem {
     double b[2][4], t[2][4];
-    uint32_t nb[4], mv[4];
+    uint32_t nb[4], mv[4], e2[4];
     uint32_t arrived;
 };
 
 template <int KIND, int PW>
-__device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, double sfb, double sft,
+__device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, double sfb, double sft, float e2max,
                                                 uint32_t nbroken, uint32_t moved, uint32_t sA, bool second,
                                                 FinishSmem& sh) {
     DevScalars* sc = d.sc;
@@ -832,10 +881,11 @@ __device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, d
         if (l == 0) { sh.b[q][w] = b; sh.t[q][w] = t; }
     }
     const uint32_t wn = __reduce_add_sync(FULL, nbroken), wm = __reduce_or_sync(FULL, moved);
+    const uint32_t we = __reduce_max_sync(FULL, __float_as_uint(e2max));
     const bool two = __any_sync(FULL, second);
     uint32_t t = 0;
     if (l == 0) {
-        sh.nb[w] = wn; sh.mv[w] = wm | (two ? 0x100u : 0u);
+        sh.nb[w] = wn; sh.mv[w] = wm | (two ? 0x100u : 0u); sh.e2[w] = we;
         __threadfence_block();
         t = atomicAdd(&sh.arrived, 1u);
     }
@@ -856,6 +906,8 @@ __device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, d
         const uint32_t nb = sh.nb[0] + sh.nb[1] + sh.nb[2] + sh.nb[3];
         if (nb) atomicAdd(&sc->broken, (unsigned long long)nb);
         if (mv & 0xFFu) atomicOr(&sc->moved, 1u);
+        const uint32_t e2 = max(max(sh.e2[0], sh.e2[1]), max(sh.e2[2], sh.e2[3]));
+        if (e2) atomicMax(&sc->d2max_next, e2);
         __threadfence();
     }
     __syncwarp();
@@ -868,10 +920,12 @@ __device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, d
         uint32_t d2max = 0, moved_any = 0;
         if (l == 0) { d2max = __ldcg(&sc->d2max_next); moved_any = __ldcg(&sc->moved); }
         bool running = false;
-        if (!S->done) {
+        const uint32_t done = S->done;
+        const SpecIn in = spec_read<KIND>(S);
+        if (!done) {
             double pb, pt;
             spec_platen_sums(d, G, CTA, pb, pt);
-            if (l == 0) running = spec_scalars<KIND>(d, c, S, s, pb, pt);
+            if (l == 0) running = spec_scalars<KIND>(d, c, S, s, in, pb, pt);
         }
         if (l == 0) S->block_counter = 0;
         if (d.nspec > 1) {
@@ -899,7 +953,7 @@ __device__ __forceinline__ void step_finish_ext(const Dev& d, const Consts& c, d
 }
 
 #define FIRE_SUMS 9     // F.v + M.w, |F|^2, |v|^2, |M|^2, |w|^2, sum |f_n|, pair count, platen sums (2)
-#define FIRE_GROUP 64   // CTAs whose partials the last of them adds up before the specimen's last CTA does
+#define FIRE_GROUP 128  // CTAs whose partials the last of them adds up before the specimen's last CTA does
 
 struct FireSmem {
     double a[2][4][FIRE_SUMS];
@@ -941,14 +995,22 @@ template <int KIND, int MODE, int MINB = RF_STEP_MIN_BLOCKS, int PW = 32>
 __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     constexpr int SUB = 32 / PW;                   // lanes a particle has in the scans
     DevScalars* sc = d.sc;
+    // (the loop state, the particles' record masks and the CTA's specimen are asked for side by side)
+    const uint32_t ip = (blockIdx.x * 4u + (threadIdx.x >> 5)) * PW + (threadIdx.x & 31u) % PW;
+    const bool first = SUB == 1 || (threadIdx.x & 31u) < (uint32_t)PW;
+    const uint32_t stopped = MODE == 0 ? sc->done : sc->fstop;
+    const unsigned long long steps = sc->steps, target = sc->target;
+    uint32_t bmask = ip < c.N && first ? d.bmask[ip] : 0u;
+    uint32_t sA = 0u;
+    if (d.blk_spec) sA = (uint32_t)d.blk_spec[(blockIdx.x * 4u * PW) >> 7];
+    if (MODE == 1 && c.fire_skip && sc->rebuild) return;
     if (c.use_graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c.h_loop, 0u);
-    if (MODE == 0 && (sc->done || sc->steps >= sc->target)) return;
-    if (MODE == 1 && sc->fstop) return;
+    if (stopped || (MODE == 0 && steps >= target)) return;
     union Finish { FinishSmem step; FireSmem fire; };
     __shared__ Finish s_fin;
     if (threadIdx.x == 0) { if (MODE == 0) s_fin.step.arrived = 0u; else s_fin.fire.arrived = 0u; }
     __syncthreads();
-    const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
+    const uint32_t cur = (uint32_t)(steps & 1ull), nxt = cur ^ 1u;
     const double4* __restrict__ P = d.posd[cur];
     const F8* __restrict__ VW = d.vw[cur];
     const uint32_t N = c.N;
@@ -958,14 +1020,23 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     const uint32_t i = wbase + pl;
     const bool mine = i < N && (SUB == 1 || sub == 0);         // the lane keeps the particle's state
     // specimen of this particle: the CTA's first one, or the next
-    uint32_t sA = d.blk_spec ? (uint32_t)d.blk_spec[(blockIdx.x * 4u * PW) >> 7] : 0u;
-    if (d.blk_spec && blockIdx.x * 4u * PW >= d.geom[sA].p1) ++sA;
-    const uint32_t sI = (i < N && i >= d.geom[sA].p1) ? sA + 1u : sA;
+    // (a batch; one specimen runs until the loop stops)
+    uint32_t sI = 0u, ended = 0u;
+    if (d.blk_spec) {
+        if (blockIdx.x * 4u * PW >= d.geom[sA].p1) ++sA;
+        const uint32_t p1 = d.geom[sA].p1;
+        ended = MODE == 0 ? d.spec[sA].done : d.spec[sA].fstop;
+        sI = sA;
+        if (i < N && i >= p1) {
+            sI = sA + 1u;
+            ended = MODE == 0 ? d.spec[sI].done : d.spec[sI].fstop;
+        }
+    }
     const SpecGeom& G = d.geom[sI];
     const DevScalars* S = d.spec + sI;
     // a finished specimen of a batch is frozen: its state is carried to the next buffer
     // (explicit steps: it reached its stop rule; FIRE: its relaxation of this increment stopped)
-    const bool frozen = i < N && (MODE == 0 ? S->done != 0 : S->fstop != 0);
+    const bool frozen = i < N && ended != 0u;
     const bool active = i < N && !frozen;                      // (on every lane of the particle)
     const bool valid = mine && !frozen;
     const uint32_t FULL = 0xffffffffu;
@@ -992,7 +1063,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     }
     float fnabs = 0.f, kt = 0.f, kr = 0.f;
     uint32_t npair = 0;
-    uint32_t bmask = valid ? d.bmask[i] : 0u;
+    if (!valid) bmask = 0u;
     bool dirty = false;          // live, bond, bmask or member changed
     // bond slots whose pair overlaps: their contact (in parallel with the bond) was taken
     // in the bond pass, with its tangential overlap kept in the slot's contact state
@@ -1456,8 +1527,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         }
     }
     if (MODE == 0) {
-        note_displacement(d, e2max);
-        step_finish_ext<KIND, PW>(d, c, sfb, sft, nbroken, moved, sA, sI != sA, s_fin.step);
+        step_finish_ext<KIND, PW>(d, c, sfb, sft, e2max, nbroken, moved, sA, sI != sA, s_fin.step);
     } else {
         const uint32_t nb = __reduce_add_sync(FULL, nbroken);
         if (lane == 0 && nb) atomicAdd(&sc->broken, (unsigned long long)nb);
@@ -1476,12 +1546,24 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     // Loop safety: clear the WHILE condition first. Only the last block's finalize,
     // which runs after every block has passed this point and advances the step
     // counter towards the target, sets it again, so the device loop always ends.
+    // (the loop state and the particles' are asked for side by side, see k_step_ext)
+    const uint32_t ip = (blockIdx.x * 4u + (threadIdx.x >> 5)) * PW + (threadIdx.x & 31u) % PW;
+    const bool first = SUB == 1 || (threadIdx.x & 31u) < (uint32_t)PW;
+    const uint32_t stopped = sc->done;
+    const unsigned long long steps = sc->steps, target = sc->target;
+    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, bmask = 0, ncand = 0;
+    unsigned long long mem = 0ull;
+    if (ip < c.N && first) {
+        live = d.live[ip]; bond = d.bond[ip]; cm = d.cmask[ip];
+        mem = d.member[ip]; ncand = d.cand_n[ip];
+        nbq = d.nbq[ip]; bmask = d.bmask[ip];
+    }
     if (c.use_graph && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(c.h_loop, 0u);
-    if (sc->done || sc->steps >= sc->target) return;
+    if (stopped || steps >= target) return;
     __shared__ FinishSmem s_fin;
     if (threadIdx.x == 0) s_fin.arrived = 0u;
     __syncthreads();
-    const uint32_t cur = (uint32_t)(sc->steps & 1ull), nxt = cur ^ 1u;
+    const uint32_t cur = (uint32_t)(steps & 1ull), nxt = cur ^ 1u;
     const float4* __restrict__ P = d.pos[cur];
     const F8* __restrict__ VW = d.vw[cur];
     const uint32_t N = c.N;
@@ -1494,13 +1576,6 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     const uint32_t FULL = 0xffffffffu;
     const uint32_t lt = (1u << lane) - 1u;
 
-    uint32_t live = 0, bond = 0, cm = 0, nbq = 0, bmask = 0, ncand = 0;
-    unsigned long long mem = 0ull;
-    if (valid) {
-        live = d.live[i]; bond = d.bond[i]; cm = d.cmask[i];
-        mem = d.member[i]; ncand = d.cand_n[i];
-        nbq = d.nbq[i]; bmask = d.bmask[i];
-    }
     const uint32_t cm0 = cm;
     bool dirty = false;
     uint32_t nbroken = 0;
@@ -1814,8 +1889,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
         if (e2 > c.hard2 && !hidden) raise_status(&d.sc->err, RF_ERR_CAPACITY);
         if (!hidden) e2max = e2;
     }
-    note_displacement(d, e2max);
-    step_finish_ext<KIND, PW>(d, c, sfb, sft, nbroken, moved, 0u, false, s_fin);
+    step_finish_ext<KIND, PW>(d, c, sfb, sft, e2max, nbroken, moved, 0u, false, s_fin);
 }
 
 // The FIRE decision of one specimen from its sums tot (FP64; n its particle count), by
@@ -1824,21 +1898,29 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
 //   P = F.v + M.w > 0: mixing v <- (1-a) v + a (|v|/|F|) F (same for w with M), and after
 //   n_delay such steps dt <- min(dt f_inc, dt_max), a <- a f_alpha;
 //   P <= 0: dt <- max(dt f_dec, dt_min), a <- a0, v = w = 0.
+// (The quotients and roots are formed side by side and every field is read before the first
+// is written, as in spec_scalars.)
 __device__ __forceinline__ void fire_decide(DevScalars* S, const Consts& c, const double* tot, uint32_t n) {
     const double P = tot[0], FF = tot[1], VV = tot[2], MM = tot[3], WW = tot[4], FN = tot[5], NP = tot[6];
+    const double ftol = S->ftol, a = S->falpha, fdt = S->fdt, finc = S->finc, fdtmax = S->fdtmax, fshrink = S->fshrink,
+                 fdec = S->fdec, fdtmin = S->fdtmin, falpha0 = S->falpha0;
+    const unsigned long long iter = S->fiter + 1, max_iter = S->fmax_iter, total = S->fiter_total, npos = S->fnpos;
+    const uint32_t ndelay = S->fndelay, warm = S->fwarm;
+    const double a1 = (double)S->_1d_Area;
     const double mean = NP > 0.0 ? FN / NP : 0.0;
     const double rms = sqrt(FF / (double)n);
+    const double vf = sqrt(VV / FF), wm = sqrt(WW / MM);
+    const double residual = mean > 0.0 ? rms / mean : (FF > 0.0 ? 1e300 : 0.0);
     S->fmean = mean;
-    S->fresidual = mean > 0.0 ? rms / mean : (FF > 0.0 ? 1e300 : 0.0);
+    S->fresidual = residual;
     S->fpower = P;
     // platen stress of this configuration (SumForcesULoading's formula)
-    const double a1 = (double)S->_1d_Area;
     S->Stress = 0.5 * (fabs(tot[7]) + fabs(tot[8])) * a1;
-    S->fiter += 1;
-    S->fiter_total += 1;
-    if (S->fresidual <= S->ftol) { S->fconverged = 1; S->fstop = 1; return; }
-    if (S->fiter >= S->fmax_iter) { S->fstop = 1; return; }
-    if (S->fwarm) {
+    S->fiter = iter;
+    S->fiter_total = total + 1;
+    if (residual <= ftol) { S->fconverged = 1; S->fstop = 1; return; }
+    if (iter >= max_iter) { S->fstop = 1; return; }
+    if (warm) {
         // first pass of an increment: the velocities only carried the start motion into
         // the state; the dynamics starts from rest
         S->fwarm = 0;
@@ -1846,20 +1928,19 @@ __device__ __forceinline__ void fire_decide(DevScalars* S, const Consts& c, cons
         S->fnpos = 0;
         S->fcv = 0.0; S->fcf = 0.0; S->fcm = 0.0;
     } else if (P > 0.0) {
-        const double a = S->falpha;
         S->fcv = 1.0 - a;
-        S->fcf = FF > 0.0 ? a * sqrt(VV / FF) : 0.0;
-        S->fcm = MM > 0.0 ? a * sqrt(WW / MM) : 0.0;
+        S->fcf = FF > 0.0 ? a * vf : 0.0;
+        S->fcm = MM > 0.0 ? a * wm : 0.0;
         S->fuphill = 0;
-        S->fnpos += 1;
-        if (S->fnpos > S->fndelay) {
-            S->fdt = fmin(S->fdt * S->finc, S->fdtmax);
-            S->falpha = a * S->fshrink;
+        S->fnpos = npos + 1;
+        if (npos + 1 > ndelay) {
+            S->fdt = fmin(fdt * finc, fdtmax);
+            S->falpha = a * fshrink;
         }
     } else {
         S->fnpos = 0;
-        S->fdt = fmax(S->fdt * S->fdec, S->fdtmin);
-        S->falpha = S->falpha0;
+        S->fdt = fmax(fdt * fdec, fdtmin);
+        S->falpha = falpha0;
         S->fuphill = 1;
         S->fcv = 0.0; S->fcf = 0.0; S->fcm = 0.0;
     }
@@ -1932,15 +2013,15 @@ __device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c,
 #pragma unroll
         for (int k = 0; k < FIRE_SUMS; ++k)
             for (int o = 16; o; o >>= 1) v[k] += __shfl_xor_sync(FULL, v[k], o);
-        if (l == 0) {
-            d.fgrp_n[gbase + g] = 0u;
+        if (l == 0) d.fgrp_n[gbase + g] = 0u;
+        if (glast) {                                 // (the sums of a single group are the specimen's)
+            if (l == 0) {
 #pragma unroll
-            for (int k = 0; k < FIRE_SUMS; ++k) d.fgrp[(gbase + g) * FIRE_SUMS + k] = v[k];
-            __threadfence();
-        }
-        __syncwarp();
-        if (!arrive_last(&S->fcounter, glast + 1u)) continue;
-        if (!S->fstop) {
+                for (int k = 0; k < FIRE_SUMS; ++k) d.fgrp[(gbase + g) * FIRE_SUMS + k] = v[k];
+                __threadfence();
+            }
+            __syncwarp();
+            if (!arrive_last(&S->fcounter, glast + 1u)) continue;
 #pragma unroll
             for (int k = 0; k < FIRE_SUMS; ++k) v[k] = 0.0;
             for (uint32_t q = l; q <= glast; q += 32u)
@@ -1949,8 +2030,8 @@ __device__ __forceinline__ void fire_force_finish(const Dev& d, const Consts& c,
 #pragma unroll
             for (int k = 0; k < FIRE_SUMS; ++k)
                 for (int o = 16; o; o >>= 1) v[k] += __shfl_xor_sync(FULL, v[k], o);
-            if (l == 0) fire_decide(S, c, v, G.p1 - G.p0);
         }
+        if (l == 0 && !S->fstop) fire_decide(S, c, v, G.p1 - G.p0);
         bool running = false;
         if (l == 0) { S->fcounter = 0u; __threadfence(); }
         if (d.nspec > 1) {
@@ -2009,30 +2090,38 @@ __global__ void __launch_bounds__(128) k_fire_bond_state(Dev d, Consts c) {
 // FIRE update of one iteration, in place on the buffers the force pass wrote:
 // mixing (or, on uphill power, stop), then semi-implicit Euler in FP64
 // positions; the rotation of the increment is accumulated for the warm-start data.
-__global__ void k_fire_update(Dev d, Consts c) {
+// (What does not depend on the loop state is loaded beside it.)
+__global__ void __launch_bounds__(128) k_fire_update(Dev d, Consts c) {
     DevScalars* sc = d.sc;
-    const uint32_t cur = (uint32_t)(sc->steps & 1ull);
-    const bool stop = sc->fstop != 0;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = i < c.N;
+    const uint32_t stop = sc->fstop, rebuild = sc->rebuild;
+    const uint32_t cur = (uint32_t)(sc->steps & 1ull);
+    float4 F = make_float4(0.f, 0.f, 0.f, 0.f), M = F, pr = F;
+    double4 r = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (in) { F = d.frc[i]; M = d.mom[i]; pr = d.pos_ref[i]; r = d.rot[i]; }
     // the particle's specimen (a batch's specimens relax on their own FIRE scalars; one
     // whose relaxation stopped stays where it is)
-    const uint32_t sA = d.blk_spec ? (uint32_t)d.blk_spec[blockIdx.x] : 0u;
-    const DevScalars* S = d.spec + ((i < c.N && i >= d.geom[sA].p1) ? sA + 1u : sA);
+    const DevScalars* S = d.spec;
+    if (d.blk_spec) {
+        const uint32_t sA = (uint32_t)d.blk_spec[blockIdx.x];
+        S += (in && i >= d.geom[sA].p1) ? sA + 1u : sA;
+    }
+    const uint32_t ended = S->fstop, uphill = S->fuphill;
+    const float dt = (float)S->fdt, cv = (float)S->fcv, cf = (float)S->fcf, cm = (float)S->fcm;
+    if (c.fire_skip && rebuild) return;
     uint32_t moved = 0;
     float e2max = 0.f;
-    if (!stop && i < c.N && !S->fstop) {
+    if (!stop && in && !ended) {
         double4 x = d.posd[cur][i];
         float4 v = d.vw[cur][i].a, w = d.vw[cur][i].b;
-        const float4 F = d.frc[i], M = d.mom[i];
-        const float dt = (float)S->fdt;
         const double dtd = (double)dt;
-        if (S->fuphill) {
+        if (uphill) {
             // stop (no half step back: the bond and contact state integrates v dt, so every
             // position change must be a v dt of the force pass that follows)
             v = make_float4(0.f, 0.f, 0.f, 0.f);
             w = v;
         } else {
-            const float cv = (float)S->fcv, cf = (float)S->fcf, cm = (float)S->fcm;
             v.x = cv * v.x + cf * F.x; v.y = cv * v.y + cf * F.y; v.z = cv * v.z + cf * F.z;
             w.x = cv * w.x + cm * M.x; w.y = cv * w.y + cm * M.y; w.z = cv * w.z + cm * M.z;
         }
@@ -2042,44 +2131,38 @@ __global__ void k_fire_update(Dev d, Consts c) {
         v.x += F.x * dtm; v.y += F.y * dtm; v.z += F.z * dtm;
         w.x += M.x * dtI; w.y += M.y * dtI; w.z += M.z * dtI;
         x.x += (double)v.x * dtd; x.y += (double)v.y * dtd; x.z += (double)v.z * dtd;
-        double4 r = d.rot[i];
         r.x += (double)w.x * dtd; r.y += (double)w.y * dtd; r.z += (double)w.z * dtd;
         d.rot[i] = r;
         d.posd[cur][i] = x;
         st8(&d.vw[cur][i], v, w);
-        const float4 pr = d.pos_ref[i];
         const float ex = (float)x.x - pr.x, ey = (float)x.y - pr.y, ez = (float)x.z - pr.z;
         const float e2 = ex * ex + ey * ey + ez * ez;
         moved = (e2 > c.disp2) ? 1u : 0u;
         if (e2 > c.hard2) raise_status(&d.sc->err, RF_ERR_CAPACITY);   // lists may have missed a neighbour
         e2max = e2;
     }
-    note_displacement(d, e2max);           // every lane of the warp takes part
-    __shared__ bool s_last;
-    __shared__ uint32_t s_m;
-    if (threadIdx.x == 0) s_m = 0;
+    __shared__ uint32_t s_m[4], s_e[4];
+    const uint32_t wm = __reduce_or_sync(0xffffffffu, moved), we = __reduce_max_sync(0xffffffffu, __float_as_uint(e2max));
+    if ((threadIdx.x & 31) == 0) { s_m[threadIdx.x >> 5] = wm; s_e[threadIdx.x >> 5] = we; }
     __syncthreads();
-    if (__reduce_or_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(&s_m, 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (s_m) atomicOr(&sc->moved, 1u);
-        __threadfence();
-        s_last = (atomicAdd(&sc->block_counter, 1u) == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
+    if (threadIdx.x != 0) return;
+    const uint32_t e2 = max(max(s_e[0], s_e[1]), max(s_e[2], s_e[3]));
+    if (s_m[0] | s_m[1] | s_m[2] | s_m[3]) atomicOr(&sc->moved, 1u);
+    if (e2) atomicMax(&sc->d2max_next, e2);
     __threadfence();
+    if (atomicAdd(&sc->block_counter, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const uint32_t mv = __ldcg(&sc->moved), d2max = __ldcg(&sc->d2max_next);
     sc->block_counter = 0;
     // largest displacement since the last candidate build of the positions the next force
     // pass reads (this update wrote them): the force pass's add-pass scan skip uses it
-    sc->dmax = sqrtf(__uint_as_float(sc->d2max_next));
+    sc->dmax = sqrtf(__uint_as_float(d2max));
     sc->d2max_next = 0;
-    const uint32_t mv = sc->moved;
     sc->moved = 0;
     sc->rebuild = mv;
     if (c.use_graph) {
-        cudaGraphSetConditional(c.h_rebuild, (mv && !sc->fstop) ? 1u : 0u);
-        cudaGraphSetConditional(c.h_loop, sc->fstop ? 0u : 1u);
+        cudaGraphSetConditional(c.h_rebuild, (mv && !stop) ? 1u : 0u);
+        cudaGraphSetConditional(c.h_loop, stop ? 0u : 1u);
     }
 }
 
@@ -2918,7 +3001,11 @@ rf_status build_graph(rf_engine* e) {
     return RF_OK;
 }
 
-// FIRE loop graph: prologue -> WHILE(not stopped) { IF(moved) {candidate rebuild}; forces; update }.
+// FIRE loop graph: prologue -> WHILE(not stopped) { IF(moved) {candidate rebuild}; RF_GRAPH_UNROLL
+// times forces, update }. A conditional node costs several microseconds, so the body holds more
+// than one iteration; once an update finds that the candidates have to be rebuilt, the rest of the
+// body leaves at once (fire_skip), and the rebuild precedes the next force pass as if every
+// iteration had its IF. Six specimens of 3000 particles: 34.8 -> 28.8 us an iteration.
 rf_status build_fire_graph(rf_engine* e) {
     cudaGraph_t g;
     RF_CUDA(cudaGraphCreate(&g, 0));
@@ -2970,12 +3057,17 @@ rf_status build_fire_graph(rf_engine* e) {
         RF_CUDA(cudaGraphAddKernelNode(&n, rb, prev ? &prev : nullptr, prev ? 1 : 0, &kp));
         prev = n;
     }
-    cudaGraphNode_t fnode, unode;
-    kp = kparams(fire_force_kernel(e), e->ncta, 128);
-    kp.sharedMemBytes = step_smem(e);
-    RF_CUDA(cudaGraphAddKernelNode(&fnode, body, &inode, 1, &kp));
-    kp = kparams((void*)k_fire_update, e->nblocks, 128);
-    RF_CUDA(cudaGraphAddKernelNode(&unode, body, &fnode, 1, &kp));
+    cudaGraphNode_t last = inode, node;
+    for (int u = 0; u < RF_GRAPH_UNROLL; ++u) {
+        cc.fire_skip = u > 0;                        // (node parameters are copied when the node is added)
+        kp = kparams(fire_force_kernel(e), e->ncta, 128);
+        kp.sharedMemBytes = step_smem(e);
+        RF_CUDA(cudaGraphAddKernelNode(&node, body, &last, 1, &kp));
+        last = node;
+        kp = kparams((void*)k_fire_update, e->nblocks, 128);
+        RF_CUDA(cudaGraphAddKernelNode(&node, body, &last, 1, &kp));
+        last = node;
+    }
     RF_CUDA(cudaGraphInstantiate(&e->fexec, g, 0));
     return RF_OK;
 }
