@@ -1321,13 +1321,24 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 2 * SUB) {      // two candidates in flight
-                uint32_t j[2];
+            // the candidates to test: most are in the row already (or were tried)
+            unsigned long long m = scan && qlim ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
+            if (SUB > 1) {                       // every SUB-th of them
+                unsigned long long all = m;
+                m = 0ull;
+                for (uint32_t r = 0; all; ++r) {
+                    if (r % SUB == sub) m |= all & (0ull - all);
+                    all &= all - 1ull;
+                }
+            }
+            while (m) {                          // two in flight
+                uint32_t j[2], q[2];
                 double4 xj[2];
 #pragma unroll
                 for (uint32_t u = 0; u < 2; ++u) {
-                    const uint32_t q = q0 + u * SUB;
-                    j[u] = q < qlim && !((tried >> q) & 1ull) ? __ldg(&d.cand[(size_t)q * N + i]) : i;
+                    q[u] = (uint32_t)__ffsll((long long)m) - 1u;     // (none left: i itself)
+                    j[u] = m ? __ldg(&d.cand[(size_t)q[u] * N + i]) : i;
+                    m &= m - 1ull;
                 }
 #pragma unroll
                 for (uint32_t u = 0; u < 2; ++u) xj[u] = ldg_d4(&P[j[u]]);
@@ -1339,7 +1350,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                     const int rank = octant_rank(oc, ref_cell(mk3((float)xj[u].x, (float)xj[u].y, (float)xj[u].z), c.g));
                     if (rank < 0) continue;
                     const unsigned long long key = ((unsigned long long)rank << 32) | j[u];
-                    if (key < best) { best = key; best_q = q0 + u * SUB; }
+                    if (key < best) { best = key; best_q = q[u]; }
                 }
             }
 #pragma unroll
@@ -1731,13 +1742,24 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
-            for (uint32_t q0 = sub; scan && q0 < qlim; q0 += 4 * SUB) {      // four candidates in flight
-                uint32_t j[4];
+            // the candidates to test: most are in the row already (or were tried)
+            unsigned long long m = scan && qlim ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
+            if (SUB > 1) {                       // every SUB-th of them
+                unsigned long long all = m;
+                m = 0ull;
+                for (uint32_t r = 0; all; ++r) {
+                    if (r % SUB == sub) m |= all & (0ull - all);
+                    all &= all - 1ull;
+                }
+            }
+            while (m) {                          // four in flight
+                uint32_t j[4], q[4];
                 float4 xj[4];
 #pragma unroll
                 for (uint32_t u = 0; u < 4; ++u) {
-                    const uint32_t q = q0 + u * SUB;
-                    j[u] = q < qlim && !((tried >> q) & 1ull) ? __ldg(&d.cand[(size_t)q * N + i]) : i;
+                    q[u] = (uint32_t)__ffsll((long long)m) - 1u;     // (none left: i itself)
+                    j[u] = m ? __ldg(&d.cand[(size_t)q[u] * N + i]) : i;
+                    m &= m - 1ull;
                 }
 #pragma unroll
                 for (uint32_t u = 0; u < 4; ++u) xj[u] = __ldg(&P[j[u]]);
@@ -1749,7 +1771,7 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
                     const int rank = octant_rank(oc, ref_cell(f4to3(xj[u]), c.g));
                     if (rank < 0) continue;
                     const unsigned long long key = ((unsigned long long)rank << 32) | j[u];
-                    if (key < best) { best = key; best_q = q0 + u * SUB; }
+                    if (key < best) { best = key; best_q = q[u]; }
                 }
             }
 #pragma unroll
