@@ -472,29 +472,23 @@ __device__ __forceinline__ void delete_far(const Dev& d, const Consts& c, const 
     }
 }
 
-// True when the candidate scan of the add pass cannot find anything: every non-member
-// candidate was at least cmargin beyond a_farcut at the last build, and since then this
-// particle moved by |x - x_build| and none by more than dmax (the largest displacement
-// of the positions this step reads). 10 % and 1e-4 a_farcut of slack cover the float
-// rounding of the margins and displacements.
-__device__ __forceinline__ bool scan_not_needed(const Dev& d, const Consts& c, uint32_t i, float x, float y, float z) {
-    const float4 pr = d.pos_ref[i];
-    const float ex = x - pr.x, ey = y - pr.y, ez = z - pr.z;
-    const float di = sqrtf(ex * ex + ey * ey + ez * ez);
-    return di + d.sc->dmax < 0.9f * d.cmargin[i] - 1e-4f * c.acut_f;
-}
-
-// How many of particle i's candidates (in bucket order) a scan must test: the candidates
-// of a bucket whose smallest margin the displacements since the build cannot have closed
-// (the test of scan_not_needed, with the bucket's lower bound for cmargin) can be skipped.
-// After a deletion (cmargin 0) every candidate is tested.
+// How many of particle i's candidates (in bucket order) the add pass must test, of n.
+// None when the scan cannot find anything: every non-member candidate was at least cmargin
+// beyond a_farcut at the last build, and since then this particle moved by |x - x_build| and
+// none by more than dmax (the largest displacement of the positions this step reads). 10 % and
+// 1e-4 a_farcut of slack cover the float rounding of the margins and displacements. Else those
+// of the buckets whose lower bound, by the same test, the displacements can have closed. After
+// a deletion (cmargin 0) every candidate is tested. (All loads side by side.)
 __device__ __forceinline__ uint32_t scan_limit(const Dev& d, const Consts& c, uint32_t i, float x, float y, float z,
                                                uint32_t n) {
-    if (!(d.cmargin[i] > 0.f)) return n;
     const float4 pr = d.pos_ref[i];
-    const float ex = x - pr.x, ey = y - pr.y, ez = z - pr.z;
-    const float reach = sqrtf(ex * ex + ey * ey + ez * ez) + d.sc->dmax + 1e-4f * c.acut_f;
+    const float margin = d.cmargin[i], dmax = d.sc->dmax;
     const uint32_t b = d.cbound[i];
+    const float ex = x - pr.x, ey = y - pr.y, ez = z - pr.z;
+    const float moved = sqrtf(ex * ex + ey * ey + ez * ez) + dmax;
+    if (moved < 0.9f * margin - 1e-4f * c.acut_f) return 0u;
+    if (!(margin > 0.f)) return n;
+    const float reach = moved + 1e-4f * c.acut_f;
     if (reach < 0.9f * RF_CB1 * c.skin_f) return b & 0xFFu;
     if (reach < 0.9f * RF_CB2 * c.skin_f) return (b >> 8) & 0xFFu;
     if (reach < 0.9f * RF_CB3 * c.skin_f) return (b >> 16) & 0xFFu;
@@ -1307,22 +1301,21 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
 
     // ---- new neighbours, in the reference's insertion order
     {
-        bool scan = valid && !scan_not_needed(d, c, i, (float)xi.x, (float)xi.y, (float)xi.z);
         const f3 xif = mk3((float)xi.x, (float)xi.y, (float)xi.z);
-        uint32_t qlim = scan ? scan_limit(d, c, i, xif.x, xif.y, xif.z, ncand) : 0u;
+        uint32_t qlim = valid ? scan_limit(d, c, i, xif.x, xif.y, xif.z, ncand) : 0u;
         unsigned long long tried = mem;
         if (SUB > 1) {                           // the particle's lanes share the candidates
-            scan = __shfl_sync(FULL, (int)scan, pl) != 0;
             qlim = __shfl_sync(FULL, qlim, pl);
             tried = __shfl_sync(FULL, tried, pl);
         }
+        bool scan = qlim != 0u;
         bool have_cells = false;
         Octant oc;
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
             // the candidates to test: most are in the row already (or were tried)
-            unsigned long long m = scan && qlim ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
+            unsigned long long m = scan ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
             if (SUB > 1) {                       // every SUB-th of them
                 unsigned long long all = m;
                 m = 0ull;
@@ -1470,6 +1463,8 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
     for (int q = 0; q < FIRE_SUMS; ++q) acc[q] = 0.0;
     if (valid) {
         const F8 vwi = ldg8(&VW[i]);
+        float4 pr = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (MODE == 0) pr = d.pos_ref[i];
         const f3 vi = f4to3(vwi.a), wi = f4to3(vwi.b);
         const float mi = c.cmass * ri * ri * ri;
         if (dirty) { d.live[i] = live; d.bond[i] = bond; d.member[i] = mem; d.bmask[i] = bmask; }
@@ -1527,7 +1522,6 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
         }
         d.posd[nxt][i] = make_double4(Rx, Ry, Rz, xi.w);
         st8(&d.vw[nxt][i], make_float4(Vx, Vy, Vz, 0.f), make_float4(Wx, Wy, Wz, 0.f));
-        const float4 pr = d.pos_ref[i];
         const float ex = (float)Rx - pr.x, ey = (float)Ry - pr.y, ez = (float)Rz - pr.z;
         const float e2 = ex * ex + ey * ey + ez * ez;
         moved = (e2 > c.disp2) ? 1u : 0u;
@@ -1729,21 +1723,20 @@ __global__ void __launch_bounds__(128, RF_STEP_MIN_BLOCKS) k_step(Dev d, Consts 
     // (skipped when no candidate can have come within a_farcut since the build: the scan
     // would add nothing)
     {
-        bool scan = valid && !scan_not_needed(d, c, i, xi.x, xi.y, xi.z);
-        uint32_t qlim = scan ? scan_limit(d, c, i, xi.x, xi.y, xi.z, ncand) : 0u;
+        uint32_t qlim = valid ? scan_limit(d, c, i, xi.x, xi.y, xi.z, ncand) : 0u;
         unsigned long long tried = mem;
         if (SUB > 1) {                           // the particle's lanes share the candidates
-            scan = __shfl_sync(FULL, (int)scan, pl) != 0;
             qlim = __shfl_sync(FULL, qlim, pl);
             tried = __shfl_sync(FULL, tried, pl);
         }
+        bool scan = qlim != 0u;
         bool have_cells = false;
         Octant oc;
         while (SUB > 1 ? __any_sync(FULL, scan) : (int)scan) {
             unsigned long long best = ~0ull;
             uint32_t best_q = 0;
             // the candidates to test: most are in the row already (or were tried)
-            unsigned long long m = scan && qlim ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
+            unsigned long long m = scan ? ~tried & (~0ull >> (64u - qlim)) : 0ull;
             if (SUB > 1) {                       // every SUB-th of them
                 unsigned long long all = m;
                 m = 0ull;
