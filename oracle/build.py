@@ -78,7 +78,7 @@ def build_oracle(force=False):
 
 def build_ref(ref_dir=None, force=False, gpu=True, cpu=True):
     ref_dir = ref_dir or os.environ.get("RF_REFERENCE_DIR") or REF_BESIDE_REPO
-    if not os.path.isdir(ref_dir):
+    if not os.path.isfile(os.path.join(ref_dir, REF_GPU_SOURCES[0])):      # absent, or an empty directory
         return None
     os.makedirs(REF_OUT, exist_ok=True)
     tmp = os.path.join(REF_OUT, "obj")
