@@ -3,14 +3,14 @@
 // One explicit step of the reference (md_calculationbraziltest.cu:170-190:
 // CellDistribution, InteractionListReConstructBPM, F=M=0, _22, _21, platen,
 // SumForcesULoading, increments, cut, DeleteFarLinks, CompressB/U) is ONE kernel
-// here, one thread per particle:
+// here, a warp taking 32 particles, or fewer where they would not fill the GPU:
 //
 //   delete  -- DeleteFarLinks of the previous step, with this step's positions
 //              (the reference runs it at the end of the previous step on the same
 //              positions, so the result is identical);
 //   add     -- new neighbours inside a_farcut, taken from a Verlet candidate list
 //              (cutoff a_farcut + skin, rebuilt only when some particle has moved
-//              more than 0.45*skin since the last build) instead of re-binning every
+//              more than 0.3*skin since the last build) instead of re-binning every
 //              step. New links are inserted in the order the reference would insert
 //              them: by (octant-cell rank, id), computed from the same float cell
 //              arithmetic, into the first free slot;
@@ -20,11 +20,12 @@
 //   load    -- per-block FP64 partial sums, the last block finishes the scalar
 //              step (SumForcesULoading, CompressB/U, fracture, load curve) on device.
 //
-// Layout in HBM: particle vectors as float4 (x, y, z, 0), double-buffered; rows
-// slot-major (ids[k*N + i]) so a warp reading slot k of 32 particles is one
-// coalesced 128-byte access; per-slot state as 12 float planes (Rij, Oijt, Mijn,
-// Mijt); per-particle 32-bit masks for occupied slots, bond slots and contacts
-// with non-zero tangential overlap (so empty and idle slots cost no state reads).
+// Layout in HBM: positions as float4 (x, y, z, 0) or double4 (x, y, z, radius), velocity and
+// spin together as one 32-byte record, both double-buffered; row ids row-major [N][K]; the
+// bonds' state as 64-byte records, ordinal-major [QB][N], so that lanes taking the q-th bond
+// of consecutive particles read consecutive whole sectors; per-particle 32-bit masks for
+// occupied slots, bond slots and contacts with non-zero tangential overlap (so empty and
+// idle slots cost no state reads).
 //
 // The step loop is a CUDA graph: WHILE(continue) { IF(rebuild) {bin, scan,
 // scatter, candidates}; step }, with both conditions set on device by the step
@@ -144,7 +145,7 @@ struct Dev {
     double4* posd[2];   // extended model: x, y, z (FP64) and radius
     float4* pos[2];
     F8* vw[2];          // [N] velocity and spin of a particle (xyz 0 each): one 32-byte sector, one load
-    // rows: slot-major, K slots per particle
+    // rows: K slots per particle
     uint32_t* ids;      // [N][K] neighbour id of each occupied slot (row-major: a thread walks its own row)
     float* il;          // [K][N] 1/L0 per slot, as the reference layout keeps it (read out only)
     float* cO[2];       // [N][K][3] tangential overlap of type-0 slots, by step parity (read cur, write next)
