@@ -2596,8 +2596,9 @@ __global__ void __launch_bounds__(128) k_rows_list(const float* __restrict__ R, 
             if (at < c.K) row[at] = j;
             ++at; --n;
         }
-    for (uint32_t k = total + sub; k < c.K; k += 8) row[k] = EMPTY32;
-    if (sub == 0) d.live[i] = total >= 32u ? 0xffffffffu : (1u << total) - 1u;
+    const uint32_t held = min(total, c.K);       // (the row is cut at K: the mask has no slot beyond it)
+    for (uint32_t k = held + sub; k < c.K; k += 8) row[k] = EMPTY32;
+    if (sub == 0) d.live[i] = held >= 32u ? 0xffffffffu : (1u << held) - 1u;
 }
 
 // Bonds of the rows, a warp a particle and a lane a slot. Reference model: pairs below the
