@@ -1402,8 +1402,12 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 }
             }
             __syncwarp();
+            const uint32_t e = base + lane < total ? s_ent[wp][lane] : 0u;
+            // (FIRE: the time step of the contact's specimen, not of the lane's: a warp may hold particles of two)
+            ExtParams cp = ep;
+            if (MODE == 1) cp.dt = __shfl_sync(FULL, ep.dt, e & 31u);
             if (base + lane < total) {
-                const uint32_t e = s_ent[wp][lane], io = wbase + (e & 31u), k = (e >> 5) & 31u;
+                const uint32_t io = wbase + (e & 31u), k = (e >> 5) & 31u;
                 const size_t so = (size_t)io * c.K + k;
                 const uint32_t j = d.ids[so];
                 const double4 xo = ldg_d4(&P[io]), xj = ldg_d4(&P[j]);
@@ -1413,7 +1417,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_ext(Dev d, Consts c) {
                 const float ro = (float)xo.w, rj = (float)xj.w;
                 const F8 vwo = ldg8(&VW[io]), vwj = ldg8(&VW[j]);
                 const ContactTerms t =
-                    contact_terms_ext(ep, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), xo.w + xj.w, ro, rj,
+                    contact_terms_ext(cp, mk3((float)rd.x, (float)rd.y, (float)rd.z), dlen2(rd), xo.w + xj.w, ro, rj,
                                       c.cmass * ro * ro * ro, c.cmass * rj * rj * rj, f4to3(vwo.a), f4to3(vwj.a),
                                       f4to3(vwo.b), f4to3(vwj.b), o);
                 float* oo = d.cO[nxt] + 3 * so;
