@@ -2877,8 +2877,8 @@ rf_status dalloc(rf_engine* e, const Arrays& a) {
 
 #define TRY(x) do { rf_status s__ = (x); if (s__ != RF_OK) return s__; } while (0)
 
-// Explicit extended-model step kernels: compiled for 5, 6 or 8 CTAs per SM at 32 particles a
-// warp; with fewer (specimens that do not fill the GPU) the register cap has nothing to give.
+// Explicit extended-model step kernels: compiled for 5, 6 and 8 CTAs per SM at 32 particles a
+// warp, for 6 alone with fewer (there minb has no effect).
 template <int KIND>
 void* ext_step_kind(int pw, int minb) {
     switch (pw) {
@@ -3822,6 +3822,7 @@ rf_status rf_engine_autotune(rf_engine* e, int steps, int* choice, float* ms_out
         return cudaStreamSynchronize(s);
     };
     const int variants[3] = {8, 6, 5};
+    const int first = e->pw == 32 ? 0 : 1, last = e->pw == 32 ? 3 : 2;     // (see ext_step_kind)
     float best = 1e30f;
     int pick = e->step_minb;
     float times[3] = {0, 0, 0};
@@ -3832,7 +3833,7 @@ rf_status rf_engine_autotune(rf_engine* e, int steps, int* choice, float* ms_out
     cudaEvent_t a0, a1;
     cudaEventCreate(&a0); cudaEventCreate(&a1);
     cudaError_t ce = cudaSuccess;
-    for (int v = 0; v < 3 && !ce; ++v) {
+    for (int v = first; v < last && !ce; ++v) {
         void* fn = ext_step_variant(e, variants[v]);
         for (int rep = 0; rep < 2 && !ce; ++rep) {             // first pass warms up
             ce = restore();
@@ -3873,7 +3874,7 @@ rf_status rf_engine_autotune(rf_engine* e, int steps, int* choice, float* ms_out
         }
     }
     if (choice) *choice = pick;
-    if (ms_out) for (int v = 0; v < 3; ++v) ms_out[v] = times[v];
+    if (ms_out) for (int v = 0; v < 3; ++v) ms_out[v] = times[std::min(std::max(v, first), last - 1)];
     return RF_OK;
 }
 

@@ -123,6 +123,16 @@ def test_autotune_leaves_results_unchanged(cuda):
     a.close(); b.close()
 
 
+def test_autotune_of_a_small_engine_times_its_one_variant(cuda):
+    """A specimen that does not fill the GPU has one compiled step kernel: one time, and the
+    pick does not depend on it."""
+    t, R, rad, x = extspec.ext_case(rfdem.RF_TEST_UNIAXIAL, 6.0, 10.0, min_stress=1e3)
+    e = rfdem.Engine(t, R, ext=x, radius=rad)
+    pick, ms = e.autotune(50)
+    e.close()
+    assert pick == 6 and ms[0] > 0 and ms[0] == ms[1] == ms[2]
+
+
 @pytest.mark.parametrize("gap", [0.0, 0.5], ids=["uniform-cutoff", "list-gap"])
 def test_ext_log_uniform_radius_ratio_3_vs_oracle(cuda, gap):
     """Radii log-uniform in [0.5, 1.5] r0 (radius ratio 3): the packer keeps the range and
