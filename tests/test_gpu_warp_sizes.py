@@ -34,8 +34,9 @@ def test_explicit_steps_bitexact(cuda, kind, d, h, tuned):
         e.autotune(20)
     e.step(steps)
     _, res = e.sync()
-    st, R64 = e.export(), e.positions_f64()
+    st, R64, curve = e.export(), e.positions_f64(), e.curve()
     e.close()
+    np.testing.assert_allclose(curve, o["curve"], rtol=1e-9, atol=1e-12)    # (FP64 sums in another order)
     N, K = int(t.N), int(t.K)
     bonds, contacts = extspec.pair_counts(o["R"], N, K, o["IL"], o["ILtype"], rad)
     start = oracle.run_ext(mc.clone(t), x, R, rad, 0)
@@ -107,3 +108,55 @@ def test_batches(cuda, nspec):
             assert abs(res[k][q].stress - ra[k].stress) <= 1e-6 * abs(ra[k].stress)
         assert np.max(np.abs(Re - Ra)) < 1e-7 * ext, (q, np.abs(Re - Ra).max() / ext)
     e.close()
+
+
+def test_two_large_specimens(cuda):
+    """A batch whose specimens' sums take the paths of many CTAs (more than 256 each, in several FIRE
+    groups) and meet in one CTA: explicit steps and load curves against the oracle, then FIRE
+    increments as in an engine of their own."""
+    specs = []
+    for q, (d, h) in enumerate([(34.0, 44.0), (33.0, 45.0)]):
+        R0, rad = extspec.lattice_ext(rfdem.RF_TEST_UNIAXIAL, d, h, seed=0xB2000000 + 300 + q)
+        t, R = rfdem.make_test_ext(rfdem.RF_TEST_UNIAXIAL, R0, rad, 0.5, v_load=-5e-2, min_stress=1e3, max_strain=1.0)
+        specs.append((t, R, rad, extspec.stiff_params(seed=0xB2000000 + 310 + q)))
+    assert all(int(s[0].N) > 256 * 128 and int(s[0].N) % 128 for s in specs)
+    e = rfdem.BatchEngine([s[0] for s in specs], [s[3] for s in specs], [s[1] for s in specs], [s[2] for s in specs])
+    steps = 40
+    e.step(steps)
+    _check_against_oracle(e, specs, [steps] * 2)
+    curves = [e.curve_spec(q) for q in range(2)]
+    p = e.relax_params(max_iter=12, strain_inc=1e-4)
+    res = [e.load_increment(p) for _ in range(2)]
+    Rall = e.positions_f64()
+    for q, (t, R, rad, x) in enumerate(specs):
+        first, m, off, tq = e.spec_info(q)
+        Rq = R.reshape(3, m).copy()
+        Rq[0] += off
+        o = oracle.run_ext(mc.clone(tq), x, Rq.reshape(-1), rad, steps)
+        assert (o["curve"] != 0).any(0).all()
+        np.testing.assert_allclose(curves[q], o["curve"], rtol=1e-9, atol=1e-12)
+        a = rfdem.Engine(mc.clone(tq), Rq.reshape(-1), ext=x, radius=rad)
+        a.step(steps)
+        ra = [a.load_increment(p) for _ in range(2)]
+        Ra = a.positions_f64()
+        a.close()
+        for k in range(2):
+            assert res[k][q].iterations == ra[k].iterations
+            assert abs(res[k][q].stress - ra[k].stress) <= 1e-6 * abs(ra[k].stress)
+            assert abs(res[k][q].residual - ra[k].residual) <= 1e-6 * ra[k].residual
+        Re = Rall.reshape(3, e.N)[:, first:first + m].reshape(-1)
+        assert np.max(np.abs(Re - Ra)) < 1e-7 * float(np.ptp(Rq[2]))
+    e.close()
+
+
+@pytest.mark.parametrize("kind,d,h,steps", [(rfdem.RF_TEST_UNIAXIAL, 21.0, 26.0, 40), (rfdem.RF_TEST_BRAZIL, 52.0, 20.0, 20),
+                                            (rfdem.RF_TEST_UNIAXIAL, 41.0, 70.0, 6)], ids=IDS)
+def test_reference_model_load_curves(cuda, kind, d, h, steps):
+    t, R = rfdem.make_test(kind, d, h, seed=0xB2000000 + 5, max_strain=1.0, v_load=-1e-2)
+    n, _, curve, status = oracle.run_f(mc.clone(t), R, steps)
+    assert n == steps and status == 0 and np.abs(curve[:, 1:]).max(0).all()
+    e = rfdem.Engine(t, R)
+    e.step(steps)
+    got = e.curve()
+    e.close()
+    np.testing.assert_allclose(got, curve, rtol=1e-9, atol=1e-12)
