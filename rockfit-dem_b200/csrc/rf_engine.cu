@@ -2875,6 +2875,21 @@ rf_status dalloc(rf_engine* e, const Arrays& a) {
     return RF_OK;
 }
 
+// Rows in the reference layout, for a read-out or an import (released with the object).
+struct RowBuffers {
+    uint_fast32_t* IL = nullptr;
+    uint8_t* type = nullptr;
+    float* iL = nullptr;
+    rf_float3* S = nullptr;                  // Rij, Oijt, Mijn, Mijt, NK each
+    void* base = nullptr;
+    cudaError_t alloc(size_t NK) {
+        Arrays A;
+        A.add(&IL, NK); A.add(&type, NK); A.add(&iL, NK); A.add(&S, 4 * NK);
+        return A.alloc(&base);
+    }
+    ~RowBuffers() { cudaFree(base); }
+};
+
 #define TRY(x) do { rf_status s__ = (x); if (s__ != RF_OK) return s__; } while (0)
 
 // Explicit extended-model step kernels: compiled for 5, 6 and 8 CTAs per SM at 32 particles a
@@ -4008,23 +4023,19 @@ rf_status rf_engine_export(rf_engine* e, float* R, float* V, float* W, uint_fast
         RF_CUDA(cudaStreamSynchronize(s));
     }
     if (IL || ILtype || _1d_iL || Rij || Oijt || Mijn || Mijt) {
-        uint_fast32_t* dIL = nullptr; uint8_t* dT = nullptr; float* dL = nullptr; rf_float3* dS = nullptr;
-        cudaError_t ce = cudaMalloc(&dIL, NK * sizeof(uint_fast32_t));
-        if (!ce) ce = cudaMalloc(&dT, NK);
-        if (!ce) ce = cudaMalloc(&dL, NK * sizeof(float));
-        if (!ce) ce = cudaMalloc(&dS, 4 * NK * sizeof(rf_float3));
+        RowBuffers b;
+        cudaError_t ce = b.alloc(NK);
         if (!ce) {
-            k_rows_export<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dL, dS, dS + NK, dS + 2 * NK, dS + 3 * NK, e->d, e->c);
+            k_rows_export<<<(N + 127) / 128, 128, 0, s>>>(b.IL, b.type, b.iL, b.S, b.S + NK, b.S + 2 * NK, b.S + 3 * NK, e->d, e->c);
             ce = cudaGetLastError();
         }
-        if (!ce && IL) ce = cudaMemcpyAsync(IL, dIL, NK * sizeof(uint_fast32_t), cudaMemcpyDeviceToHost, s);
-        if (!ce && ILtype) ce = cudaMemcpyAsync(ILtype, dT, NK, cudaMemcpyDeviceToHost, s);
-        if (!ce && _1d_iL) ce = cudaMemcpyAsync(_1d_iL, dL, NK * sizeof(float), cudaMemcpyDeviceToHost, s);
+        if (!ce && IL) ce = cudaMemcpyAsync(IL, b.IL, NK * sizeof(uint_fast32_t), cudaMemcpyDeviceToHost, s);
+        if (!ce && ILtype) ce = cudaMemcpyAsync(ILtype, b.type, NK, cudaMemcpyDeviceToHost, s);
+        if (!ce && _1d_iL) ce = cudaMemcpyAsync(_1d_iL, b.iL, NK * sizeof(float), cudaMemcpyDeviceToHost, s);
         rf_float3* outs3[4] = {Rij, Oijt, Mijn, Mijt};
         for (int q = 0; q < 4 && !ce; ++q)
-            if (outs3[q]) ce = cudaMemcpyAsync(outs3[q], dS + q * NK, NK * sizeof(rf_float3), cudaMemcpyDeviceToHost, s);
+            if (outs3[q]) ce = cudaMemcpyAsync(outs3[q], b.S + q * NK, NK * sizeof(rf_float3), cudaMemcpyDeviceToHost, s);
         if (!ce) ce = cudaStreamSynchronize(s);
-        cudaFree(dIL); cudaFree(dT); cudaFree(dL); cudaFree(dS);
         if (ce) return cuda_status(ce, "rf_engine_export");
     }
     return RF_OK;
@@ -4057,29 +4068,25 @@ rf_status rf_engine_import(rf_engine* e, const float* R, const float* V, const f
         RF_CHECK_LAUNCH("k_planar_to_f4");
         RF_CUDA(cudaStreamSynchronize(s));
     }
-    uint_fast32_t* dIL = nullptr; uint8_t* dT = nullptr; float* dL = nullptr; rf_float3* dS = nullptr;
-    cudaError_t ce = cudaMalloc(&dIL, NK * sizeof(uint_fast32_t));
-    if (!ce) ce = cudaMalloc(&dT, NK);
-    if (!ce) ce = cudaMalloc(&dL, NK * sizeof(float));
-    if (!ce) ce = cudaMalloc(&dS, 4 * NK * sizeof(rf_float3));
-    if (!ce) ce = cudaMemcpyAsync(dIL, IL, NK * sizeof(uint_fast32_t), cudaMemcpyHostToDevice, s);
-    if (!ce) ce = cudaMemcpyAsync(dT, ILtype, NK, cudaMemcpyHostToDevice, s);
-    if (!ce) ce = cudaMemcpyAsync(dL, _1d_iL, NK * sizeof(float), cudaMemcpyHostToDevice, s);
+    RowBuffers b;
+    cudaError_t ce = b.alloc(NK);
+    if (!ce) ce = cudaMemcpyAsync(b.IL, IL, NK * sizeof(uint_fast32_t), cudaMemcpyHostToDevice, s);
+    if (!ce) ce = cudaMemcpyAsync(b.type, ILtype, NK, cudaMemcpyHostToDevice, s);
+    if (!ce) ce = cudaMemcpyAsync(b.iL, _1d_iL, NK * sizeof(float), cudaMemcpyHostToDevice, s);
     const rf_float3* ins3[4] = {Rij, Oijt, Mijn, Mijt};
     for (int q = 0; q < 4 && !ce; ++q)
-        ce = cudaMemcpyAsync(dS + q * NK, ins3[q], NK * sizeof(rf_float3), cudaMemcpyHostToDevice, s);
+        ce = cudaMemcpyAsync(b.S + q * NK, ins3[q], NK * sizeof(rf_float3), cudaMemcpyHostToDevice, s);
     uint32_t qb = 0;
     if (!ce) ce = cudaMemsetAsync(e->maxq_dev, 0, sizeof(uint32_t), s);
-    if (!ce) { k_count_records<<<148 * 4, 256, 0, s>>>(dIL, dT, dS, N, K, e->maxq_dev); ce = cudaGetLastError(); }
+    if (!ce) { k_count_records<<<148 * 4, 256, 0, s>>>(b.IL, b.type, b.S, N, K, e->maxq_dev); ce = cudaGetLastError(); }
     if (!ce) ce = cudaMemcpyAsync(&qb, e->maxq_dev, sizeof(qb), cudaMemcpyDeviceToHost, s);
     if (!ce) ce = cudaStreamSynchronize(s);
     if (!ce && qb > e->d.QB) {
-        cudaFree(dIL); cudaFree(dT); cudaFree(dL); cudaFree(dS);
         set_error("rf_engine_import: a row holds %u bond records, the engine was sized for %u", qb, e->d.QB);
         return RF_ERR_CAPACITY;
     }
     if (!ce) {
-        k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(dIL, dT, dL, dS, dS + NK, dS + 2 * NK, dS + 3 * NK, e->d, e->c);
+        k_rows_import<<<(N + 127) / 128, 128, 0, s>>>(b.IL, b.type, b.iL, b.S, b.S + NK, b.S + 2 * NK, b.S + 3 * NK, e->d, e->c);
         ce = cudaGetLastError();
     }
     if (!ce) {
@@ -4087,7 +4094,6 @@ rf_status rf_engine_import(rf_engine* e, const float* R, const float* V, const f
         ce = cudaGetLastError();
     }
     if (!ce) ce = cudaStreamSynchronize(s);
-    cudaFree(dIL); cudaFree(dT); cudaFree(dL); cudaFree(dS);
     if (ce) return cuda_status(ce, "rf_engine_import");
     return RF_OK;
 }
