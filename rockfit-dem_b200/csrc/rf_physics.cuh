@@ -24,15 +24,9 @@ __device__ __forceinline__ float norm3(float x, float y, float z) {
     return __fsqrt_rn(x * x + y * y + z * z);
 }
 
-// A slot's force and moment terms, in the order the reference adds them to the particle's
-// sums. SumTerms adds them at once; KeepTerms keeps them apart, for a particle's lane to add
-// in slot order when other lanes evaluated its slots (the rounding of the sums is the same).
-struct SumTerms {
-    f3 &fs, &ms;
-    __device__ __forceinline__ void f(float x, float y, float z) { fs.x += x; fs.y += y; fs.z += z; }
-    __device__ __forceinline__ void m(float x, float y, float z) { ms.x += x; ms.y += y; ms.z += z; }
-    __device__ __forceinline__ void clear_m() { ms = mk3(0.f, 0.f, 0.f); }
-};
+// A slot's force and moment terms, in the order the reference adds them to the particle's sums,
+// kept apart for the particle's lane to add in slot order: other lanes evaluate its slots (the
+// rounding of the sums is that of adding at once).
 struct KeepTerms {
     f3 ft[2], mt[3];
     int nf = 0, nm = 0;
@@ -43,13 +37,12 @@ struct KeepTerms {
 };
 
 // One bond slot i->j (d_CalculateForcesDEM_22 loop body, :441-473). r = Rj - Ri.
-// Hands its terms (two of force, three of moment) to `acc` in the reference's order and
+// Leaves its terms (two of force, three of moment) in `acc` in the reference's order and
 // updates the slot state. Returns true when the break check fired (the slot is then type 0
 // and its Oijt, Mijn, Mijt are zero).
-template <class Acc>
 __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const f3 vi, const f3 vj,
                                           const f3 wi, const f3 wj, const float il, f3& Rij, f3& Oijt,
-                                          f3& Mijn, f3& Mijt, Acc& acc) {
+                                          f3& Mijn, f3& Mijt, KeepTerms& acc) {
     // dd_Calculate_rijm_nij_2 (:38-52)
     const float rijm = norm3(r.x, r.y, r.z);
     const float inv_rm = __frcp_rn(rijm);
@@ -135,11 +128,10 @@ __device__ __forceinline__ bool bond_slot(const BondParams& p, const f3 r, const
 
 // One overlapping contact slot of type 0 (d_CalculateForcesDEM_21 loop body, :356-402);
 // r = Rj - Ri, rijm = norm3(r) < 2 rP (a pair that does not overlap has its Oijt set to zero
-// by the caller, as the reference does). Hands two force and two moment terms to `acc`, or
+// by the caller, as the reference does). Leaves two force and two moment terms in `acc`, or
 // one moment term and the clear of the moment sum.
-template <class Acc>
 __device__ __forceinline__ void contact_pair(const ContactParams& p, const f3 r, const float rijm, const f3 vi,
-                                             const f3 vj, const f3 wi, const f3 wj, f3& Oijt, Acc& acc) {
+                                             const f3 vj, const f3 wi, const f3 wj, f3& Oijt, KeepTerms& acc) {
     const float inv_rm = __frcp_rn(rijm);
     const float nx = r.x * inv_rm, ny = r.y * inv_rm, nz = r.z * inv_rm;
     // dd_Calculate_fijn_ppHM_2 (:199-253)
