@@ -342,8 +342,8 @@ __global__ void k_rb_scatter(Dev d, Consts c) {
 // run of float4 records, nine runs a particle). A particle first only collects, in shared memory,
 // the places of its candidates in that order (what else a candidate needs would be run by the
 // whole warp for each of its lanes' hits in turn); the buckets and the row's members, found by
-// their places, follow. 4M particles: 3.0 ms with an id and a position gathered for
-// every occupant and the list ordered and matched in memory, 2.5 ms so.
+// their places, follow. A build of 4M particles takes 2.2 ms (2.03 of it this kernel), 3.0 with
+// an id and a position gathered for every occupant and the list ordered and matched in memory.
 #define RF_RB_CTA 128
 __global__ void __launch_bounds__(RF_RB_CTA) k_rb_cand(Dev d, Consts c) {
     if (gate_closed(d, c)) return;
@@ -2551,7 +2551,7 @@ struct BondSpec {
 // test); else the extended model's pair test |r| < min(a_farcut, r_i + r_j + gap) on the FP64
 // positions. Nothing of a row exists in the reference layout in between: seven FP32 triples a
 // slot, their zeroing and about 60 allocations were most of a creation. Creation, an affine
-// strain, 100 steps and the read-back of 200k particles: 42 -> 18 ms.
+// strain, 100 steps and the read-back of 200k particles: 43 -> 15 ms (with the faster steps).
 __global__ void __launch_bounds__(128) k_rows_list(const float* __restrict__ R, Dev d, Consts c,
                                                    const uint_fast32_t* __restrict__ CIs,
                                                    const uint_fast32_t* __restrict__ pnC, double a_farcut, double gap,
@@ -2893,7 +2893,8 @@ struct RowBuffers {
 #define TRY(x) do { rf_status s__ = (x); if (s__ != RF_OK) return s__; } while (0)
 
 // Explicit extended-model step kernels: compiled for 5, 6 and 8 CTAs per SM at 32 particles a
-// warp, for 6 alone with fewer (there minb has no effect).
+// warp (96, 80 and 64 registers), for 6 alone with fewer (80 registers, 164 to 172 bytes of
+// spill stores), where minb has no effect.
 template <int KIND>
 void* ext_step_kind(int pw, int minb) {
     switch (pw) {
@@ -3041,7 +3042,10 @@ rf_status build_graph(rf_engine* e) {
 // times forces, update }. A conditional node costs several microseconds, so the body holds more
 // than one iteration; once an update finds that the candidates have to be rebuilt, the rest of the
 // body leaves at once (fire_skip), and the rebuild precedes the next force pass as if every
-// iteration had its IF. Six specimens of 3000 particles: 34.8 -> 28.8 us an iteration.
+// iteration had its IF. Six specimens of 3000 particles: 34.8 -> 28.8 us an iteration. An increment
+// that stops inside a body still launches its other iterations, which leave at once: with 20k
+// particles one iteration takes 297 us (237 with an IF each), 16 take as long as before, and
+// from there on the longer body gains.
 rf_status build_fire_graph(rf_engine* e) {
     cudaGraph_t g;
     RF_CUDA(cudaGraphCreate(&g, 0));

@@ -1,4 +1,5 @@
-// BF16 tensor-core GEMM for sm_100a (tcgen05 + TMEM) and the warm-start MLP built on it.
+// BF16 tensor-core GEMM for sm_100a (tcgen05 + TMEM) and, with fused kernels of its own, the
+// warm-start MLP.
 //
 // rf_gemm_bf16 computes C[M x N] = A[M x K] * B[N x K]^T with both operands K-major
 // (row-major with K contiguous), BF16 inputs and FP32 accumulation in tensor memory:
@@ -11,9 +12,8 @@
 //     tcgen05.mma.kind::f16 (M=128, K=16 each) into the TMEM accumulator and commits
 //     them to an mbarrier that all threads wait on (bounded);
 //   - the epilogue reads the accumulator with tcgen05.ld (warp w owns TMEM lanes
-//     32w..32w+31, one row per thread) and applies bias/ReLU, the ReLU mask of the
-//     backward pass, or the split-K atomic add, writing BF16 rows, their transpose
-//     (the next GEMM's K-major operand) or FP32.
+//     32w..32w+31, one row per thread) and applies bias/ReLU, a ReLU mask, or the split-K
+//     atomic add, writing BF16 rows, their transpose or FP32.
 // Waits give up after a bounded number of polls, raise an error flag and still free the
 // tensor memory before returning.
 #include <cuda_bf16.h>
@@ -320,10 +320,11 @@ extern "C" rf_status rf_gemm_status(rf_stream stream) {
 // gradients stay in tensor memory until the CTA has seen all its tiles. What a step must
 // move is then the features and targets (152 B a row) and, for the bias sums, dZ (800 B a
 // row, written and read); the arithmetic is about 235 kFLOP a row (0.31 ms at the measured
-// tensor rate for 2M rows). Measured on a B200: a training step on 2M rows 2.3 ms, inference of 300k rows 67 us with the host's wait;
-// layer-by-layer GEMMs with the activations and their transposes in memory took 58 ms and
-// 1.59 ms. What bounds both is the chain of a tile (GEMM, accumulator read, conversion,
-// shared-memory write, barrier, seven times over in training): the tensor cores idle in it.
+// tensor rate for 2M rows). Measured on a B200: a training step on 2M rows 2.4 ms, inference
+// of 300k rows 66 us with the host's wait; layer-by-layer GEMMs with the activations and
+// their transposes in memory took 58 ms and 1.58 ms. What bounds both is the chain of a tile
+// (GEMM, accumulator read, conversion, shared-memory write, barrier, seven times over in
+// training): the tensor cores idle in it.
 //
 // Every matrix in shared memory is in 8-row x 16-byte core matrices (128 contiguous
 // bytes): core (rg, cg) of a buffer of R rows at cg * R * 16 + rg * 128, so that element
@@ -605,7 +606,7 @@ k_mlp_forward(MlpWeights w, const __nv_bfloat16* __restrict__ X, int rows, float
 // A split's weight gradients are one tensor-memory accumulation over its rows in order, the
 // splits those of a split-K GEMM over 64-row chunks: the FP32 accumulator's rounding over tens
 // of thousands of rows is the largest error of a step, and with other splits (one per SM, every
-// 148th tile: 0.97 ms a step at 2M rows against 2.3 ms) the gradients moved by 5e-5.
+// 148th tile: 0.97 ms a step at 2M rows against 2.4 ms) the gradients moved by 5e-5.
 __global__ void __launch_bounds__(MLP_T_THREADS, 1)
 k_mlp_train(MlpWeights w, const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, int rows, long split,
             int residual, float* __restrict__ part, double* __restrict__ loss_part, BiasRows out_rows, uint32_t* err) {
